@@ -203,6 +203,23 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree,
                       const void *coefs, int32_t coef_type, int32_t nrhs,
                       void *result, void *stream);
 
+/* The same sums as vl1_eval_fp64 over a tile schedule of the tree: on the
+ * tensor cores with 8 + 8 exact digits per product, so that every target box
+ * keeps FP64 accuracy against its own largest list-1 density (see
+ * csrc/vl1_wide.cu); rows with non-finite sources are summed in FP64.
+ * schedule: built for nrhs rows per box (2 nrhs for complex coefficients),
+ * its work items at most vl1_eval_fp64_item_keys keys long.  The first call
+ * with a plan builds its table digits and synchronises the stream; scratch
+ * is allocated and freed in stream order.  Evaluates as vl1_eval_fp64 while
+ * the stream is being captured, where the scratch cannot be had, or where a
+ * box has more than 256 points. */
+int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
+                            const vl1_mixed_schedule *schedule, const void *coefs,
+                            int32_t coef_type, int32_t nrhs, void *result, void *stream);
+
+/* The most keys a work item may have in vl1_eval_fp64_tiles. */
+int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan);
+
 /* Table key (table_level * n_cases + case) of every list-1 pair, computed with
  * the reference's FP64 case encoding (list1.py:439-459, 1084-1091) and table
  * level rule (list1.py:361-437); keys: device array [nnz], -1 for pairs whose

@@ -416,6 +416,48 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree, const void *coe
                       static_cast<cudaStream_t>(stream));
 }
 
+// a work item's digit sums of weights 2^-56 .. 2^-72 must fit an int32:
+// (2^16 + 7 * 2^14) K < 2^31
+int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan) {
+  if (!plan) return 0;
+  const int kp = vl1::wide_geometry(plan->d.nq, plan->d.table_cplx).kp;
+  return kp >= 8192 ? 1 : 8192 / kp;
+}
+
+int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
+                            const vl1_mixed_schedule *schedule, const void *coefs,
+                            int32_t coef_type, int32_t nrhs, void *result, void *stream) {
+  if (!plan || !schedule) {
+    set_error("vl1_eval_fp64_tiles: null plan or schedule");
+    return VL1_E_ARG;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaError_t e = cudaStreamIsCapturing(s, &cap);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
+  // beyond vl1_eval_fp64's own limits its error is reported
+  if (cap != cudaStreamCaptureStatusNone || plan->d.nq > 256 || nrhs < 1 || nrhs > 65535 ||
+      !coefs || !result || (coef_type != VL1_REAL64 && coef_type != VL1_COMPLEX128))
+    return vl1_eval_fp64(plan, tree, coefs, coef_type, nrhs, result, stream);
+  TreeDev tr;
+  int32_t st = make_tree(plan, tree, tr);
+  if (st) return st;
+  if (tr.n_tgt_boxes == 0) return VL1_OK;
+  const vl1_mixed_schedule &sc = *schedule;
+  if (sc.n_tiles < 0 || sc.n_items < 0 || sc.n_splits < 0 || sc.n_slots < 0 ||
+      (sc.n_tiles > 0 &&
+       (!sc.tile_rows || !sc.tile_key_start || !sc.key_ids || !sc.key_xrow)) ||
+      (sc.n_items > 0 && !sc.items) || (sc.n_items == 0 && sc.n_splits > 0)) {
+    set_error("vl1_eval_fp64_tiles: invalid schedule");
+    return VL1_E_ARG;
+  }
+  st = launch_wide(plan, tr, sc, static_cast<const double *>(coefs),
+                   coef_type == VL1_COMPLEX128, nrhs, static_cast<double *>(result), s);
+  if (st == VL1_E_NOMEM || st == VL1_E_UNSUPPORTED)
+    return vl1_eval_fp64(plan, tree, coefs, coef_type, nrhs, result, stream);
+  return st;
+}
+
 int32_t vl1_classify_pairs(vl1_plan *plan, const vl1_tree_view *tree, int32_t *keys,
                            void *stream) {
   if (!plan || !keys) {

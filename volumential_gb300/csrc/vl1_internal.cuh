@@ -6,6 +6,7 @@
 
 #include "vl1.h"
 #include "vl1_mixed.cuh"
+#include "vl1_wide.cuh"
 
 namespace vl1 {
 
@@ -65,6 +66,7 @@ struct vl1_plan {
   int n_allocs;
   vl1_status *status;   // device
   vl1::MixedPlan mixed;
+  vl1::WidePlan wide;
 };
 
 namespace vl1 {
@@ -82,6 +84,14 @@ int32_t launch_expand_blocks(vl1_plan *plan, cudaStream_t s);
 int32_t launch_index_map(vl1_plan *plan, int32_t *rows, int8_t *signs, cudaStream_t s);
 int32_t launch_plain(vl1_plan *plan, const TreeDev &tree, const double *coefs,
                      int coef_cplx, int nrhs, double *result, cudaStream_t s);
+// FP64-accurate tensor-core evaluation over a tile schedule of nrhs (complex
+// coefficients: 2 nrhs) rows per box; its table digits take
+// wide_operand_bytes of the plan
+int64_t wide_operand_bytes(const vl1_plan *plan);
+WideGeom wide_geometry(int nq, int table_cplx);
+int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_mixed_schedule &sched,
+                    const double *coefs, int coef_cplx, int nrhs, double *result,
+                    cudaStream_t s);
 // operand geometry; kc / nch 0: the default choice (else 16 or 32 / 16, 32
 // or 64, validated by the caller)
 MixedGeom mixed_geometry(int nq, int table_cplx, int kc = 0, int nch = 0);

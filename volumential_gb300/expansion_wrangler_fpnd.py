@@ -792,7 +792,7 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
                               device="cuda")
             stream = stream_handle(self.queue)
             if precision == "fp64":
-                plan.eval_fp64(view, c, out, stream=stream, nrhs=nrhs)
+                plan.eval_fp64(view, c, out, stream=stream, nrhs=nrhs, keep=keep)
             else:
                 from .batched import eval_mixed
                 eval_mixed(plan, view, c, out, stream=stream, nrhs=nrhs, keep=keep)

@@ -633,7 +633,7 @@ class NearFieldFromCSR(NearFieldEvalBase):
         stream = stream_handle(queue)
         precision = self.extra_kwargs.get("list1_precision", "fp64")
         if precision == "fp64":
-            plan.eval_fp64(view, coefs, out, stream=stream, nrhs=1)
+            plan.eval_fp64(view, coefs, out, stream=stream, nrhs=1, keep=keep)
         elif precision == "mixed":
             from .batched import eval_mixed
             eval_mixed(plan, view, coefs, out, stream=stream, nrhs=1, keep=keep)

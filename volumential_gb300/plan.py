@@ -20,6 +20,14 @@ __all__ = ["Plan", "plan_cache_get", "tree_view_from_arrays", "as_device_tensor"
            "stream_handle", "require_cuda", "PLAN_CACHE_MAX"]
 
 PLAN_CACHE_MAX = 16
+#: modelled time of the per-box FP64 kernel from which the tensor-core path is
+#: taken, and from which a tree's schedule is built on its first evaluation
+#: (``Plan._fp64_schedule``): at 60 us both take the same time (2D, q = 4,
+#: level 6: 75 and 57 us; 3D, q = 3, level 3: 49 and 51 us; 2D, level 5: 21
+#: and 53 us), at 1.5 ms the schedule costs what it saves at once (3D, q = 4,
+#: level 4: 875 us against 700 + 75 us)
+FP64_TILE_US = 60.0
+FP64_BUILD_US = 1500.0
 _cache: "collections.OrderedDict" = collections.OrderedDict()
 _cache_lock = threading.Lock()
 
@@ -311,8 +319,13 @@ class Plan:
         except Exception:
             pass
 
-    def eval_fp64(self, view, coefs, out, *, stream, nrhs=1):
-        """Plain FP64 kernel; ``coefs``/``out`` are CUDA tensors [nrhs*N]."""
+    def eval_fp64(self, view, coefs, out, *, stream, nrhs=1, keep=None):
+        """FP64 evaluation; ``coefs``/``out`` are CUDA tensors [nrhs*N].
+
+        With ``keep`` (the tree's device tensors, as ``tree_view_from_arrays``
+        returns them beside ``view``) large sums run on the tensor cores with
+        FP64-accurate digit products (``vl1_eval_fp64_tiles``), see
+        ``_fp64_schedule``; without it, in the per-box FP64 kernel."""
         import torch
         if coefs.dtype not in (torch.float64, torch.complex128):
             raise TypeError("coefs must be float64 or complex128")
@@ -322,9 +335,68 @@ class Plan:
             raise ValueError(f"coefs/result must hold nrhs*n_particles = {nrhs * n} values")
         if not (coefs.is_cuda and out.is_cuda and coefs.is_contiguous() and out.is_contiguous()):
             raise ValueError("coefs and result must be contiguous CUDA tensors")
+        sched = None
+        if keep is not None:
+            sched = self._fp64_schedule(view, keep, coefs.is_complex(), int(nrhs), stream)
+        if sched is not None:
+            st = self._lib.vl1_eval_fp64_tiles(
+                self.handle, C.byref(view), C.byref(sched.c_struct), coefs.data_ptr(), ctype,
+                int(nrhs), out.data_ptr(), C.c_void_p(stream))
+            _lib.check(st, "vl1_eval_fp64_tiles")
+            return
         st = self._lib.vl1_eval_fp64(self.handle, C.byref(view), coefs.data_ptr(), ctype,
                                      int(nrhs), out.data_ptr(), C.c_void_p(stream))
         _lib.check(st, "vl1_eval_fp64")
+
+    def _fp64_schedule(self, view, keep, complex_coefs, nrhs, stream):
+        """The tile schedule for a tensor-core FP64 evaluation, or None where
+        the per-box kernel is the faster way (or the only one).
+
+        A call of the tensor-core path takes 50 us and more, the per-box
+        kernel ``_per_box_us``.  A tree seen for the first time has no
+        schedule yet, and building one takes 0.4 ms (2D, a thousand boxes) to
+        1.5 ms (3D, 23,000 boxes): below FP64_BUILD_US only a tree that comes
+        again (the same view object) gets one.  Trees that no schedule
+        describes (two sources of a box in one mode, two list-1 boxes of one
+        case) stay with the per-box kernel, as do calls under graph capture
+        that would have to build one."""
+        rows = 2 * nrhs if complex_coefs else nrhs
+        us = self._per_box_us(view, keep, rows)
+        if us < FP64_TILE_US or self.nq > 256:
+            return None
+        known = view.__dict__.setdefault("fp64_schedules", {})
+        hit = known.get(rows)
+        if hit is not None and hit[0] is self:
+            return hit[1]
+        if hit is None and us < FP64_BUILD_US:
+            known[rows] = (None, None)      # built when the tree comes again
+            return None
+        import torch
+
+        from .batched import get_schedule
+        if torch.cuda.is_current_stream_capturing():
+            return None
+        try:
+            cap = int(self._lib.vl1_eval_fp64_item_keys(self.handle))
+            sched = get_schedule(self, view, keep, rows, stream)
+            if sched.max_keys_per_item > cap:
+                sched = get_schedule(self, view, keep, rows, stream, max_keys_per_item=cap)
+        except (ValueError, RuntimeError):
+            sched = None
+        known[rows] = (self, sched)
+        return sched
+
+    def _per_box_us(self, view, keep, rows):
+        """Modelled time of the per-box FP64 kernel: its products at the
+        0.95 TFLOP/s that the FP64 pipe gives it, or, with few boxes, one
+        box's chain of sources (0.38 us each, split over up to 128 / q^d
+        threads per target point); within 20 % of the measured times from
+        60 us to 7 ms."""
+        pairs = keep["lists"].numel()
+        flops = 2.0 * pairs * self.nq * self.nq * rows * (2.0 if self.complex_table else 1.0)
+        split = min(max(round(128.0 / self.nq), 1), 8)
+        chain = pairs / max(int(view.n_target_boxes), 1) * self.nq / split
+        return max(flops / 0.95e6, 0.38 * chain)
 
     def mixed_geometry(self):
         out = (C.c_int32 * 5)()

@@ -411,6 +411,16 @@ typedef struct {
 
 int32_t vl1_duffy_table(const vl1_duffy_desc *desc, double *result, void *stream);
 
+/* The same values with the entries grouped by target: entry_group [n_entries]
+ * (device) is the group of each entry, group_entry [n_groups] (device) an
+ * entry of each group; the entries of a group have the same target_points and
+ * decomposition_targets.  All modes of a target share its quadrature nodes'
+ * kernel values.  Kernels that are not radial, derivatives and orders without
+ * an instance are built as by vl1_duffy_table. */
+int32_t vl1_duffy_table_grouped(const vl1_duffy_desc *desc, int32_t n_groups,
+                                const int32_t *entry_group, const int32_t *group_entry,
+                                double *result, void *stream);
+
 /* ---- Helmholtz split correction ---------------------------------------
  * The split mode's list-1 remainder (volumential/expansion_wrangler_fpnd.py:
  * 3491-3836, series remainder kernel :212-332; for split orders above 1 the

@@ -13,11 +13,27 @@
 // whose Jacobian prod_{i<d-1} r_i^(d-1-i) cancels the singularity at the
 // target; r_0 (radial) takes a tanh-sinh rule, r_1.. a Gauss-Legendre rule.
 //
-// GPU layout: one CTA per entry, threads striding over the quadrature nodes
-// (sign vector x axis order x regular nodes x radial nodes, decoded from the
-// node index; only the 1D rules are read), FP64 sums reduced per CTA.  The
-// node count per entry is 2^d d! n_reg^(d-1) n_rad (3D, default orders:
-// 8 x 6 x 400 x 123 = 2.4M), so the kernel is bound by the FP64 pipe.
+// The node count per target is 2^d d! n_reg^(d-1) n_rad (3D, default orders:
+// 8 x 6 x 400 x 123 = 2.4M) and the FP64 pipe bounds both kernels below.
+//
+// duffy_group_kernel (radial kernels): all q^d modes of one target together.
+// On a simplex the coordinate along the i-th axis of its order is
+// dc + s r_0 .. r_i, so the sums over r_{d-1}, .., r_0 nest: for a fixed
+// (r_0, .., r_{d-2}) the last axis' basis functions are polynomials of
+// degree q - 1 in r_{d-1}, and the sum over r_{d-1} is taken once against
+// the Lagrange basis on q Chebyshev points xi_k of [0, 1] (moments M_k, one
+// FMA per k and node), then turned into all q modes through their values at
+// r_0 .. r_{d-2} xi_k.  Per node: the distance, one kernel value and q FMAs,
+// against the kernel value and d (q - 1) products per node *and entry* of
+// duffy_entry_kernel.
+//
+// Measured (GB300, default orders, whole build calls): 3D Laplace q = 4
+// (12,936 entries, 636 targets) 370 -> 12 ms, 3D Helmholtz q = 4 604 -> 32 ms,
+// 2D Helmholtz q = 5 4.3 -> 1.3 ms; entries within 1e-15 of the per-entry
+// sums, relative to the largest.
+//
+// duffy_entry_kernel (plane waves, derivatives, q beyond the instances): one
+// CTA per entry and simplex, threads striding over the nodes.
 
 #include <cuda_runtime.h>
 
@@ -300,6 +316,315 @@ __global__ void duffy_reduce_kernel(const double *part, int n_entries, int n_chu
   }
 }
 
+// ---------------------------------------------- all modes of a target
+
+// G(r) times the kernel's scaling constant for the radial kernels
+__device__ __forceinline__ void green_radial(int kind, double k, int power, double r2,
+                                             double &re, double &im) {
+  im = 0.0;
+  switch (kind) {
+    case VL1_DUFFY_LAPLACE2D:   // -log(r) / (2 pi)
+      re = -0.5 * log(r2) * (0.5 / 3.141592653589793);
+      break;
+    case VL1_DUFFY_LAPLACE3D:   // 1 / (4 pi r)
+      re = rsqrt(r2) * (0.25 / 3.141592653589793);
+      break;
+    case VL1_DUFFY_HELMHOLTZ2D: {
+      const double kr = k * sqrt(r2);
+      re = -0.25 * y0(kr);
+      im = 0.25 * j0(kr);
+      break;
+    }
+    case VL1_DUFFY_HELMHOLTZ3D: {
+      const double r = sqrt(r2);
+      double s, c;
+      sincos(k * r, &s, &c);
+      const double f = (0.25 / 3.141592653589793) / r;
+      re = c * f;
+      im = s * f;
+      break;
+    }
+    case VL1_DUFFY_CONSTANT:
+      re = 1.0;
+      break;
+    default: {   // VL1_DUFFY_POWER, VL1_DUFFY_POWER_LOG
+      double v = 1.0;
+      for (int i = 0; i < power / 2; ++i) v *= r2;
+      if (power & 1) v *= sqrt(r2);
+      re = kind == VL1_DUFFY_POWER ? v : v * (0.5 * log(r2));
+      break;
+    }
+  }
+}
+
+// values of the Q Lagrange polynomials on the nodes x at y (first form,
+// products from the left and from the right)
+template <int Q>
+__device__ __forceinline__ void lagrange_values(double y, const double *x, const double *bw,
+                                                double (&l)[Q]) {
+  double left = 1.0;
+#pragma unroll
+  for (int m = 0; m < Q; ++m) {
+    l[m] = bw[m] * left;
+    left *= y - x[m];
+  }
+  double right = 1.0;
+#pragma unroll
+  for (int m = Q - 1; m >= 0; --m) {
+    l[m] *= right;
+    right *= y - x[m];
+  }
+}
+
+struct DuffyGroupArgs {
+  vl1_duffy_desc d;
+  int n_groups, n_perm, n_chunks;
+  const int32_t *group_entry;   // an entry with the group's target
+  double *part;                 // [group][chunk][mode][re (, im)]
+};
+
+constexpr int kGroupThreads = 128;
+// radial nodes below this carry no weight that a double could hold beside
+// the others (their products with the Jacobian are below 1e-60), and their
+// distances could leave the FP64 range
+constexpr double kLeastRadius = 1e-60;
+
+template <int DIM, int Q, bool CPLX>
+constexpr int group_smem_doubles(int n_reg) {
+  constexpr int NU = (DIM == 3 ? Q * Q : Q) * (CPLX ? 2 : 1);
+  return 3 * Q + n_reg * (2 + Q) + kGroupThreads * (NU + 1 + Q);
+}
+
+// One CTA per (target, simplex) work item, or a capped grid striding over
+// them; a thread takes one radial node at a time and sums over the regular
+// nodes, its sums over the last d - 1 axes' modes in registers (U), and the
+// CTA then contracts them with the first axis' basis over its radial nodes.
+template <int DIM, int Q, bool CPLX>
+__global__ void __launch_bounds__(kGroupThreads) duffy_group_kernel(const DuffyGroupArgs A) {
+  const vl1_duffy_desc &D = A.d;
+  constexpr int CV = CPLX ? 2 : 1;
+  constexpr int NU = (DIM == 3 ? Q * Q : Q) * CV;
+  constexpr int NM = (DIM == 3 ? Q * Q * Q : Q * Q) * CV;   // outputs
+  constexpr int US = NU + 1;   // odd strides: the contraction reads a column of a thread each
+  extern __shared__ __align__(16) double sm[];
+  double *s_x = sm, *s_bw = s_x + Q, *s_xi = s_bw + Q;
+  double *s_r = s_xi + Q, *s_w = s_r + D.n_reg, *s_phi = s_w + D.n_reg;   // [n_reg][Q]
+  double *s_u = s_phi + D.n_reg * Q, *s_l0 = s_u + kGroupThreads * US;    // [thread][..]
+  const int tid = threadIdx.x;
+  if (tid < Q) {
+    s_x[tid] = D.interp_nodes[tid];
+    s_bw[tid] = D.interp_weights[tid];
+    s_xi[tid] = 0.5 - 0.5 * cospi((2 * tid + 1) / (2.0 * Q));
+  }
+  __syncthreads();
+  for (int i = tid; i < D.n_reg; i += kGroupThreads) {
+    s_r[i] = D.regular_nodes[i];
+    s_w[i] = D.regular_weights[i];
+    for (int k = 0; k < Q; ++k) {   // weight x Lagrange basis on the Chebyshev points
+      double v = D.regular_weights[i];
+      for (int j = 0; j < Q; ++j)
+        if (j != k) v *= (D.regular_nodes[i] - s_xi[j]) / (s_xi[k] - s_xi[j]);
+      s_phi[i * Q + k] = v;
+    }
+  }
+  __syncthreads();
+  const int64_t n_work = (int64_t)A.n_groups * A.n_chunks;
+  for (int64_t item = blockIdx.x; item < n_work; item += gridDim.x) {
+    const int g = (int)(item / A.n_chunks), chunk = (int)(item - (int64_t)g * A.n_chunks);
+    const int e = A.group_entry[g];
+    const int iperm = chunk % A.n_perm, isub = chunk / A.n_perm;
+    double *part = A.part + item * NM;
+    // along axis a: source coordinate dc + s c, displacement b - s c
+    double dc[3] = {}, b[3] = {}, s[3] = {};
+    bool active = true;
+    double len_prod = 1.0;
+#pragma unroll
+    for (int i = 0; i < DIM; ++i) {   // in the order of the simplex
+      const int a = DIM == 3 ? kPerm3[iperm][i] : kPerm2[iperm][i];
+      const double t = D.target_points[(int64_t)a * D.n_entries + e];
+      dc[i] = D.decomposition_targets[(int64_t)a * D.n_entries + e];
+      b[i] = t - dc[i];
+      const bool up = (isub >> (DIM - 1 - a)) & 1;
+      const double len = up ? D.extent - dc[i] : dc[i];
+      active = active && len > 0.0;
+      len_prod *= len;
+      s[i] = up ? len : -len;
+    }
+    if (!active) {   // uniform: an empty sub-box
+      for (int m = tid; m < NM; m += kGroupThreads) part[m] = 0.0;
+      continue;
+    }
+    double sum[(NM + kGroupThreads - 1) / kGroupThreads] = {};
+    for (int i0 = 0; i0 < D.n_rad; i0 += kGroupThreads) {
+      const int i = i0 + tid;
+      const double r0 = i < D.n_rad ? D.radial_nodes[i] : 0.0;
+      double u[NU];
+#pragma unroll
+      for (int n = 0; n < NU; ++n) u[n] = 0.0;
+      if (r0 >= kLeastRadius) {
+        const double d0 = fma(-s[0], r0, b[0]);
+        const double base0 = d0 * d0;
+        const int n1 = DIM == 3 ? D.n_reg : 1;
+        for (int j1 = 0; j1 < n1; ++j1) {
+          const double a = DIM == 3 ? r0 * s_r[j1] : r0;
+          double base = base0;
+          if (DIM == 3) {
+            const double d1 = fma(-s[1], a, b[1]);
+            base = fma(d1, d1, base0);
+          }
+          const double c = s[DIM - 1] * a;
+          double mom[Q * CV];
+#pragma unroll
+          for (int k = 0; k < Q * CV; ++k) mom[k] = 0.0;
+#pragma unroll 2
+          for (int j2 = 0; j2 < D.n_reg; ++j2) {
+            const double d2 = fma(-c, s_r[j2], b[DIM - 1]);
+            const double r2 = fma(d2, d2, base);
+            double gre = 0.0, gim = 0.0;
+            if (r2 > 0.0) green_radial(D.kernel, D.k, D.power, r2, gre, gim);
+#pragma unroll
+            for (int k = 0; k < Q; ++k) {
+              mom[k * CV] = fma(gre, s_phi[j2 * Q + k], mom[k * CV]);
+              if (CPLX) mom[k * CV + 1] = fma(gim, s_phi[j2 * Q + k], mom[k * CV + 1]);
+            }
+          }
+          // the last axis' modes from the moments
+          double tm[Q * CV];
+#pragma unroll
+          for (int k = 0; k < Q * CV; ++k) tm[k] = 0.0;
+#pragma unroll
+          for (int k = 0; k < Q; ++k) {
+            double l[Q];
+            lagrange_values<Q>(fma(c, s_xi[k], dc[DIM - 1]), s_x, s_bw, l);
+#pragma unroll
+            for (int m = 0; m < Q; ++m) {
+              tm[m * CV] = fma(l[m], mom[k * CV], tm[m * CV]);
+              if (CPLX) tm[m * CV + 1] = fma(l[m], mom[k * CV + 1], tm[m * CV + 1]);
+            }
+          }
+          if (DIM == 3) {
+            double l[Q];
+            lagrange_values<Q>(fma(s[1], a, dc[1]), s_x, s_bw, l);
+            const double w1 = s_w[j1] * s_r[j1];
+#pragma unroll
+            for (int m1 = 0; m1 < Q; ++m1) {
+              const double lw = l[m1] * w1;
+#pragma unroll
+              for (int m = 0; m < Q * CV; ++m)
+                u[m1 * Q * CV + m] = fma(lw, tm[m], u[m1 * Q * CV + m]);
+            }
+          } else {
+#pragma unroll
+            for (int m = 0; m < Q * CV; ++m) u[m] = tm[m];
+          }
+        }
+      }
+      double l[Q];
+      lagrange_values<Q>(fma(s[0], r0, dc[0]), s_x, s_bw, l);
+      const double w0 = i < D.n_rad ? D.radial_weights[i] * len_prod *
+                                          (DIM == 3 ? r0 * r0 : r0)
+                                    : 0.0;
+#pragma unroll
+      for (int m = 0; m < Q; ++m) s_l0[tid * Q + m] = l[m] * w0;
+#pragma unroll
+      for (int n = 0; n < NU; ++n) s_u[tid * US + n] = u[n];
+      __syncthreads();
+      const int n_act = min(kGroupThreads, D.n_rad - i0);
+#pragma unroll
+      for (int o = 0; o < (NM + kGroupThreads - 1) / kGroupThreads; ++o) {
+        const int m = o * kGroupThreads + tid;
+        if (m < NM) {
+          const int m0 = m / NU, n = m - m0 * NU;
+          double v = sum[o];
+          for (int q = 0; q < n_act; ++q) v = fma(s_l0[q * Q + m0], s_u[q * US + n], v);
+          sum[o] = v;
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int o = 0; o < (NM + kGroupThreads - 1) / kGroupThreads; ++o) {
+      const int m = o * kGroupThreads + tid;
+      if (m < NM) {
+        // simplex order (m0, m1, (m2)) to axis order, axis 0 slowest
+        int rest = m / CV, mode = 0;
+#pragma unroll
+        for (int i = DIM - 1; i >= 0; --i) {
+          const int a = DIM == 3 ? kPerm3[iperm][i] : kPerm2[iperm][i];
+          int stride = 1;
+          for (int x = a; x < DIM - 1; ++x) stride *= Q;
+          mode += (rest % Q) * stride;
+          rest /= Q;
+        }
+        part[mode * CV + m % CV] = sum[o];
+      }
+    }
+  }
+}
+
+// the entries' values: the partial sums of their target and mode over the
+// simplices, in order (a fixed one, whatever the grid)
+__global__ void duffy_group_reduce_kernel(const vl1_duffy_desc D, const double *part,
+                                          const int32_t *entry_group, int n_chunks, int cv,
+                                          double *out) {
+  const int nm = (D.dim == 3 ? D.q * D.q * D.q : D.q * D.q) * cv;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < D.n_entries;
+       e += gridDim.x * blockDim.x) {
+    int mode = 0;
+    bool ok = true;
+    for (int a = 0; a < D.dim; ++a) {
+      const int m = D.mode_axes[(int64_t)a * D.n_entries + e];
+      ok = ok && m >= 0 && m < D.q;
+      mode = mode * D.q + m;
+    }
+    double re = 0.0, im = 0.0;
+    if (ok) {
+      const double *p = part + (int64_t)entry_group[e] * n_chunks * nm + mode * cv;
+      for (int c = 0; c < n_chunks; ++c) {
+        re += p[(int64_t)c * nm];
+        if (cv == 2) im += p[(int64_t)c * nm + 1];
+      }
+    } else {   // an invalid entry yields NaN (the host checks its inputs)
+      re = im = __longlong_as_double(0x7FF8000000000000ll);
+    }
+    if (D.complex_output) {
+      out[2 * (int64_t)e] = re;
+      out[2 * (int64_t)e + 1] = im;
+    } else {
+      out[e] = re;
+    }
+  }
+}
+
+template <int DIM, int Q, bool CPLX>
+cudaError_t launch_group(const DuffyGroupArgs &A, int64_t cap, cudaStream_t s) {
+  const size_t smem = sizeof(double) * (size_t)group_smem_doubles<DIM, Q, CPLX>(A.d.n_reg);
+  if (smem > 200 * 1024) return cudaErrorInvalidValue;
+  cudaError_t e = cudaSuccess;
+  if (smem > 48 * 1024)
+    e = cudaFuncSetAttribute(duffy_group_kernel<DIM, Q, CPLX>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return e;
+  const int64_t n_work = (int64_t)A.n_groups * A.n_chunks;
+  const int64_t grid = std::min<int64_t>(std::min(n_work, cap > 0 ? cap : n_work), 0x7FFFFFFF);
+  duffy_group_kernel<DIM, Q, CPLX><<<(unsigned)grid, kGroupThreads, smem, s>>>(A);
+  return cudaGetLastError();
+}
+
+// the instances: q up to 6 in 3D (5 with complex values: U of a thread is
+// q^2 values in registers), up to 8 in 2D
+using GroupLaunch = cudaError_t (*)(const DuffyGroupArgs &, int64_t, cudaStream_t);
+GroupLaunch group_launch(int dim, int q, bool cplx) {
+#define VL1_G(DIM, Q)                                        \
+  if (dim == DIM && q == Q)                                  \
+    return cplx ? launch_group<DIM, Q, true> : launch_group<DIM, Q, false>;
+  VL1_G(2, 1) VL1_G(2, 2) VL1_G(2, 3) VL1_G(2, 4) VL1_G(2, 5) VL1_G(2, 6) VL1_G(2, 7) VL1_G(2, 8)
+  VL1_G(3, 1) VL1_G(3, 2) VL1_G(3, 3) VL1_G(3, 4) VL1_G(3, 5)
+#undef VL1_G
+  if (dim == 3 && q == 6 && !cplx) return launch_group<3, 6, false>;
+  return nullptr;
+}
+
 }  // namespace
 }  // namespace vl1
 
@@ -368,4 +693,51 @@ extern "C" int32_t vl1_duffy_table(const vl1_duffy_desc *desc, double *result, v
   }
   cudaFreeAsync(scratch, s);
   return e == cudaSuccess ? VL1_OK : cuda_fail(e, "duffy_entry_kernel launch");
+}
+
+extern "C" int32_t vl1_duffy_table_grouped(const vl1_duffy_desc *desc, int32_t n_groups,
+                                           const int32_t *entry_group,
+                                           const int32_t *group_entry, double *result,
+                                           void *stream) {
+  if (!desc || !result || n_groups < 0) {
+    set_error("vl1_duffy_table_grouped: null descriptor or result, or n_groups < 0");
+    return VL1_E_ARG;
+  }
+  const vl1_duffy_desc &D = *desc;
+  const bool cplx = D.kernel == VL1_DUFFY_HELMHOLTZ2D || D.kernel == VL1_DUFFY_HELMHOLTZ3D;
+  const GroupLaunch launch = group_launch(D.dim, D.q, cplx);
+  // what the group kernel does not take, and every invalid descriptor, is the
+  // per-entry build's
+  if (!launch || n_groups == 0 || !entry_group || !group_entry || D.derivative != 0 ||
+      D.kernel == VL1_DUFFY_PLANE_WAVE || D.kernel < 0 || D.kernel > VL1_DUFFY_POWER_LOG ||
+      D.n_entries < 1 || D.n_reg < 1 || D.n_reg > 128 || D.n_rad < 1 || !(D.extent > 0.0) ||
+      (D.kernel == VL1_DUFFY_POWER && (D.power < 0 || D.power > 64)) ||
+      (D.kernel == VL1_DUFFY_POWER_LOG && (D.power < 1 || D.power > 64)) ||
+      !D.target_points || !D.decomposition_targets || !D.mode_axes || !D.regular_nodes ||
+      !D.regular_weights || !D.radial_nodes || !D.radial_weights || !D.interp_nodes ||
+      !D.interp_weights)
+    return vl1_duffy_table(desc, result, stream);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  DuffyGroupArgs A;
+  A.d = D;
+  A.n_groups = n_groups;
+  A.n_perm = D.dim == 3 ? 6 : 2;
+  A.n_chunks = (1 << D.dim) * A.n_perm;
+  A.group_entry = group_entry;
+  const int cv = cplx ? 2 : 1;
+  const int64_t nm = (int64_t)(D.dim == 3 ? D.q * D.q * D.q : D.q * D.q) * cv;
+  void *scratch = nullptr;
+  cudaError_t e =
+      lib_malloc_async(&scratch, sizeof(double) * (size_t)(n_groups * A.n_chunks * nm), s);
+  if (e != cudaSuccess) return cuda_fail(e, "allocation of the Duffy partial sums");
+  A.part = static_cast<double *>(scratch);
+  e = launch(A, D.max_ctas, s);
+  if (e == cudaSuccess) {
+    const int blocks = (int)std::min<int64_t>(((int64_t)D.n_entries + 127) / 128, 4096);
+    duffy_group_reduce_kernel<<<blocks, 128, 0, s>>>(D, A.part, entry_group, A.n_chunks, cv,
+                                                    result);
+    e = cudaGetLastError();
+  }
+  cudaFreeAsync(scratch, s);
+  return e == cudaSuccess ? VL1_OK : cuda_fail(e, "duffy_group_kernel launch");
 }

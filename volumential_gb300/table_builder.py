@@ -245,8 +245,13 @@ def build_table_values(table, *, radial_rule_name="tanh-sinh-fast", regular_quad
     d.radial_nodes, d.radial_weights = arrs["rx"].data_ptr(), arrs["rw"].data_ptr()
     d.interp_nodes, d.interp_weights = arrs["xi"].data_ptr(), arrs["bw"].data_ptr()
     sh = stream if stream is not None else torch.cuda.current_stream().cuda_stream
-    _lib.check(_lib.lib().vl1_duffy_table(C.byref(d), C.c_void_p(out.data_ptr() if n else 0),
-                                          C.c_void_p(sh)), "vl1_duffy_table")
+    # entries of one (case, target point) share the quadrature's kernel values
+    target = entry_ids // table.n_pairs * table.n_q_points + entry_ids % table.n_q_points
+    _, first, group = np.unique(target, return_index=True, return_inverse=True)
+    grp = dev(np.concatenate([group.ravel(), first]), torch.int32)
+    _lib.check(_lib.lib().vl1_duffy_table_grouped(
+        C.byref(d), len(first), C.c_void_p(grp.data_ptr()), C.c_void_p(grp.data_ptr() + 4 * n),
+        C.c_void_p(out.data_ptr() if n else 0), C.c_void_p(sh)), "vl1_duffy_table_grouped")
     # wait for the build on its stream first: a device-to-host copy queued
     # behind the build kernel holds up other host threads' CUDA calls (a
     # serving loop's launches) until the kernel finishes

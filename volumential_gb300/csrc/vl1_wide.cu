@@ -35,12 +35,14 @@
 // densities, densities over 6 and 200 decades) the relative l2 error is
 // 4e-17 .. 2e-16, the per-box kernel's 1e-16 .. 2e-15.
 //
-// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 248 us here
-// (digits 22 us, tensor-core kernel 220 us, its tensor pipe busy 105 us of
-// them); 3D q = 5, 512,000 points 3,240 and 171 us; 3D q = 3, 110,592 points
-// x 8 right-hand sides 1,530 and 137 us; 2D complex q = 5, 102,400 points 185
-// and 51 us.  Bound: the L2's delivery to all SMs (~30 bytes per SM and clock)
-// of the rows' digits and the table's, close behind it the tensor pipe.
+// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 236 us here
+// (digits 22 us, tensor-core kernel 208 us, its tensor pipe busy 105 us of
+// them); 3D q = 5, 512,000 points 3,240 and 168 us; 3D q = 3, 110,592 points
+// x 8 right-hand sides 1,530 and 131 us; 2D complex q = 5, 102,400 points 185
+// and 46 us.  Bound: shared memory (per unit 120 KB of operand reads and 48 KB
+// of stores, 1,350 of the ~1,750 clocks) and the L2's delivery to all SMs (36
+// KB at ~30 bytes per SM and clock, 1,200), close behind them the tensor pipe
+// (1,176); per work item ~12 us of start and result write.
 //
 // Density rows with an infinite or NaN value (or whose scaled value
 // overflows) cannot be written in fixed point: every target row with such a
@@ -1096,50 +1098,59 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
     const bool tcx = p.d.table_cplx, pair = tcx && p.cc;
     const int cv = tcx ? 2 : 1;
     const int nq = p.d.nq;
-    // one warp per row, lanes over the box's target points
-    for (int row = warp; row < 128; row += R::kThreads / 32) {
-      const int cnt = s_cnt[row];            // 0: empty row
-      const int odd = s_row[row] & 1;        // with complex coefficients: the imaginary part
-      if (pair && odd) continue;             // written with its even partner
-      // rows with non-finite sources are summed below
-      if (s_bad[row] || (p.cc && s_bad[row ^ 1])) continue;
-      const int *mode = p.tr.tmode + s_tbeg[row];
-      const int E = s_E[row] + 2, E2 = s_E[row | 1] + 2;
-      for (int t = lane; t < cnt; t += 32) {
-        int m = s_plain[row] ? t : mode[t];
-        const bool bad_mode = m < 0 || m >= nq;
-        if (bad_mode) {
-          if (chunk == 0) report(p.st, VL1_E_LAYOUT, s_row[row] / p.nv, -1 - t);
-          m = 0;
+    // A warp takes one output row at a time, lanes over the box's target
+    // points, and four values per lane and pass (four rows, or two rows of
+    // real and imaginary parts, or the four products of complex tables with
+    // complex coefficients).
+    constexpr int NW = R::kThreads / 32;
+    const int n_out = pair ? 64 : 128, per = pair ? 1 : (tcx ? 2 : 4);
+    for (int i0 = warp; i0 < n_out; i0 += per * NW) {
+      for (int t = lane; t < nq; t += 32) {
+        double y[4];
+        bool on[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          const int i = i0 + (pair ? 0 : (tcx ? v >> 1 : v)) * NW;
+          const int out = pair ? 2 * i : i;              // the output's row
+          const int row = pair ? out + (v >> 1) : out;   // (odd rows: imaginary coefficients)
+          on[v] = false;
+          y[v] = 0.0;
+          // rows with non-finite sources are summed below
+          if (i >= n_out || t >= s_cnt[out] || s_bad[out] || (p.cc && s_bad[out ^ 1])) continue;
+          const int m = s_plain[out] ? t : p.tr.tmode[s_tbeg[out] + t];
+          const bool bad_mode = m < 0 || m >= nq;
+          if (bad_mode && chunk == 0 && (!tcx || (pair ? v == 0 : (v & 1) == 0)))
+            report(p.st, VL1_E_LAYOUT, s_row[out] / p.nv, -1 - t);
+          const int col = (bad_mode ? 0 : m) * cv - chunk * NCH;
+          if (col < 0 || col >= NCH) continue;
+          on[v] = true;
+          if (bad_mode) continue;
+          const int part = tcx ? v & 1 : 0, at = row * PARK + col + part;
+          y[v] = wide_value(s_S[at], s_L[at], s_E[row] + 2);
+          if (p.wbox) y[v] += s_disp[row][part];
         }
-        const int col = m * cv - chunk * NCH;
-        if (col < 0 || col >= NCH) continue;
-        const int at = row * PARK + col;
-        double re = wide_value(s_S[at], s_L[at], E), im = 0.0;
-        if (tcx) im = wide_value(s_S[at + 1], s_L[at + 1], E);
-        if (p.wbox) {
-          re += s_disp[row][0];
-          if (tcx) im += s_disp[row][1];
+        if (pair) {
+          // (T_re + i T_im)(x_re + i x_im)
+          if (on[0])
+            reinterpret_cast<double2 *>(p.result)[s_out[2 * i0] + t] =
+                make_double2(y[0] - y[3], y[1] + y[2]);
+        } else if (tcx) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (on[2 * j])
+              reinterpret_cast<double2 *>(p.result)[s_out[i0 + j * NW] + t] =
+                  make_double2(y[2 * j], y[2 * j + 1]);
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (on[j]) {
+              const long long o = s_out[i0 + j * NW] + t;
+              if (p.cc)
+                p.result[2 * o + (s_row[i0 + j * NW] & 1)] = y[j];
+              else
+                p.result[o] = y[j];
+            }
         }
-        if (pair) {   // (T_re + i T_im)(x_re + i x_im): the next row holds x_im
-          const int at2 = at + PARK;
-          double re2 = wide_value(s_S[at2], s_L[at2], E2);
-          double im2 = wide_value(s_S[at2 + 1], s_L[at2 + 1], E2);
-          if (p.wbox) {
-            re2 += s_disp[row + 1][0];
-            im2 += s_disp[row + 1][1];
-          }
-          re -= im2;
-          im += re2;
-        }
-        if (bad_mode) re = im = 0.0;
-        const long long o = s_out[row] + t;
-        if (tcx)
-          reinterpret_cast<double2 *>(p.result)[o] = make_double2(re, im);
-        else if (p.cc)
-          p.result[2 * o + odd] = re;
-        else
-          p.result[o] = re;
       }
     }
     if (s_any_bad) {

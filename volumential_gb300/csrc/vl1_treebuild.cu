@@ -238,6 +238,7 @@ struct vl1_tree_builder {
   long long *box_keys = nullptr;
   KeyHash leaf_hash{};
   std::vector<int32_t> level_start;   // host [max_level + 2]
+  cudaStream_t stream = nullptr;      // of the last call: the buffers are freed in its order
 };
 
 namespace {
@@ -245,15 +246,15 @@ namespace {
 template <class T>
 int32_t tb_alloc(vl1_tree_builder *b, T **out, size_t bytes) {
   void *p = nullptr;
-  cudaError_t e = cudaMalloc(&p, bytes ? bytes : 16);
-  if (e != cudaSuccess) return cuda_fail(e, "cudaMalloc(tree builder)");
+  cudaError_t e = lib_malloc_async(&p, bytes ? bytes : 16, b->stream);
+  if (e != cudaSuccess) return cuda_fail(e, "allocation of the tree builder");
   b->bufs.push_back(p);
   *out = static_cast<T *>(p);
   return VL1_OK;
 }
 
 void tb_free(vl1_tree_builder *b) {
-  for (void *p : b->bufs) cudaFree(p);
+  for (void *p : b->bufs) cudaFreeAsync(p, b->stream);
   b->bufs.clear();
 }
 
@@ -263,13 +264,12 @@ int32_t balance(int dim, int32_t *n_leaves, int capacity, uint8_t *levels, int32
   int n = *n_leaves;
   std::vector<void *> tmp;
   auto alloc = [&](void **p, size_t bytes) {
-    cudaError_t e = cudaMalloc(p, bytes ? bytes : 16);
+    cudaError_t e = lib_malloc_async(p, bytes ? bytes : 16, s);
     if (e == cudaSuccess) tmp.push_back(*p);
     return e;
   };
   auto release = [&]() {
-    cudaStreamSynchronize(s);
-    for (void *p : tmp) cudaFree(p);
+    for (void *p : tmp) cudaFreeAsync(p, s);   // after the pass, in stream order
   };
   uint8_t *lv2 = nullptr;
   int32_t *co2 = nullptr, *flag = nullptr, *ctr = nullptr;
@@ -284,7 +284,7 @@ int32_t balance(int dim, int32_t *n_leaves, int capacity, uint8_t *levels, int32
       (e = alloc((void **)&hk, 8 * cap)) != cudaSuccess ||
       (e = alloc((void **)&hv, 4 * cap)) != cudaSuccess) {
     release();
-    return cuda_fail(e, "cudaMalloc(tree balance)");
+    return cuda_fail(e, "allocation of the tree balance");
   }
   KeyHash h{hk, hv, cap - 1};
   for (int pass = 0; pass < 64; ++pass) {
@@ -360,6 +360,7 @@ extern "C" int32_t vl1_tree_build_begin(int32_t dim, int32_t q, int32_t n_leaves
   b->q = q;
   b->n_leaves = n_leaves;
   b->root_extent = root_extent;
+  b->stream = s;
   for (int a = 0; a < dim; ++a) b->root_vertex[a] = root_vertex[a];
   auto fail = [&](int32_t st) {
     cudaStreamSynchronize(s);
@@ -462,6 +463,7 @@ extern "C" int32_t vl1_tree_build_fill(vl1_tree_builder *b, const double *ref_no
     return VL1_E_ARG;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  b->stream = s;
   const int nb = b->nboxes;
   int32_t *iota = nullptr, *n_sel = nullptr;
   int32_t st;

@@ -469,6 +469,12 @@ typedef struct {
   int64_t workspace_bytes;
 } vl1_csr_desc;
 
+/* Bounds of a tree view's indices: CSR starts run from 0 to nnz, box ids lie in
+ * [0, nboxes), the particle ranges of boxes with points in [0, n_particles),
+ * counts are not negative and levels at most 60.  VL1_E_LAYOUT if not.  One
+ * kernel; synchronises the stream. */
+int32_t vl1_tree_check(const vl1_tree_view *tree, int64_t nnz, void *stream);
+
 int64_t vl1_list1_csr_workspace_bytes(int32_t n_leaves);
 int32_t vl1_list1_csr(const vl1_csr_desc *desc, int64_t *nnz, void *stream);
 

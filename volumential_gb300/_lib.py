@@ -212,6 +212,7 @@ SIGNATURES = {
     "vl1_duffy_table_grouped": (C.c_int32, [C.POINTER(DuffyDesc), C.c_int32, C.c_void_p,
                                             C.c_void_p, C.c_void_p, C.c_void_p]),
     "vl1_split_correction": (C.c_int32, [C.POINTER(SplitDesc), C.c_void_p]),
+    "vl1_tree_check": (C.c_int32, [C.POINTER(TreeView), C.c_int64, C.c_void_p]),
     "vl1_list1_csr_workspace_bytes": (C.c_int64, [C.c_int32]),
     "vl1_tree_balance": (C.c_int32, [C.c_int32, C.POINTER(C.c_int32), C.c_int32, C.c_void_p,
                                      C.c_void_p, C.c_void_p]),

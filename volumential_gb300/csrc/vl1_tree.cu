@@ -19,6 +19,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "vl1_hash.cuh"
@@ -376,5 +377,72 @@ extern "C" int32_t vl1_list1_csr(const vl1_csr_desc *desc, int64_t *nnz, void *s
     return VL1_E_ARG;
   }
   *nnz = host[1];
+  return VL1_OK;
+}
+
+// ---- Bounds of every index that the kernels load through (tree arrays given
+// by a caller): one kernel and one read-back.
+
+namespace vl1 {
+namespace {
+
+__global__ void tree_check_kernel(const vl1_tree_view T, int64_t nnz, int *bad) {
+  const int64_t n = (int64_t)gridDim.x * blockDim.x;
+  const int64_t i0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int n_tb = T.n_target_boxes;
+  const int64_t nb = T.nboxes, np = T.n_particles;
+  bool fault = false;
+  if (n_tb > 0) {
+    if (i0 == 0)
+      fault = T.neighbor_source_boxes_starts[0] != 0 ||
+              T.neighbor_source_boxes_starts[n_tb] != nnz;
+    for (int64_t i = i0; i < n_tb; i += n) {
+      const int b = T.target_boxes[i];
+      fault = fault || b < 0 || b >= nb ||
+              T.neighbor_source_boxes_starts[i + 1] < T.neighbor_source_boxes_starts[i];
+    }
+  }
+  for (int64_t i = i0; i < nnz; i += n) {
+    const int b = T.neighbor_source_boxes_lists[i];
+    fault = fault || b < 0 || b >= nb;
+  }
+  for (int64_t i = i0; i < nb; i += n) {
+    const int64_t ss = T.box_source_starts[i], sc = T.box_source_counts_nonchild[i];
+    const int64_t ts = T.box_target_starts[i], tc = T.box_target_counts_nonchild[i];
+    fault = fault || T.box_levels[i] > 60 || sc < 0 || tc < 0 ||
+            (sc > 0 && (ss < 0 || ss + sc > np)) || (tc > 0 && (ts < 0 || ts + tc > np));
+  }
+  if (fault) *bad = 1;
+}
+
+}  // namespace
+}  // namespace vl1
+
+extern "C" int32_t vl1_tree_check(const vl1_tree_view *tree, int64_t nnz, void *stream) {
+  if (!tree || tree->n_target_boxes < 0 || nnz < 0) {
+    set_error("vl1_tree_check: null tree or negative sizes");
+    return VL1_E_ARG;
+  }
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  void *flag = nullptr;
+  int host = 0;
+  cudaError_t e = lib_malloc_async(&flag, 16, s);
+  if (e != cudaSuccess) return cuda_fail(e, "vl1_tree_check: allocation");
+  e = cudaMemsetAsync(flag, 0, 4, s);
+  if (e == cudaSuccess) {
+    const int64_t n = std::max<int64_t>(std::max<int64_t>(tree->n_target_boxes, nnz),
+                                        std::max<int64_t>(tree->nboxes, 1));
+    tree_check_kernel<<<(unsigned)std::min<int64_t>((n + 255) / 256, 152 * 8), 256, 0, s>>>(
+        *tree, nnz, static_cast<int *>(flag));
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&host, flag, 4, cudaMemcpyDeviceToHost, s);
+  cudaFreeAsync(flag, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (e != cudaSuccess) return cuda_fail(e, "vl1_tree_check");
+  if (host) {
+    set_error("invalid list-1 tree arrays");
+    return VL1_E_LAYOUT;
+  }
   return VL1_OK;
 }

@@ -156,7 +156,7 @@ def _tree_view_from_arrays(*, target_boxes, neighbor_source_boxes_starts,
     v.n_particles = int(keep["tmode"].numel())
     v.nboxes = int(keep["levels"].numel())
     v.root_extent = float(root_extent)
-    validate_tree_arrays(keep, dim=int(keep["centers"].shape[0]))
+    validate_tree_arrays(keep, dim=int(keep["centers"].shape[0]), view=v)
     return v, keep
 
 
@@ -167,12 +167,14 @@ def _token(t):
     return (t.data_ptr(), t._version, tuple(t.shape), str(t.dtype))
 
 
-def validate_tree_arrays(keep, dim):
+def validate_tree_arrays(keep, dim, view):
     """Bounds of every index the kernels load through (cached per array set).
 
     The kernels check case codes, box counts against q^dim and mode ids
-    themselves; everything else that addresses memory is checked here, so that
-    an invalid tree raises on the host and never reaches a device load.
+    themselves; everything else that addresses memory is checked here
+    (``vl1_tree_check``, one kernel; as some twenty tensor operations the
+    checks took 0.7 ms of a first call), so that an invalid tree raises on the
+    host and never reaches a device load.
     """
     key = tuple(_token(t) for t in keep.values())
     if key in _validated:
@@ -181,9 +183,6 @@ def validate_tree_arrays(keep, dim):
     torch = require_cuda()
     nboxes = int(keep["levels"].numel())
     npart = int(keep["tmode"].numel())
-    ntb = int(keep["target_boxes"].numel())
-    st = keep["starts"]
-    ls = keep["lists"]
     if dim not in (2, 3):
         raise ValueError(f"box_centers must have 2 or 3 rows, got {dim}")
     if int(keep["smode"].numel()) != npart:
@@ -194,26 +193,15 @@ def validate_tree_arrays(keep, dim):
             raise ValueError(f"box array {name} has fewer than nboxes={nboxes} entries")
     if int(keep["centers"].shape[1]) < nboxes:
         raise ValueError("box_centers has fewer columns than boxes")
-    checks = []
-    if ntb:
-        checks += [st[0] != 0, st[-1] != ls.numel(), (st[1:] < st[:-1]).any(),
-                   keep["target_boxes"].min() < 0, keep["target_boxes"].max() >= nboxes]
-    if ls.numel():
-        checks += [ls.min() < 0, ls.max() >= nboxes]
-    if nboxes:
-        lv = keep["levels"]
-        checks += [lv.max() > 60]
-        for s_name, c_name in (("src_starts", "src_counts"), ("tgt_starts", "tgt_counts")):
-            s = keep[s_name][:nboxes].to(torch.int64)
-            c = keep[c_name][:nboxes].to(torch.int64)
-            used = c > 0
-            checks += [(used & (s < 0)).any(), (used & (s + c > npart)).any(), (c < 0).any()]
-    if checks and bool(torch.stack([torch.as_tensor(x, device="cuda").reshape(())
-                                    for x in checks]).any()):
+    lib = _lib.lib()
+    st = lib.vl1_tree_check(C.byref(view), int(keep["lists"].numel()),
+                            C.c_void_p(torch.cuda.current_stream().cuda_stream))
+    if st == _lib.VL1_E_LAYOUT:
         raise ValueError(
             "invalid list-1 tree arrays: CSR starts must run from 0 to len(lists), box "
             "ids must lie in [0, nboxes), box particle ranges in [0, n_particles) and "
             "levels below 61")
+    _lib.check(st, "vl1_tree_check")
     # the entry holds the validated tensors, so their memory cannot be reused
     # by other arrays while the key is cached
     _validated[key] = dict(keep)

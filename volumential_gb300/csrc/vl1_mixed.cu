@@ -146,11 +146,9 @@ __global__ void build_adig_kernel(DevDesc d, MixedGeom g, __half *adig, int a_ex
     const int kc = (int)(q % g.n_kc);
     const int key = (int)(q / g.n_kc);
     const int s = kc * g.kc + k;
-    int t = n, part = 0;
-    if (d.table_cplx && n >= d.nq) {
-      t = n - d.nq;
-      part = 1;
-    }
+    // complex tables: real and imaginary parts of a target point in
+    // neighbouring columns, as in the result
+    const int t = d.table_cplx ? n >> 1 : n, part = d.table_cplx ? n & 1 : 0;
     double v = 0.0;
     if (s < d.nq && t < d.nq) {
       const int64_t bi = ((int64_t)key * d.nq + s) * d.nq + t;
@@ -613,6 +611,27 @@ __device__ __forceinline__ long long f32_scaled_to_i64(float x, float two_s) {
   return ((long long)__float2int_rz(h) << 31) + (long long)__float2int_rn(rem);
 }
 
+// The same for |x| * 2^S <= 2^44, plus the constant kTailBitsConst, in four
+// FP32 operations and no conversion: h = x * 2^(S - 22) rounded to an integer
+// by adding 1.5 * 2^23, whose raw bits are then kMagicBits + h; the remainder
+// x * 2^S - h * 2^22 (exact, at most 2^21) the same way.
+constexpr unsigned long long kTailBitsConst =
+    (unsigned long long)kMagicBits * ((1ull << 22) + 1ull);
+template <int S>
+__device__ __forceinline__ unsigned long long tail_bits(float x) {
+  constexpr float up = (float)(1 << (22 - S));
+  const float hm = __fmaf_rn(x, 1.0f / up, kMagic);
+  const float rem = __fmaf_rn(-(hm - kMagic), up, x);            // exact
+  const float lm = __fmaf_rn(rem, (float)(1 << S), kMagic);
+  return (unsigned long long)__float_as_uint(hm) * (1ull << 22) +
+         (unsigned long long)__float_as_uint(lm);
+}
+// Source points of an item up to which its tails take tail_bits: a tail adds
+// at most 4 products of 2^14 per source point, so the bound above holds up to
+// 2^20 points; the line is drawn where the conversions of the general form
+// are lost in the item's products (512 units of ~1500 clocks).
+constexpr int kSmallTailK = 1 << 14;
+
 // ---------------------------------------------------------- main kernel
 
 struct MixedParams {
@@ -641,19 +660,19 @@ struct MixedParams {
 };
 
 // Warp roles of mixed_kernel (warp index w):
-//   w <  8      producers: per pipeline unit, warp w copies the density digit
-//               planes of tile rows 16w .. 16w+15 into the unit's stage with
+//   w <  4      producers: per pipeline unit, warp w copies the density digit
+//               planes of tile rows 32w .. 32w+31 into the unit's stage with
 //               cp.async (16-byte pieces straight into the swizzled K-major
 //               layout, zero-filled for rows without a source box); each
 //               lane's arrival on xfull[stage] fires when its copies land
 //               (cp.async.mbarrier.arrive), so the producers never wait for
-//               data, only for a free stage.  Eight warps keep enough
-//               requests in flight to cover the L2 latency of these scattered
-//               rows.
-//   w == 8      table loader (one lane): the five table digit tiles of the
-//               unit's key by bulk copies (TMA), counted on afull[stage]
-//   w == 9      tensor-core issuer (one lane)
-//   w >= 10     readout: TMEM lane quadrant w % 4, RC columns each
+//               data, only for a free stage.  They also put out where each
+//               row's results go (rfull).
+//   w == 4      loader (one lane): the work items, and the five table digit
+//               tiles of the unit's key by bulk copies (TMA), counted on
+//               afull[stage]
+//   w == 5      tensor-core issuer
+//   w >= 6      readout: TMEM lane quadrant w % 4, 16 columns each
 // Pipeline unit = (key, K chunk of kc <= 32 source points); a "round" = the
 // consecutive units (of one or more keys) that share an exact accumulation
 // (K <= kRoundK = 128).  Exact
@@ -667,24 +686,29 @@ struct MixedParams {
 // only, R = X4 + X5 / 256 rounded to FP16 (11 significant bits: the density
 // keeps ~2^-36 of its rhs's scale in the tails, far below the 2^-24 weight of
 // the tails; the exact diagonals use X1..X3 only).
-// Roles and pipeline depth per column chunk width.  64 output columns: 8
-// producer warps, 4 stages, one CTA per SM (214 KB of shared memory, all 512
-// TMEM columns).  16 or 32 columns: 4 producer warps, 2 stages and two CTAs
-// per SM (at most 91 KB and 256 TMEM columns each, <= 73 registers per
-// thread), so that one CTA's pipeline fill, readout and result write overlap
-// the other's tensor-core work.
+// Roles and pipeline depth per column chunk width.  64 output columns: 4
+// producer warps, 3 stages, one CTA per SM (205 KB of shared memory, all 512
+// TMEM columns; with 8 producer warps the readout warps' registers spill and
+// the kernel is 3 to 6 % slower).  16 or 32 columns: 4 producer warps, 2
+// stages and two CTAs per SM (at most 113 KB and 256 TMEM columns each, <= 72
+// registers per thread).
 template <int NCH>
 struct MixedRoles {
-  static constexpr int kProducers = NCH >= 64 ? 8 : 4;
+  static constexpr int kProducers = 4;
   static constexpr int kRowsPerProducer = 128 / kProducers;
   static constexpr int kLoader = kProducers;
   static constexpr int kMma = kProducers + 1;
   static constexpr int kRead0 = kProducers + 2;
-  static constexpr int kStages = NCH >= 64 ? 4 : 2;
   static constexpr int kCtasPerSm = NCH >= 64 ? 1 : 2;
   static constexpr int kThreads = 32 * (kRead0 + 4 * (NCH / 16));
 };
+// pipeline stages: as many as fit beside the readout warps' slices
+__host__ __device__ constexpr int mixed_stages(int nch, int kc) {
+  return nch >= 64 ? (kc > 16 ? 3 : 4) : 2;
+}
 constexpr int kMaxStages = 4;
+// a readout warp's slice of shared memory: 32 rows of 8 (+ 1) outputs
+constexpr int kParkBytes = 32 * 9 * 8;
 // source points of one exact round: with balanced digits (|digit| <= 128) a
 // diagonal sum over 128 points is at most 2^21 (i + j = 2), 2^22 (i + j = 3)
 // and 3 * 2^21 (i + j = 4), all exact in FP32
@@ -697,12 +721,30 @@ constexpr int kSplitPoison = 1 << 16;
 // in a layout that leaves room for per-piece counts)
 constexpr int kSplitCounterStride = 16;
 
+// records of work items between the loader and the other roles
+constexpr int kWorkSlots = 4;
+enum WorkKind : int32_t { kWorkRun = 0, kWorkEnd = 1, kWorkSkip = 2 };
+struct WorkRec {
+  int32_t tile, k0, k1, chunk;
+  int32_t split, part, nparts, slot;
+  int32_t problem, kind;
+};
+// where a tile row's outputs go: first result value << 16 | number of values
+// (0: none), and the exponent of one unit of its sums
+struct RowOut {
+  long long where;
+  int32_t ex, row;   // row: the schedule's row number (-1: none)
+};
+
 struct Barriers {
   uint64_t xfull[kMaxStages];   // every producer lane's density copies have landed
   uint64_t afull[kMaxStages];   // the table digit tiles have landed
   uint64_t empty[kMaxStages];
   uint64_t accf[2];
   uint64_t acce[2];
+  uint64_t taile;            // the item's tail accumulators have been read
+  uint64_t wfull[kWorkSlots], wempty[kWorkSlots];   // work item records
+  uint64_t rfull[kWorkSlots];   // the item's row data
   uint64_t drain;            // after an abort: every issued MMA has completed
 };
 
@@ -713,10 +755,10 @@ struct BatchItem {
   vl1_mixed_item item;
 };
 struct BatchLaunch {
-  const MixedParams *probs;   // [n_problems]
-  const BatchItem *items;     // [n_items], launched in this order
-  int n_items;
-  int *queue;                 // next item to take; zero before the launch
+  const MixedParams *probs;   // [n_problems] (several problems)
+  const BatchItem *items;     // [n_items], taken in this order (several problems)
+  unsigned long long n_items; // work items, column chunks counted
+  unsigned long long *queue;  // items taken beyond each CTA's first; zero before the launch
   uint32_t wait_limit_us;     // as MixedParams::wait_limit_us (persistent launches)
   int32_t withhold_arrival;   // as MixedParams::withhold_arrival
 };
@@ -731,20 +773,134 @@ struct MmaGroup {
 // R = X4 + X5 / 256: R A1 = X4 A1 + X5 A1 / 256 covers (4, 1) and (5, 1),
 // R A2 covers (4, 2) (plus the negligible (5, 2) / 256)
 constexpr int kGroupCount = 7;
+constexpr int kExactGroups = 3;   // the exact ones come first
 __device__ constexpr MmaGroup kGroups[kGroupCount] = {{1, 1, 3, 1}, {2, 1, 2, 1}, {3, 1, 1, 1},
                                                       {1, 4, 2, 0}, {2, 3, 2, 0}, {3, 2, 2, 0},
                                                       {4, 1, 2, 0}};
 
-// MULTI == false: one work item per CTA (blockIdx.x; column chunk blockIdx.y)
-// of the single problem p1.  MULTI == true: a persistent launch over the
-// items of several problems, each CTA taking the next item from bl.queue; the
-// item's problem parameters are copied to shared memory, and the pipeline
-// barriers keep their phases across items (CTA-wide unit / round counters).
+// The checked record of work index w.
+template <int NCH, bool MULTI>
+__device__ WorkRec load_work(const MixedParams &p1, const BatchLaunch &bl,
+                             unsigned long long w) {
+  WorkRec r{};
+  vl1_mixed_item item;
+  int wi;
+  if (MULTI) {
+    const BatchItem bi = bl.items[w];
+    wi = (int)w;
+    r.problem = bi.problem;
+    r.chunk = bi.chunk;
+    item = bi.item;
+  } else {
+    const vl1_mixed_schedule &sc = p1.sched;
+    const unsigned n_x = (unsigned)(sc.n_items > 0 ? sc.n_items : sc.n_tiles);
+    r.chunk = (int)(w / n_x);
+    wi = (int)(w - (unsigned long long)r.chunk * n_x);
+    if (sc.n_items > 0) {
+      item = sc.items[wi];
+    } else {
+      item.tile = wi;
+      item.key_begin = sc.tile_key_start[wi];
+      item.key_end = sc.tile_key_start[wi + 1];
+      item.split = -1;
+      item.part = 0;
+      item.nparts = 1;
+      item.slot = -1;
+    }
+  }
+  const MixedParams &p = MULTI ? bl.probs[r.problem] : p1;
+  bool bad = item.tile < 0 || item.tile >= p.sched.n_tiles || r.chunk < 0 ||
+             r.chunk >= p.g.np / NCH;
+  if (!bad) {
+    const int t0 = p.sched.tile_key_start[item.tile], t1 = p.sched.tile_key_start[item.tile + 1];
+    bad = item.key_begin < t0 || item.key_end > t1 || item.key_begin > item.key_end;
+  }
+  if (item.split >= 0)
+    bad = bad || item.split >= p.sched.n_splits || item.part < 0 ||
+          item.part >= item.nparts || item.nparts >= kSplitPoison ||
+          item.slot - item.part < 0 ||
+          item.slot - item.part + item.nparts > p.sched.n_slots;
+  else
+    bad = bad || item.split != -1;
+  r.kind = bad ? kWorkSkip : kWorkRun;
+  if (bad) {
+    report(p.st, VL1_E_ARG, wi, -1);
+    return r;
+  }
+  r.tile = item.tile;
+  r.k0 = item.key_begin;
+  r.k1 = item.key_end;
+  r.split = item.split;
+  r.part = item.part;
+  r.nparts = item.nparts;
+  r.slot = item.slot;
+  return r;
+}
+
+// After an abort, one thread: report work index w as timed out, or count the
+// part of a split tile that no CTA will run (the tile's last arrival clears
+// what its other parts added).
+template <int NCH, bool MULTI>
+__device__ void abandon_work(const MixedParams &p1, const BatchLaunch &bl, unsigned long long w,
+                             bool report_it) {
+  const WorkRec r = load_work<NCH, MULTI>(p1, bl, w);
+  const MixedParams &p = MULTI ? bl.probs[r.problem] : p1;
+  if (report_it) {
+    report(p.st, VL1_E_TIMEOUT, r.tile, r.chunk);
+    return;
+  }
+  if (r.kind != kWorkRun || r.split < 0) return;
+  const int n_chunks = p.g.np / NCH;
+  int *ctr = p.sched.split_counters +
+             ((int64_t)r.split * n_chunks + r.chunk) * kSplitCounterStride;
+  const int done = atomicAdd(ctr, kSplitPoison + 1) + kSplitPoison + 1;
+  if ((done & (kSplitPoison - 1)) != r.nparts) return;
+  unsigned long long *acc = reinterpret_cast<unsigned long long *>(
+      static_cast<uint8_t *>(p.sched.split_partials) +
+      ((int64_t)(r.slot - r.part) * n_chunks + r.chunk) * (128 * NCH * 8));
+  for (int i = 0; i < 128 * NCH; ++i) acc[i] = 0ull;
+  *ctr = 0;
+}
+
+// barrier among the readout warps
+template <int THREADS>
+__device__ __forceinline__ void readout_barrier() {
+  asm volatile("bar.sync 1, %0;" ::"n"(THREADS) : "memory");
+}
+
+// A persistent launch: each CTA runs its blockIdx'th work item and then takes
+// the next one from bl.queue until none is left.  MULTI == false: the items of
+// the single problem p1 (work index w: item w % n_x, column chunk w / n_x).
+// MULTI == true: a list of items of several problems, whose parameters are
+// read from global memory.
+//
+// The roles walk the items on their own, so that an item's pipeline fill and
+// its result write overlap the products of its neighbours: the loader takes
+// an item's number from the queue while it still issues the item before, puts
+// the checked record into a ring of kWorkSlots entries, and every other role
+// picks it up there when it gets to it.  Stages, exact buffers and their
+// barrier phases run on across items; the one hand-over between items is the
+// tail accumulators (d = 5, 6), which the next item's first unit may only
+// overwrite once the readout warps have taken them (taile).  The readout
+// warps hold a tile's sums in registers, round them there and write them
+// through a private slice of shared memory (64 consecutive bytes of a row per
+// eight lanes), so no other role waits for the results.
+//
+// What bounds it: the copies of the digits from L2 (32 + 20 KB a unit of 64
+// columns) at ~30 bytes per clock and SM with every SM at it, 1750 clocks a
+// unit; the products' own operand reads and the copies' stores take 1300
+// clocks of shared memory.  With one item per CTA the fill (barriers, TMEM,
+// four dependent loads) and the results (24,000 clocks, of which the branchy
+// rounding took most) stood between the items' pipelines.  Before and after:
+// 2D Helmholtz q = 5, 4096 boxes, 256 right-hand sides (8192 items of 9
+// units) 1013 -> 573 us; uniform 3D level 5 q = 4 106 -> 95 us; 3D level 4
+// q = 5 65 -> 59 us; adaptive 3D q = 4 with two items of 46
+// units per SM 98.5 -> 95.8 us.
 template <int NCH, int KC, bool MULTI>
 __global__ void __launch_bounds__(MixedRoles<NCH>::kThreads, MixedRoles<NCH>::kCtasPerSm)
 mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ BatchLaunch bl) {
   using Roles = MixedRoles<NCH>;
-  constexpr int kStages = Roles::kStages;
+  constexpr int kStages = mixed_stages(NCH, KC);
   constexpr int kProducerWarps = Roles::kProducers;
   constexpr int kRowsPerProducer = Roles::kRowsPerProducer;
   constexpr int kLoaderWarp = Roles::kLoader;
@@ -758,9 +914,6 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
   constexpr uint32_t ABYTES = (uint32_t)NCH * KC * 2u;   // one digit plane of the table
   constexpr uint32_t STAGE_BYTES = kXPlanes * XBYTES + kDigits * ABYTES;
   constexpr uint32_t ROW_BYTES = KC * 2u;
-  // parked int64 sums: rows padded by one value, so that the 32 lanes of a
-  // readout warp (32 rows) store one column into distinct banks
-  constexpr int PARK_STRIDE = NCH + 1;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // swizzle atoms need a 1024-byte aligned base (the launch adds 1 KiB slack)
   uint8_t *smem = reinterpret_cast<uint8_t *>(
@@ -768,10 +921,11 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
   __shared__ Barriers bars;
   __shared__ uint32_t tmem_base;
   __shared__ volatile int s_abort;
-  __shared__ int s_rows[128];
-  __shared__ __align__(16) MixedParams s_p;   // MULTI: the current item's problem
-  __shared__ int s_next;
-  const MixedParams &p = MULTI ? s_p : p1;
+  __shared__ WorkRec s_rec[kWorkSlots];
+  __shared__ RowOut s_out[kWorkSlots][128];
+  __shared__ unsigned long long s_claim[2 * kWorkSlots];   // work indexes, by ordinal
+  __shared__ int s_nclaimed, s_ndone;   // items taken / items whose split count is settled
+  __shared__ int s_go[2], s_last, s_poison;
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -779,8 +933,8 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
   const uint32_t lim = MULTI ? bl.wait_limit_us : p1.wait_limit_us;
   const uint32_t limit_us = lim ? lim : kWaitLimitUs;
   // test hook: this CTA's producer warp 0 withholds its first arrival
-  const bool withhold = (MULTI ? bl.withhold_arrival : p1.withhold_arrival) != 0 &&
-                        blockIdx.x == 0 && blockIdx.y == 0;
+  const bool withhold =
+      (MULTI ? bl.withhold_arrival : p1.withhold_arrival) != 0 && blockIdx.x == 0;
 
   if (tid == 0) {
     tc::mbar_init(&bars.drain, 1);
@@ -793,8 +947,15 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
       tc::mbar_init(&bars.accf[b], 1);
       tc::mbar_init(&bars.acce[b], NREAD);
     }
+    tc::mbar_init(&bars.taile, NREAD);
+    for (int b = 0; b < kWorkSlots; ++b) {
+      tc::mbar_init(&bars.wfull[b], 1);
+      tc::mbar_init(&bars.wempty[b], kProducerWarps + 1 + NREAD);
+      tc::mbar_init(&bars.rfull[b], kProducerWarps);
+    }
     tc::fence_mbar_init();
     s_abort = 0;
+    s_nclaimed = s_ndone = 0;
   }
   if (warp == kMmaWarp) {
     tc::tmem_alloc(&tmem_base, COLS);
@@ -804,108 +965,12 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
   __syncthreads();
   tc::tc_fence_after();
   const uint32_t tbase = tmem_base;
-
-  // pipeline units and K rounds this CTA has run in earlier items (stage and
-  // buffer phases continue across items)
-  int ubase = 0, rbase = 0;
-  for (int pass = 0;; ++pass) {
-  int wi;
-  if (MULTI) {
-    if (tid == 0) s_next = s_abort ? bl.n_items : atomicAdd(bl.queue, 1);
-    __syncthreads();
-    wi = s_next;
-    if (wi >= bl.n_items) break;
-    const uint64_t *src = reinterpret_cast<const uint64_t *>(bl.probs + bl.items[wi].problem);
-    for (int i = tid; i < (int)(sizeof(MixedParams) / 8); i += blockDim.x)
-      reinterpret_cast<uint64_t *>(&s_p)[i] = src[i];
-    __syncthreads();
-  } else {
-    if (pass > 0) break;
-    wi = blockIdx.x;
-  }
-  const int chunk = MULTI ? bl.items[wi].chunk : blockIdx.y;
-  const int n_chunks = p.g.np / NCH;
-
-  // this CTA's work item: a tile, or a key range of a split tile
-  vl1_mixed_item item;
-  if (MULTI) {
-    item = bl.items[wi].item;
-  } else if (p.sched.n_items > 0) {
-    item = p.sched.items[wi];
-  } else {
-    item.tile = wi;
-    item.key_begin = p.sched.tile_key_start[wi];
-    item.key_end = p.sched.tile_key_start[wi + 1];
-    item.split = -1;
-    item.part = 0;
-    item.nparts = 1;
-    item.slot = -1;
-  }
-  const int tile = item.tile;
-  {
-    bool bad = tile < 0 || tile >= p.sched.n_tiles || chunk < 0 || chunk >= n_chunks;
-    if (!bad) {
-      const int t0 = p.sched.tile_key_start[tile], t1 = p.sched.tile_key_start[tile + 1];
-      bad = item.key_begin < t0 || item.key_end > t1 || item.key_begin > item.key_end;
-    }
-    if (item.split >= 0)
-      bad = bad || item.split >= p.sched.n_splits || item.part < 0 ||
-            item.part >= item.nparts || item.nparts >= kSplitPoison ||
-            item.slot - item.part < 0 ||
-            item.slot - item.part + item.nparts > p.sched.n_slots;
-    else
-      bad = bad || item.split != -1;
-    if (bad) {   // uniform across the CTA
-      if (tid == 0) report(p.st, VL1_E_ARG, wi, -1);
-      __syncthreads();
-      continue;
-    }
-  }
-
-  const int k0 = item.key_begin, k1 = item.key_end;
-  const int n_keys = k1 - k0;
-  // units of the item, and exact rounds of up to kRoundK source points (a
-  // round may span several keys: the exact diagonals of every key of a tile
-  // row are in the same units)
-  const int n_units = n_keys * p.g.n_kc;
   constexpr int upr = kRoundK / KC;   // units per round
-  const int n_rounds = (n_units + upr - 1) / upr;
-
-  // the rows of the tile, and (for the result write at the end of the item,
-  // loaded now so that their latency hides behind the pipeline) each row's
-  // first result index, point count and output exponent
-  __shared__ long long s_obase[128];   // result index of the row's first target point
-  __shared__ int s_ocnt[128];          // target points of the row's box (0: empty row)
-  __shared__ int s_oexp[128];          // an output is (parked sum) * 2^s_oexp
-  if (tid < 128) {
-    int v = p.sched.tile_rows[(int64_t)tile * 128 + tid];
-    if (v >= (int64_t)p.n_tgt_boxes * p.nrhs) {
-      report(p.st, VL1_E_ARG, tile, tid);
-      v = -1;
-    }
-    s_rows[tid] = v;
-    int cnt = 0, ex = 0;
-    long long ob = 0;
-    if (v >= 0) {
-      const int j = v / p.nrhs, r = v - (v / p.nrhs) * p.nrhs;
-      const int tbox = p.target_boxes[j];
-      cnt = min(p.tgt_counts[tbox], p.d.nq);
-      ob = (long long)r * p.n_particles + p.tgt_starts[tbox];
-      // table values are m_a 2^(a_exp - kFixedBits), densities
-      // m_x 2^(e - kXFixedBits) with e the scale exponent of the rhs; the
-      // parked sums count units of 2^32 of m_a m_x
-      ex = p.a_exp + (p.x_exp[r] - kExpBias) - (kFixedBits + kXFixedBits) + 32;
-    }
-    s_obase[tid] = ob;
-    s_ocnt[tid] = cnt;
-    s_oexp[tid] = ex;
-  }
-  __syncthreads();
 
   if (warp < kProducerWarps) {
     // ------------------------------------------------------------ producers
     // Per unit: wait for the unit's stage to be free, then copy the four
-    // digit planes of this warp's 16 rows (8 * KC bytes of a row: PPR 16-byte
+    // digit planes of this warp's rows (8 * KC bytes of a row: PPR 16-byte
     // pieces of 8 values of one plane) into the stage's swizzled K-major
     // planes with cp.async; each lane's arrival on xfull fires when its own
     // copies have landed.  A warp none of whose rows has a source box in the
@@ -914,191 +979,347 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
     constexpr int PPR = kXPlanes * PPP;                  // pieces per row and unit
     constexpr int NIT = kRowsPerProducer * PPR / 32;     // pieces per lane and unit
     static_assert(kRowsPerProducer * PPR % 32 == 0, "whole pieces per lane");
-    const int64_t row_halves = (int64_t)p.g.kp * kXPlanes;   // FP16 values per density row
+    // Piece it * 32 + lane of the warp's rows: row it * (32 / PPR) + lane / PPR,
+    // 16-byte piece q = lane % PPR of the row's 8 * KC contiguous bytes (plane
+    // q / PPP, values 8 (q % PPP) .. + 7 of the K chunk).  A warp's rows start
+    // at a multiple of 8 and 32 / PPR rows are 128 bytes of a plane, so the
+    // swizzled position is linear in `it` but for the piece's bits 4.. , which
+    // are xored with it.
+    const int q = lane % PPR;
+    const uint32_t dst0 = tc::smem_addr(smem) + (uint32_t)(q / PPP) * XBYTES +
+                          (uint32_t)(warp * kRowsPerProducer) * ROW_BYTES +
+                          (uint32_t)(lane / PPR) * ROW_BYTES + ((uint32_t)(q % PPP) << 4);
     // lanes < kRowsPerProducer hold the density row of tile row my_row,
     // fetched one key ahead
     const int my_row = kRowsPerProducer * warp + (lane % kRowsPerProducer);
-    int nkey = 0, nxr = -1;
-    if (n_keys > 0) {
-      nkey = p.sched.key_ids[k0];
-      nxr = p.sched.key_xrow[(int64_t)k0 * 128 + my_row];
-    }
-    // bit s: this warp's rows of stage s hold zero planes (the stages are
-    // overwritten by the parked sums at the end of an item, so the bits
-    // start clear per item)
+    // bit s: this warp's rows of stage s hold zero planes
     uint32_t zero_stages = 0;
-    int u = 0;
+    int s = 0;
+    uint32_t use = 0;       // units this CTA has put into stage s before
     bool aborted = false;
-    for (int kidx = k0; kidx < k1 && !aborted; ++kidx) {
-      const int key = nkey;
-      int xr_lane = nxr;
-      if (kidx + 1 < k1) {
-        nkey = p.sched.key_ids[kidx + 1];
-        nxr = p.sched.key_xrow[(int64_t)(kidx + 1) * 128 + my_row];
-      }
-      const bool key_ok = key >= 0 && key < p.d.n_tables * p.d.n_cases;
-      if (!key_ok) {
-        if (warp == 0 && lane == 0) report(p.st, VL1_E_ARG, tile, kidx);
-        xr_lane = -1;
-      }
-      if (xr_lane >= p.n_xrows) {
-        report(p.st, VL1_E_ARG, tile, my_row);
-        xr_lane = -1;
-      }
-      const bool key_empty =
-          __ballot_sync(0xffffffffu, lane < kRowsPerProducer && xr_lane >= 0) == 0u;
-      for (int kc = 0; kc < p.g.n_kc; ++kc, ++u) {
-        const int s = (ubase + u) % kStages;
-        const int use = (ubase + u) / kStages;
-        if (use > 0 &&
-            !wait_or_abort(&bars.empty[s], (use - 1) & 1, &s_abort, limit_us, true)) {
-          aborted = true;
-          break;
-        }
-        uint8_t *xs = smem + (size_t)s * STAGE_BYTES;
-        const bool hold = withhold && warp == 0 && ubase + u == 0;
-        if (key_empty) {
-          // no source rows: zero planes (rows 16w .. 16w + 15 of a swizzled
-          // K-major plane are one contiguous block), written once per stage
-          if (!((zero_stages >> s) & 1u)) {
-            constexpr int BLK = kRowsPerProducer * (int)ROW_BYTES;
-#pragma unroll
-            for (int dg = 0; dg < kXPlanes; ++dg)
-              for (int o = lane * 16; o < BLK; o += 32 * 16)
-                *reinterpret_cast<uint4 *>(xs + dg * XBYTES + warp * BLK + o) =
-                    make_uint4(0u, 0u, 0u, 0u);
-            zero_stages |= 1u << s;
+    for (uint32_t j = 0; !aborted; ++j) {
+      const int slot = j % kWorkSlots;
+      if (!wait_or_abort(&bars.wfull[slot], (j / kWorkSlots) & 1, &s_abort, limit_us, true))
+        break;
+      const WorkRec rec = s_rec[slot];
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&bars.wempty[slot]);
+      if (rec.kind == kWorkEnd) break;
+      const MixedParams &p = MULTI ? bl.probs[rec.problem] : p1;
+      const uint8_t *const xpl = reinterpret_cast<const uint8_t *>(p.xpl) + q * 16;
+      const int32_t *const key_ids = p.sched.key_ids, *const key_xrow = p.sched.key_xrow;
+      const int n_kc = p.g.n_kc, n_xrows = p.n_xrows, n_table_keys = p.d.n_tables * p.d.n_cases;
+      const uint32_t row_bytes = (uint32_t)p.g.kp * kXPlanes * 2u;   // of a density row
+      const int k0 = rec.k0, k1 = rec.k1;
+      // the output data of this warp's rows, put out once the item's first
+      // copies are under way
+      auto put_rows = [&]() {
+        for (int r = kRowsPerProducer * warp + lane; r < kRowsPerProducer * (warp + 1); r += 32) {
+          RowOut o;
+          o.where = 0;
+          o.ex = 0;
+          o.row = -1;
+          int v = rec.kind == kWorkRun ? p.sched.tile_rows[(int64_t)rec.tile * 128 + r] : -1;
+          if (v >= (int64_t)p.n_tgt_boxes * p.nrhs) {
+            report(p.st, VL1_E_ARG, rec.tile, r);
+            v = -1;
           }
-          tc::fence_proxy_async_smem();
-          __syncwarp();
-          if (!hold) mbar_arrive(&bars.xfull[s]);
-          continue;
+          if (v >= 0) {
+            const int jb = v / p.nrhs, rh = v - jb * p.nrhs;
+            const int tbox = p.target_boxes[jb];
+            const int per = p.d.table_cplx ? 2 : 1;
+            const int n_out = per * max(min(p.tgt_counts[tbox], p.d.nq), 0);
+            const long long first =
+                per * ((long long)rh * p.n_particles + p.tgt_starts[tbox]);
+            o.where = (first << 16) | n_out;
+            // table values are m_a 2^(a_exp - kFixedBits), densities
+            // m_x 2^(e - kXFixedBits) with e the scale exponent of the rhs;
+            // the sums count units of 2^32 of m_a m_x
+            o.ex = p.a_exp + (p.x_exp[rh] - kExpBias) - (kFixedBits + kXFixedBits) + 32;
+            o.row = v;
+          }
+          s_out[slot][r] = o;
         }
-        zero_stages &= ~(1u << s);
-#pragma unroll
-        for (int it = 0; it < NIT; ++it) {
-          // piece pc of the warp's rows: row pc / PPR, plane q / PPP, values
-          // 8 (q % PPP) .. +7 of the K chunk (consecutive lanes read one
-          // row's 8 * KC contiguous bytes)
-          const int pc = it * 32 + lane;
-          const int rl = pc / PPR, q = pc - (pc / PPR) * PPR;
-          const int pl = q / PPP, k8 = q - (q / PPP) * PPP;
-          const int xr = __shfl_sync(0xffffffffu, xr_lane, rl);
-          const int row = kRowsPerProducer * warp + rl;
-          const bool have = xr >= 0;
-          const __half *src =
-              p.xpl + (have ? (int64_t)xr * row_halves + ((int64_t)kc * kXPlanes + pl) * KC +
-                                  k8 * 8
-                            : 0);
-          tc::cp_async16_zfill(xs + pl * XBYTES + tc::kmajor_swizzled_offset(row, k8 * 8, KC),
-                               src, have ? 16u : 0u);
-        }
-        if (!hold) tc::cp_async_mbar_arrive_noinc(&bars.xfull[s]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.rfull[slot]);
+      };
+      bool rows_put = false;
+      int nkey = 0, nxr = -1;
+      if (k1 > k0) {
+        nkey = key_ids[k0];
+        nxr = key_xrow[(int64_t)k0 * 128 + my_row];
       }
+      for (int kidx = k0; kidx < k1 && !aborted; ++kidx) {
+        const int key = nkey;
+        int xr_lane = nxr;
+        if (kidx + 1 < k1) {
+          nkey = key_ids[kidx + 1];
+          nxr = key_xrow[(int64_t)(kidx + 1) * 128 + my_row];
+        }
+        const bool key_ok = key >= 0 && key < n_table_keys;
+        if (!key_ok) {
+          if (warp == 0 && lane == 0) report(p.st, VL1_E_ARG, rec.tile, kidx);
+          xr_lane = -1;
+        }
+        if (xr_lane >= n_xrows) {
+          report(p.st, VL1_E_ARG, rec.tile, my_row);
+          xr_lane = -1;
+        }
+        const bool key_empty =
+            __ballot_sync(0xffffffffu, lane < kRowsPerProducer && xr_lane >= 0) == 0u;
+        for (int kc = 0; kc < n_kc; ++kc) {
+          if (use > 0 &&
+              !wait_or_abort(&bars.empty[s], (use - 1) & 1, &s_abort, limit_us, true)) {
+            aborted = true;
+            break;
+          }
+          uint8_t *xs = smem + (size_t)s * STAGE_BYTES;
+          const bool hold = withhold && warp == 0 && use == 0 && s == 0;
+          if (key_empty) {
+            // no source rows: zero planes (the warp's rows of a swizzled
+            // K-major plane are one contiguous block), written once per stage
+            if (!((zero_stages >> s) & 1u)) {
+              constexpr int BLK = kRowsPerProducer * (int)ROW_BYTES;
+#pragma unroll
+              for (int dg = 0; dg < kXPlanes; ++dg)
+                for (int o = lane * 16; o < BLK; o += 32 * 16)
+                  *reinterpret_cast<uint4 *>(xs + dg * XBYTES + warp * BLK + o) =
+                      make_uint4(0u, 0u, 0u, 0u);
+              zero_stages |= 1u << s;
+            }
+            tc::fence_proxy_async_smem();
+            __syncwarp();
+            if (!hold) mbar_arrive(&bars.xfull[s]);
+          } else {
+            zero_stages &= ~(1u << s);
+            const uint8_t *const src0 = xpl + (uint32_t)kc * (2u * kXPlanes * KC);
+            const uint32_t dst = dst0 + (uint32_t)s * STAGE_BYTES;
+#pragma unroll
+            for (int it = 0; it < NIT; ++it) {
+              const int xr = __shfl_sync(0xffffffffu, xr_lane, it * (32 / PPR) + lane / PPR);
+              tc::cp_async16_zfill((dst ^ (uint32_t)((it % PPP) << 4)) + (uint32_t)it * 128u,
+                                   src0 + (uint64_t)(uint32_t)max(xr, 0) * row_bytes,
+                                   xr >= 0 ? 16u : 0u);
+            }
+            if (!hold) tc::cp_async_mbar_arrive_noinc(&bars.xfull[s]);
+          }
+          if (++s == kStages) {
+            s = 0;
+            ++use;
+          }
+          if (!rows_put) {
+            put_rows();
+            rows_put = true;
+          }
+        }
+      }
+      if (!rows_put && !aborted) put_rows();
     }
     tc::cp_async_wait_all();
     __syncwarp();
   } else if (warp == kLoaderWarp) {
-    // ---------------------------------------------------------- table loader
+    // ------------------------------------- work items and table digit tiles
     if (lane == 0) {
-      int u = 0;
-      bool aborted = false;
-      int nkey = n_keys > 0 ? p.sched.key_ids[k0] : 0;
-      for (int kidx = k0; kidx < k1 && !aborted; ++kidx) {
-        int key = nkey;
-        if (kidx + 1 < k1) nkey = p.sched.key_ids[kidx + 1];
-        if (key < 0 || key >= p.d.n_tables * p.d.n_cases) key = 0;   // reported by warp 0
-        for (int kc = 0; kc < p.g.n_kc; ++kc, ++u) {
-          const int s = (ubase + u) % kStages;
-          const int use = (ubase + u) / kStages;
-          if (use > 0 &&
-              !wait_or_abort(&bars.empty[s], (use - 1) & 1, &s_abort, limit_us, false)) {
-            aborted = true;
-            break;
-          }
-          uint8_t *as = smem + (size_t)s * STAGE_BYTES + kXPlanes * XBYTES;
-          tc::mbar_arrive_expect_tx(&bars.afull[s], kDigits * ABYTES);
-          const int64_t base = (((int64_t)key * p.g.n_kc + kc) * kDigits) * p.g.np * KC +
-                               (int64_t)chunk * NCH * KC;
-          if (n_chunks == 1) {
-            // one column chunk: the five digit tiles are contiguous
-            tc::bulk_g2s(as, p.adig + base, kDigits * ABYTES, &bars.afull[s]);
-          } else {
+      // put the record of work index w into the ring as ordinal j (false:
+      // the launch is being given up)
+      auto publish = [&](unsigned long long w, uint32_t j) -> bool {
+        const int slot = j % kWorkSlots;
+        WorkRec r{};
+        r.kind = kWorkEnd;
+        if (w < bl.n_items) {
+          s_claim[j % (2 * kWorkSlots)] = w;
+          s_nclaimed = (int)j + 1;
+          r = load_work<NCH, MULTI>(p1, bl, w);
+        }
+        if (j >= kWorkSlots && !wait_or_abort(&bars.wempty[slot], (j / kWorkSlots - 1) & 1,
+                                              &s_abort, limit_us, false))
+          return false;
+        s_rec[slot] = r;
+        mbar_arrive(&bars.wfull[slot]);
+        return true;
+      };
+      int s = 0;
+      uint32_t use = 0;
+      uint32_t issued = 0;   // units issued (bulk copies)
+      bool aborted = !publish(blockIdx.x, 0);
+      for (uint32_t j = 0; !aborted; ++j) {
+        const WorkRec rec = s_rec[j % kWorkSlots];   // this lane's own write
+        if (rec.kind == kWorkEnd) break;
+        const MixedParams &p = MULTI ? bl.probs[rec.problem] : p1;
+        const __half *const adig = p.adig;
+        const int32_t *const key_ids = p.sched.key_ids;
+        const int n_kc = p.g.n_kc, np = p.g.np, n_table_keys = p.d.n_tables * p.d.n_cases;
+        const int n_units = (rec.k1 - rec.k0) * n_kc;
+        // the next item is taken four units before this one's end (late, so
+        // that unequal items even out over the CTAs) and its record is put
+        // out before the last unit
+        unsigned long long next = 0;
+        bool taken = false, put = false;
+        int nkey = rec.k1 > rec.k0 ? key_ids[rec.k0] : 0;
+        int u = 0;
+        for (int kidx = rec.k0; kidx < rec.k1 && !aborted; ++kidx) {
+          int key = nkey;
+          if (kidx + 1 < rec.k1) nkey = key_ids[kidx + 1];
+          if (key < 0 || key >= n_table_keys) key = 0;   // reported by producer warp 0
+          for (int kc = 0; kc < n_kc; ++kc, ++u) {
+            if (!taken && u + 4 >= n_units) {
+              next = atomicAdd(bl.queue, 1ull) + gridDim.x;
+              taken = true;
+            }
+            if (u + 1 == n_units) {
+              put = true;
+              if (!publish(next, j + 1)) {
+                aborted = true;
+                break;
+              }
+            }
+            if (use > 0 &&
+                !wait_or_abort(&bars.empty[s], (use - 1) & 1, &s_abort, limit_us, false)) {
+              aborted = true;
+              break;
+            }
+            uint8_t *as = smem + (size_t)s * STAGE_BYTES + kXPlanes * XBYTES;
+            tc::mbar_arrive_expect_tx(&bars.afull[s], kDigits * ABYTES);
+            const int64_t base = (((int64_t)key * n_kc + kc) * kDigits) * np * KC +
+                                 (int64_t)rec.chunk * NCH * KC;
+            if (np == NCH) {
+              // one column chunk: the five digit tiles are contiguous
+              tc::bulk_g2s(as, adig + base, kDigits * ABYTES, &bars.afull[s]);
+            } else {
 #pragma unroll
-            for (int dg = 0; dg < kDigits; ++dg)
-              tc::bulk_g2s(as + dg * ABYTES, p.adig + base + (int64_t)dg * p.g.np * KC, ABYTES,
-                           &bars.afull[s]);
+              for (int dg = 0; dg < kDigits; ++dg)
+                tc::bulk_g2s(as + dg * ABYTES, adig + base + (int64_t)dg * np * KC, ABYTES,
+                             &bars.afull[s]);
+            }
+            ++issued;
+            if (++s == kStages) {
+              s = 0;
+              ++use;
+            }
           }
+        }
+        if (aborted) {
+          // an item taken but not yet put out is this CTA's to account for
+          if (taken && !put && next < bl.n_items) {
+            s_claim[(j + 1) % (2 * kWorkSlots)] = next;
+            s_nclaimed = (int)j + 2;
+          }
+          break;
+        }
+        if (!put) {   // an item without units
+          next = atomicAdd(bl.queue, 1ull) + gridDim.x;
+          if (!publish(next, j + 1)) aborted = true;
         }
       }
       if (aborted || s_abort) {
         // copies of the last (up to kStages) issued units may still be in
         // flight into this CTA's stages: let them land before the CTA exits
-        for (int v = u - kStages < 0 ? 0 : u - kStages; v < u; ++v)
-          wait_bounded(&bars.afull[(ubase + v) % kStages], ((ubase + v) / kStages) & 1,
-                       limit_us);
+        for (uint32_t v = issued < kStages ? 0 : issued - kStages; v < issued; ++v)
+          wait_bounded(&bars.afull[v % kStages], (v / kStages) & 1, limit_us);
       }
     }
     __syncwarp();
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------- tensor cores
-    if (lane == 0) {
-      const uint32_t tail_col = tbase + kExactCols * NCH;
-      int u = 0;
-      bool aborted = false;
-      for (int round = 0; round < n_rounds && !aborted; ++round) {
-        const int R = rbase + round;
+    // The whole warp runs the loop (waits included) in step and one elected
+    // lane executes the products, so that their operands are warp-uniform
+    // (issued from a one-lane branch a product takes ~100 clocks of the
+    // thread's time, more than the product itself).
+    const uint32_t el = tc::elect_one();
+    const uint32_t td = __shfl_sync(0xffffffffu, tbase, 0);
+    const uint64_t desc0 = tc::smem_desc_kmajor_swizzled(tc::smem_addr(smem), ROW_BYTES);
+    const uint32_t hi = (uint32_t)(desc0 >> 32);
+    const uint32_t lo0 = __shfl_sync(0xffffffffu, (uint32_t)desc0, 0);
+    const uint32_t tail_col = td + kExactCols * NCH;
+    auto wait = [&](uint64_t *bar, uint32_t phase) {
+      return wait_or_abort(bar, phase, &s_abort, limit_us, false);
+    };
+    int s = 0;
+    uint32_t ph = 0;   // phase parity of stage s
+    uint32_t R = 0;    // exact rounds of this CTA
+    // the barriers of the next unit are looked at between the products of
+    // this one, and waited for at its start only if they were not complete
+    bool have_a = false, have_x = false, aborted = false;
+    for (uint32_t j = 0; !aborted; ++j) {
+      const int slot = j % kWorkSlots;
+      if (!wait(&bars.wfull[slot], (j / kWorkSlots) & 1)) {
+        aborted = true;
+        break;
+      }
+      const int kind = __shfl_sync(0xffffffffu, s_rec[slot].kind, 0);
+      const int n_keys = __shfl_sync(0xffffffffu, s_rec[slot].k1 - s_rec[slot].k0, 0);
+      const int n_kc = __shfl_sync(
+          0xffffffffu, MULTI ? bl.probs[s_rec[slot].problem].g.n_kc : p1.g.n_kc, 0);
+      if (lane == 0) mbar_arrive(&bars.wempty[slot]);
+      __syncwarp();
+      if (kind == kWorkEnd) break;
+      const int n_units = n_keys * n_kc;
+      int iu = 0;          // unit within its round
+      for (int u = 0; u < n_units; ++u) {
         const int b = R & 1;
-        if (R >= 2 &&
-            !wait_or_abort(&bars.acce[b], ((R >> 1) - 1) & 1, &s_abort, limit_us, false)) {
+        if (iu == 0 && R >= 2 && !wait(&bars.acce[b], ((R >> 1) - 1) & 1)) {
           aborted = true;
           break;
         }
-        tc::tc_fence_after();
-        const uint32_t exact_col = tbase + (uint32_t)b * 5 * NCH;
-        for (int iu = 0; iu < upr && u < n_units; ++iu, ++u) {
-          const int s = (ubase + u) % kStages;
-          const uint32_t ph = ((ubase + u) / kStages) & 1;
-          if (!wait_or_abort(&bars.afull[s], ph, &s_abort, limit_us, false)) {
-            aborted = true;
-            break;
-          }
-          if (!wait_or_abort(&bars.xfull[s], ph, &s_abort, limit_us, false)) {
-            aborted = true;
-            break;
-          }
-          // the digit rows were written by cp.async (generic proxy): order
-          // them before the tensor cores' (async proxy) reads
-          tc::fence_proxy_async_smem();
-          tc::tc_fence_after();
-          const uint32_t xa = tc::smem_addr(smem + (size_t)s * STAGE_BYTES);
-          // descriptors advance by (byte offset >> 4) in their address field
-          const uint64_t xd = tc::smem_desc_kmajor_swizzled(xa, ROW_BYTES);
-          const uint64_t adsc = tc::smem_desc_kmajor_swizzled(xa + kXPlanes * XBYTES, ROW_BYTES);
-#pragma unroll
-          for (int kk = 0; kk < KC / 16; ++kk) {
-#pragma unroll
-            for (int g = 0; g < kGroupCount; ++g) {
-              const MmaGroup gr = kGroups[g];
-              const uint32_t col = gr.exact ? exact_col + (uint32_t)(gr.i + gr.j0 - 2) * NCH
-                                            : tail_col + (uint32_t)(gr.i + gr.j0 - 5) * NCH;
-              const bool first = gr.exact ? (g == 0 && iu == 0 && kk == 0)
-                                          : (g == 3 && u == 0 && kk == 0);
-              const uint64_t ad = xd + (((uint32_t)(gr.i - 1) * XBYTES + kk * 32u) >> 4);
-              const uint64_t bd = adsc + (((uint32_t)(gr.j0 - 1) * ABYTES + kk * 32u) >> 4);
-              tc::mma_f16(col, ad, bd, tc::idesc_f16_f32(128, NCH * gr.nb), first ? 0u : 1u);
-            }
-          }
-          tc::mma_commit(&bars.empty[s]);   // stage free once these products finish
+        if ((!have_a && !wait(&bars.afull[s], ph)) || (!have_x && !wait(&bars.xfull[s], ph))) {
+          aborted = true;
+          break;
         }
-        if (!aborted) tc::mma_commit(&bars.accf[b]);
+        // the digit rows were written by cp.async (generic proxy): order
+        // them before the tensor cores' (async proxy) reads
+        tc::fence_proxy_async_smem();
+        tc::tc_fence_after();
+        const uint32_t exact_col = td + (uint32_t)b * 5 * NCH;
+        const uint32_t x_lo = lo0 + (((uint32_t)s * STAGE_BYTES) >> 4);
+        const uint32_t a_lo = x_lo + ((kXPlanes * XBYTES) >> 4);
+        const int s_next = s + 1 == kStages ? 0 : s + 1;
+        const uint32_t ph_next = s_next == 0 ? ph ^ 1u : ph;
+        auto group = [&](int kk, int g, uint32_t accumulate) {
+          const MmaGroup gr = kGroups[g];
+          const uint32_t col = gr.exact ? exact_col + (uint32_t)(gr.i + gr.j0 - 2) * NCH
+                                        : tail_col + (uint32_t)(gr.i + gr.j0 - 5) * NCH;
+          tc::mma_f16_elected(col, x_lo + (((uint32_t)(gr.i - 1) * XBYTES + kk * 32u) >> 4),
+                              a_lo + (((uint32_t)(gr.j0 - 1) * ABYTES + kk * 32u) >> 4), hi,
+                              tc::idesc_f16_f32(128, NCH * gr.nb), accumulate, el);
+        };
+        // the exact groups first: an item's first unit has its tail groups
+        // wait until the readout warps have taken the item before's tails
+#pragma unroll
+        for (int kk = 0; kk < KC / 16; ++kk)
+#pragma unroll
+          for (int g = 0; g < kExactGroups; ++g)
+            group(kk, g, g == 0 && kk == 0 && iu == 0 ? 0u : 1u);
+        if (u == 0 && j > 0) {
+          if (!wait(&bars.taile, (j - 1) & 1)) {
+            aborted = true;
+            break;
+          }
+          tc::tc_fence_after();
+        }
+        have_a = tc::mbar_test(&bars.afull[s_next], ph_next);
+#pragma unroll
+        for (int kk = 0; kk < KC / 16; ++kk)
+#pragma unroll
+          for (int g = kExactGroups; g < kGroupCount; ++g)
+            group(kk, g, g == kExactGroups && kk == 0 && u == 0 ? 0u : 1u);
+        have_x = tc::mbar_test(&bars.xfull[s_next], ph_next);
+        tc::mma_commit_elected(&bars.empty[s], el);   // stage free once these finish
+        s = s_next;
+        ph = ph_next;
+        if (++iu == upr || u + 1 == n_units) {
+          tc::mma_commit_elected(&bars.accf[b], el);
+          iu = 0;
+          ++R;
+        }
       }
-      if (aborted || s_abort) {
-        // MMAs issued before the abort still write TMEM and read the stages:
-        // wait for all of them before the TMEM is released
-        tc::mma_commit(&bars.drain);
-        wait_bounded(&bars.drain, 0, limit_us);
-      }
+      // every phase of taile is waited for, also by an item without units
+      if (!aborted && n_units == 0 && j > 0 && !wait(&bars.taile, (j - 1) & 1)) aborted = true;
+    }
+    if (aborted || s_abort) {
+      // MMAs issued before the abort still write TMEM and read the stages:
+      // wait for all of them before the TMEM is released
+      tc::mma_commit_elected(&bars.drain, el);
+      wait_bounded(&bars.drain, 0, limit_us);
     }
     __syncwarp();
   } else {
@@ -1108,199 +1329,226 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
     const int cb = rw >> 2;                // RC-column block
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
     const int row = quad * 32 + lane;
-    // exact sum of the diagonals per output, units of 2^(e-32); the d = 2
-    // and d = 3 terms enter as the raw bits of (d + 1.5 * 2^23), whose
-    // constant part is taken out once after the loop
-    unsigned long long acc[RC];
+    // this warp's slice of shared memory: eight columns of finished outputs
+    // at a time (rows padded by one value, so that the 32 rows of a column lie
+    // in distinct banks; it holds the row's place in the result)
+    double *park = reinterpret_cast<double *>(smem + (size_t)kStages * STAGE_BYTES +
+                                              (size_t)rw * kParkBytes);
+    uint32_t R = 0;
+    for (uint32_t j = 0;; ++j) {
+      // one decision for all readout warps, so that every barrier among them
+      // inside an item is reached by all of them
+      const int slot = j % kWorkSlots;
+      if (rw == 0) {
+        const bool got = wait_or_abort(&bars.wfull[slot], (j / kWorkSlots) & 1, &s_abort,
+                                       limit_us, true);
+        if (lane == 0) s_go[j & 1] = got && s_rec[slot].kind != kWorkEnd;
+      }
+      readout_barrier<NREAD * 32>();
+      if (!s_go[j & 1]) break;
+      const WorkRec rec = s_rec[slot];
+      const MixedParams &p = MULTI ? bl.probs[rec.problem] : p1;
+      const bool oc = p.d.table_cplx;
+      const int n_units = (rec.k1 - rec.k0) * p.g.n_kc;
+      const int n_rounds = (n_units + upr - 1) / upr;
+      // exact sum of the digit products per output, units of 2^32: the
+      // diagonals 2, 3, 4 (weights 2^64, 2^56, 2^48) as integers, the FP32
+      // tails d5, d6 (weights 2^40, 2^32) rounded to the unit.  The d = 2
+      // and d = 3 terms enter as the raw bits of (d + 1.5 * 2^23), whose
+      // constant part is taken out once after the loop
+      unsigned long long acc[RC];
 #pragma unroll
-    for (int c = 0; c < RC; ++c) acc[c] = 0;
-    bool ok = true;
-    int rounds_read = 0;
-    for (int round = 0; round < n_rounds; ++round) {
-      const int R = rbase + round;
-      const int b = R & 1;
-      if (!wait_or_abort(&bars.accf[b], (R >> 1) & 1, &s_abort, limit_us, true)) {
+      for (int c = 0; c < RC; ++c) acc[c] = 0;
+      bool ok = true;
+      for (int round = 0; round < n_rounds; ++round, ++R) {
+        const int b = R & 1;
+        if (!wait_or_abort(&bars.accf[b], (R >> 1) & 1, &s_abort, limit_us, true)) {
+          ok = false;
+          break;
+        }
+        tc::tc_fence_after();
+        const uint32_t col = tbase + lane_off + (uint32_t)b * 5 * NCH + cb * RC;
+        uint32_t r2[16], r3[16];
+        if (round == n_rounds - 1) {
+          // the tails first: the next item's products wait for them
+          const uint32_t tcol = tbase + lane_off + kExactCols * NCH + cb * RC;
+          tc::tmem_ld16(tcol, r2);               // d5, weight 2^40
+          tc::tmem_ld16(tcol + NCH, r3);         // d6, weight 2^32
+          tc::tmem_ld_wait();
+          tc::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&bars.taile);
+          if (n_units <= kSmallTailK / KC) {
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              acc[c] += tail_bits<8>(__uint_as_float(r2[c]));
+              acc[c] += tail_bits<0>(__uint_as_float(r3[c]));
+            }
+          } else {
+            const unsigned long long both = 2ull * kTailBitsConst;   // taken out below
+#pragma unroll
+            for (int c = 0; c < 16; ++c)
+              acc[c] += (unsigned long long)f32_scaled_to_i64(__uint_as_float(r2[c]), 256.0f) +
+                        (unsigned long long)f32_scaled_to_i64(__uint_as_float(r3[c]), 1.0f) +
+                        both;
+          }
+        }
+        uint32_t r4[16];
+        tc::tmem_ld16(col, r2);                // i + j = 2: |x| <= 128 * 128 * 128 = 2^21
+        tc::tmem_ld16(col + NCH, r3);          // i + j = 3: |x| <= 2 * 2^21 = 2^22
+        tc::tmem_ld16(col + 2 * NCH, r4);      // i + j = 4: |x| <= 3 * 2^21 < 2^24
+        tc::tmem_ld_wait();
+        tc::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.acce[b]);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          // 1.5 * 2^23 + x for |x| <= 2^22 is exact and its raw bits are
+          // kMagicBits + x (also at x = 2^22, where the sum is 2^24); weights
+          // 2^32 and 2^24 of the d = 2 and d = 3 terms
+          const uint32_t b2 = __float_as_uint(__uint_as_float(r2[c]) + kMagic);
+          const uint32_t b3 = __float_as_uint(__uint_as_float(r3[c]) + kMagic);
+          acc[c] += ((unsigned long long)b2 << 32) + (unsigned long long)b3 * 16777216ull;
+          acc[c] += (unsigned long long)((long long)__float2int_rn(__uint_as_float(r4[c])) * 65536);
+        }
+      }
+      if (n_rounds == 0) {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.taile);
+      }
+      {
+        // the constant parts of the raw bits, (kMagicBits << 32) +
+        // (kMagicBits << 24) per round and those of the two tails (modulo
+        // 2^64: the true sum fits an int64)
+        const unsigned long long magic_total =
+            (unsigned long long)n_rounds * (((unsigned long long)kMagicBits * 65792ull) << 16) +
+            (n_rounds > 0 ? 2ull * kTailBitsConst : 0ull);
+#pragma unroll
+        for (int c = 0; c < 16; ++c) acc[c] -= magic_total;
+      }
+      if (!wait_or_abort(&bars.rfull[slot], (j / kWorkSlots) & 1, &s_abort, limit_us, true))
         ok = false;
-        break;
-      }
-      tc::tc_fence_after();
-      const uint32_t col = tbase + lane_off + (uint32_t)b * 5 * NCH + cb * RC;
-      uint32_t r2[16], r3[16];
-      tc::tmem_ld16(col, r2);                // i + j = 2: |x| <= 128 * 128 * 128 = 2^21
-      tc::tmem_ld16(col + NCH, r3);          // i + j = 3: |x| <= 2 * 2^21 = 2^22
-      tc::tmem_ld_wait();
+      bool write = ok && rec.kind == kWorkRun;
+      if (rec.split >= 0 && rec.kind == kWorkRun) {
+        // ---- a split tile: the parts add their exact int64 sums into the
+        // slot of part 0 (integer addition: the total does not depend on the
+        // order; column-major, so that a warp's 32 rows are adjacent); the
+        // part that arrives last reads the total and leaves the accumulator
+        // and the counter at zero for the next call (also after an abort, so
+        // that a timed-out call does not spoil the schedule)
+        const int n_chunks = p.g.np / NCH;
+        unsigned long long *g_acc =
+            reinterpret_cast<unsigned long long *>(
+                static_cast<uint8_t *>(p.sched.split_partials) +
+                ((int64_t)(rec.slot - rec.part) * n_chunks + rec.chunk) * (128 * NCH * 8)) +
+            (cb * RC) * 128 + row;
+        int *g_ctr = p.sched.split_counters +
+                     ((int64_t)rec.split * n_chunks + rec.chunk) * kSplitCounterStride;
+        if (ok) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        // 1.5 * 2^23 + x for |x| <= 2^22 is exact and its raw bits are
-        // kMagicBits + x (also at x = 2^22, where the sum is 2^24); weights
-        // 2^16 and 2^8 of the d = 2 and d = 3 terms
-        const uint32_t b2 = __float_as_uint(__uint_as_float(r2[c]) + kMagic);
-        const uint32_t b3 = __float_as_uint(__uint_as_float(r3[c]) + kMagic);
-        acc[c] += (unsigned long long)b2 * 65536ull + (unsigned long long)b3 * 256ull;
+          for (int c = 0; c < 16; ++c) atomicAdd(g_acc + c * 128, acc[c]);
+        }
+        __threadfence();
+        readout_barrier<NREAD * 32>();
+        if (rw == 0 && lane == 0) {
+          // parts count in the low 16 bits; a part that aborted (and may not
+          // have added all its sums) also adds to the high bits, so that the
+          // last part writes nothing for the tile
+          const int inc = s_abort ? kSplitPoison + 1 : 1;
+          const int done = atomicAdd(g_ctr, inc) + inc;
+          s_last = (done & (kSplitPoison - 1)) == rec.nparts;
+          s_poison = done >= kSplitPoison;
+          if (s_last) *g_ctr = 0;
+          s_ndone = (int)j + 1;
+        }
+        readout_barrier<NREAD * 32>();
+        write = write && s_last && !s_poison;
+        if (s_last) {
+          __threadfence();
+#pragma unroll
+          for (int c = 0; c < 16; ++c) acc[c] = __ldcg(g_acc + c * 128);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) g_acc[c * 128] = 0ull;
+        }
       }
-      tc::tmem_ld16(col + 2 * NCH, r2);      // i + j = 4: |x| <= 3 * 2^21 < 2^24
-      tc::tmem_ld_wait();
-      tc::tc_fence_before();
+      if (write) {
+        // ---- one rounding to FP64 per output (integer operations: the FP64
+        // pipe is narrow on this GPU), then eight columns of the 32 rows at a
+        // time through the warp's slice: 64 consecutive bytes of a row per
+        // eight lanes
+        const long long where = s_out[slot][row].where;
+        const int ex = s_out[slot][row].ex;
+        const int n_cols = (oc ? 2 : 1) * p.d.nq;
+        const bool disp = p.disp != nullptr;
+        double d0 = 0.0, d1 = 0.0;
+        if (disp && s_out[slot][row].row >= 0) {
+          const int64_t v = s_out[slot][row].row;   // j * nrhs + r
+          d0 = oc ? p.disp[2 * v] : p.disp[v];
+          d1 = oc ? p.disp[2 * v + 1] : d0;
+        }
+        double *const result = p.result;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int c0 = rec.chunk * NCH + cb * RC + h * 8;
+          if (c0 >= n_cols) break;   // padding columns only
+          __syncwarp();
+          bool rare = false;
+          double y[8];
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            y[c] = scaled_i64_select((long long)acc[h * 8 + c], ex, rare);
+          if (rare) {
+#pragma unroll
+            for (int c = 0; c < 8; ++c)
+              park[lane * 9 + c] = __longlong_as_double((long long)acc[h * 8 + c]);
+#pragma unroll 1
+            for (int c = 0; c < 8; ++c) {
+              const long long v = __double_as_longlong(park[lane * 9 + c]);
+              park[lane * 9 + c] = scaled_i64_to_double(v, ex);
+            }
+#pragma unroll
+            for (int c = 0; c < 8; ++c) y[c] = park[lane * 9 + c];
+          }
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            if (disp) y[c] += (c & 1) ? d1 : d0;
+            park[lane * 9 + c] = y[c];
+          }
+          park[lane * 9 + 8] = __longlong_as_double(where);
+          __syncwarp();
+          const int c = lane & 7;
+#pragma unroll
+          for (int it = 0; it < 8; ++it) {
+            const int rl = it * 4 + (lane >> 3);
+            const long long at = __double_as_longlong(park[rl * 9 + 8]);
+            if (c0 + c < (int)(at & 0xFFFFll)) result[(at >> 16) + c0 + c] = park[rl * 9 + c];
+          }
+        }
+        __syncwarp();
+      }
       __syncwarp();
-      if (lane == 0) mbar_arrive(&bars.acce[b]);
-#pragma unroll
-      for (int c = 0; c < 16; ++c)
-        acc[c] += (unsigned long long)(long long)__float2int_rn(__uint_as_float(r2[c]));
-      ++rounds_read;
-    }
-    // ---- park one int64 per output: the sum of digit products in units of
-    // 2^32 (integer diagonals 2..4, weights 2^64..2^48, shifted by 16, plus
-    // the FP32 tails d5, d6 of weights 2^40, 2^32 rounded to that unit)
-    if (ok && !s_abort) {
-      long long *s_tot = reinterpret_cast<long long *>(smem);
-      const uint32_t col = tbase + lane_off + kExactCols * NCH + cb * RC;
-      // the constant parts of the raw bits, (kMagicBits << 16) + (kMagicBits
-      // << 8) per round (modulo 2^64: the true sum fits an int64)
-      const unsigned long long magic_total =
-          (unsigned long long)rounds_read * ((unsigned long long)kMagicBits * 65792ull);
-#pragma unroll
-      for (int c = 0; c < 16; ++c) acc[c] = (acc[c] - magic_total) << 16;
-      if (n_rounds > 0) {
-        uint32_t r16[16];
-        tc::tmem_ld16(col, r16);                 // d5, weight 2^40
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          acc[c] += (unsigned long long)f32_scaled_to_i64(__uint_as_float(r16[c]), 256.0f);
-        tc::tmem_ld16(col + NCH, r16);           // d6, weight 2^32
-        tc::tmem_ld_wait();
-#pragma unroll
-        for (int c = 0; c < 16; ++c)
-          acc[c] += (unsigned long long)f32_scaled_to_i64(__uint_as_float(r16[c]), 1.0f);
-      }
-#pragma unroll
-      for (int c = 0; c < 16; ++c)
-        s_tot[row * PARK_STRIDE + cb * RC + c] = (long long)acc[c];
+      if (lane == 0) mbar_arrive(&bars.wempty[slot]);   // the record and the row data are used
+      if (rw == 0 && lane == 0 && ok) s_ndone = (int)j + 1;
     }
   }
 
-  // ---- all warps: final values and coalesced writes (a row's outputs are
-  // the consecutive target points of one box).  A split tile's parts store
-  // their exact partial sums; the part that finishes last adds them (exactly,
-  // in int64) and writes the results.  The one rounding to FP64 is done with
-  // integer operations (the FP64 pipe is narrow on this GPU).
   tc::tc_fence_before();
   __syncthreads();
-  __shared__ int s_last, s_poison;
-  const long long *tot_src = reinterpret_cast<const long long *>(smem);
-  bool write = !s_abort;
-  // a split tile's accumulator: the parts add their exact int64 sums into
-  // the slot of part 0 (integer addition: the total does not depend on the
-  // order); the part that arrives last writes the results and clears it
-  unsigned long long *g_acc = nullptr;
-  const int64_t slot_bytes = (int64_t)128 * NCH * 8;
-  int *g_ctr = nullptr;
-  if (item.split >= 0) {
-    g_acc = reinterpret_cast<unsigned long long *>(
-        static_cast<uint8_t *>(p.sched.split_partials) +
-        ((int64_t)(item.slot - item.part) * n_chunks + chunk) * slot_bytes);
-    g_ctr = p.sched.split_counters + ((int64_t)item.split * n_chunks + chunk) * kSplitCounterStride;
-    if (!s_abort) {
-      for (int i = tid; i < 128 * NCH; i += blockDim.x)
-        atomicAdd(g_acc + i, (unsigned long long)tot_src[(i / NCH) * PARK_STRIDE + i % NCH]);
-    }
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-      // parts count in the low 16 bits; a part that aborted (and added no
-      // sums) also adds to the high bits, so that the last part writes
-      // nothing for the tile
-      const int inc = s_abort ? kSplitPoison + 1 : 1;
-      const int done = atomicAdd(g_ctr, inc) + inc;
-      s_last = (done & (kSplitPoison - 1)) == item.nparts;
-      s_poison = done >= kSplitPoison;
-    }
-    __syncthreads();
-    write = write && s_last && !s_poison;
-    if (s_last) __threadfence();
-  } else {
-    __syncthreads();
-  }
-  if (write) {
-    const bool oc = p.d.table_cplx;
-    // BATCH outputs per thread and pass: their loads (parked sums, or the
-    // parts of a split tile from L2) are issued before any conversion
-    constexpr int BATCH = 4;
-    for (int it0 = tid; it0 < 128 * NCH; it0 += BATCH * (int)blockDim.x) {
-      long long tot[BATCH];
-#pragma unroll
-      for (int bi = 0; bi < BATCH; ++bi) {
-        const int it = it0 + bi * (int)blockDim.x;
-        tot[bi] = 0;
-        if (it >= 128 * NCH) continue;
-        if (item.split >= 0) {
-          tot[bi] = (long long)__ldcg(g_acc + it);
-        } else {
-          tot[bi] = tot_src[(it / NCH) * PARK_STRIDE + it % NCH];
-        }
-      }
-#pragma unroll
-      for (int bi = 0; bi < BATCH; ++bi) {
-        const int it = it0 + bi * (int)blockDim.x;
-        if (it >= 128 * NCH) continue;
-        const int rw_ = it / NCH, cc = it - rw_ * NCH;
-        int t = chunk * NCH + cc, part = 0;
-        if (oc && t >= p.d.nq) {
-          t -= p.d.nq;
-          part = 1;
-        }
-        if (t >= s_ocnt[rw_]) continue;   // also empty rows and padding columns
-        double y = scaled_i64_to_double(tot[bi], s_oexp[rw_]);
-        if (p.disp) {
-          const int64_t di = s_rows[rw_];   // j * nrhs + r
-          y += oc ? p.disp[2 * di + part] : p.disp[di];
-        }
-        const int64_t o = s_obase[rw_] + t;
-        if (oc)
-          p.result[2 * o + part] = y;
-        else
-          p.result[o] = y;
-      }
-    }
-  }
-  // the last part leaves the accumulator and the counter at zero for the
-  // next call (also after an abort, so that a timed-out call does not spoil
-  // the schedule); each thread clears the entries it read
-  if (item.split >= 0 && s_last) {
-    for (int i = tid; i < 128 * NCH; i += blockDim.x) g_acc[i] = 0ull;
-    if (tid == 0) *g_ctr = 0;
-  }
-  __syncthreads();
   if (s_abort && tid == 0) {
-    report(p.st, VL1_E_TIMEOUT, tile, chunk);
-    if (MULTI) {
-      // the items this launch will no longer run still count their parts,
-      // so that every split counter ends at zero
-      for (;;) {
-        const int wj = atomicAdd(bl.queue, 1);
-        if (wj >= bl.n_items) break;
-        const BatchItem bj = bl.items[wj];
-        if (bj.item.split < 0) continue;
-        const MixedParams *pj = bl.probs + bj.problem;
-        const int nchk = pj->g.np / NCH;
-        int *ctr = pj->sched.split_counters +
-                   ((int64_t)bj.item.split * nchk + bj.chunk) * kSplitCounterStride;
-        const int done = atomicAdd(ctr, kSplitPoison + 1) + kSplitPoison + 1;
-        if ((done & (kSplitPoison - 1)) == bj.item.nparts) {
-          // the tile's last arrival: clear what its other parts added
-          unsigned long long *acc = reinterpret_cast<unsigned long long *>(
-              static_cast<uint8_t *>(pj->sched.split_partials) +
-              ((int64_t)(bj.item.slot - bj.item.part) * nchk + bj.chunk) * slot_bytes);
-          for (int i = 0; i < 128 * NCH; ++i) acc[i] = 0ull;
-          *ctr = 0;
-        }
-      }
+    // report the first item that is not done, and let the items that this CTA
+    // took or nobody has taken still count their parts, so that every split
+    // counter ends at zero
+    const int nc = s_nclaimed, nd = s_ndone;
+    abandon_work<NCH, MULTI>(p1, bl, s_claim[(nd < nc ? nd : nc - 1) % (2 * kWorkSlots)], true);
+    for (int o = nd; o < nc; ++o)
+      abandon_work<NCH, MULTI>(p1, bl, s_claim[o % (2 * kWorkSlots)], false);
+    for (;;) {
+      const unsigned long long w = atomicAdd(bl.queue, 1ull) + gridDim.x;
+      if (w >= bl.n_items) break;
+      abandon_work<NCH, MULTI>(p1, bl, w, false);
     }
   }
-  ubase += n_units;
-  rbase += n_rounds;
   __syncthreads();
-  }   // work items
   if (warp == kMmaWarp) tc::tmem_dealloc(tbase, COLS);
 }
 
@@ -1316,10 +1564,8 @@ const void *mixed_kernel_ptr(int nch, int kc, bool multi) {
 }
 
 size_t mixed_smem_bytes(int nch, int kc) {
-  const int stages = nch >= 64 ? MixedRoles<64>::kStages : MixedRoles<32>::kStages;
-  const size_t pipe = (size_t)stages * (kXPlanes * 128 + kDigits * nch) * kc * 2;
-  const size_t park = (size_t)128 * (nch + 1) * 8;   // int64 sums, padded rows
-  return (pipe > park ? pipe : park) + 1024;
+  return (size_t)mixed_stages(nch, kc) * (kXPlanes * 128 + kDigits * nch) * kc * 2 +
+         (size_t)4 * (nch / 16) * kParkBytes + 1024;
 }
 
 int mixed_threads(int nch) {
@@ -1328,6 +1574,12 @@ int mixed_threads(int nch) {
 }
 
 int mixed_ctas_per_sm(int nch) { return nch >= 64 ? 1 : 2; }
+
+// persistent CTAs of a launch over n_items work items
+int mixed_grid(unsigned long long n_items, int n_sm, int nch) {
+  return (int)std::min<unsigned long long>(n_items, (unsigned long long)n_sm *
+                                                        mixed_ctas_per_sm(nch));
+}
 
 cudaError_t launch_mixed_kernel(int nch, int kc, bool multi, dim3 grid, cudaStream_t s,
                                 const MixedParams &mp, const BatchLaunch &bl) {
@@ -1393,7 +1645,7 @@ int64_t mixed_workspace_bytes(const vl1_plan *plan, int64_t nboxes, int64_t n_tg
   const MixedGeom &g = plan->mixed.geom;
   const int cv = plan->d.table_cplx ? 2 : 1;
   int64_t b = 0;
-  b += ((int64_t)nrhs * 4 + 255) / 256 * 256;                       // rhs scale exponents
+  b += (8 + (int64_t)nrhs * 4 + 255) / 256 * 256;                   // queue, rhs scale exponents
   b += (nboxes * nrhs * g.kp * kXPlanes * 2 + 255) / 256 * 256;    // density digit planes
   if (plan->d.disp_kind == VL1_DISP_LOG2D) {
     b += (nboxes * nrhs * cv * 8 + 255) / 256 * 256;            // per-box displacement
@@ -1449,8 +1701,9 @@ int32_t launch_mixed(vl1_plan *plan, const TreeDev &tree, int64_t nboxes,
               (long long)n_xrows);
     return VL1_E_UNSUPPORTED;
   }
-  int *x_exp = reinterpret_cast<int *>(w);
-  w += ((int64_t)nrhs * 4 + 255) / 256 * 256;
+  unsigned long long *queue = reinterpret_cast<unsigned long long *>(w);
+  int *x_exp = reinterpret_cast<int *>(w + 8);
+  w += (8 + (int64_t)nrhs * 4 + 255) / 256 * 256;
   __half *xpl = reinterpret_cast<__half *>(w);
   w += (n_xrows * g.kp * kXPlanes * 2 + 255) / 256 * 256;
   double *wbox = nullptr, *disp = nullptr;
@@ -1461,9 +1714,9 @@ int32_t launch_mixed(vl1_plan *plan, const TreeDev &tree, int64_t nboxes,
   }
   cudaError_t e;
   const int64_t nbr = n_xrows;
-  // the rhs scale exponents (maximum over all density rows), then the digit
-  // planes of every density row
-  e = cudaMemsetAsync(x_exp, 0, sizeof(int) * nrhs, s);
+  // the work queue's count, the rhs scale exponents (maximum over all density
+  // rows), then the digit planes of every density row
+  e = cudaMemsetAsync(queue, 0, 8 + sizeof(int) * (size_t)nrhs, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(rhs exponents)");
   // a few blocks per SM, each warp striding over several rows: one global
   // atomic per block and rhs
@@ -1521,11 +1774,16 @@ int32_t launch_mixed(vl1_plan *plan, const TreeDev &tree, int64_t nboxes,
     set_error("mixed path: unsupported column chunk %d / K chunk %d", g.nch, g.kc);
     return VL1_E_UNSUPPORTED;
   }
-  dim3 grid(sched.n_items > 0 ? sched.n_items : sched.n_tiles, g.np / g.nch);
-  BatchLaunch none{};
+  int n_sm = 0;
+  e = cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, plan->device);
+  if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
+  BatchLaunch bl{};
+  bl.n_items = (unsigned long long)(sched.n_items > 0 ? sched.n_items : sched.n_tiles) *
+               (unsigned long long)(g.np / g.nch);
+  bl.queue = queue;
   int32_t st = record_kernel_event(g_kernel_begin, s);
   if (st) return st;
-  e = launch_mixed_kernel(g.nch, g.kc, false, grid, s, mp, none);
+  e = launch_mixed_kernel(g.nch, g.kc, false, mixed_grid(bl.n_items, n_sm, g.nch), s, mp, bl);
   if (e != cudaSuccess) return cuda_fail(e, "mixed_kernel launch");
   return record_kernel_event(g_kernel_end, s);
 }
@@ -1544,14 +1802,13 @@ struct BatchGroup {   // problems sharing one kernel shape: one persistent launc
   int grid;
 };
 
-// A problem large enough to fill the GPU on its own (two waves of CTAs or
-// more): launched with one work item per CTA, its parameters by value (the
-// persistent variant reads them from shared memory per item and is slower
-// per item).
+// A problem large enough to fill the GPU on its own (two items per CTA or
+// more): launched by itself, its parameters by value (the variant for several
+// problems reads them from global memory per item).
 struct SoloLaunch {
   int problem;
   int nch, kc;
-  int grid_x, grid_y;
+  unsigned long long n_items;
   vl1::MixedParams mp;
 };
 
@@ -1568,7 +1825,9 @@ struct vl1_batch {
   int n_problems = 0;
   void *d_probs = nullptr, *d_prep = nullptr, *d_tasks = nullptr, *d_items = nullptr;
   int n_tasks = 0;
-  int *d_queue = nullptr;
+  // one work queue count per launch (problems on their own, then groups),
+  // followed by d_exp: cleared together by each evaluation
+  unsigned long long *d_queue = nullptr;
   void *d_ttasks = nullptr;   // target-row tasks of the 2D displacement sums
   int n_ttasks = 0;
   int *d_exp = nullptr;       // every problem's rhs scale exponents, contiguous
@@ -1600,7 +1859,8 @@ struct BatchLayout {
   std::vector<BatchItem> all;
   std::vector<BatchGroup> groups;
   std::vector<SoloLaunch> solos;
-  int64_t o_probs = 0, o_prep = 0, o_tasks = 0, o_items = 0, o_queue = 0, o_ttasks = 0;
+  int64_t o_probs = 0, o_prep = 0, o_tasks = 0, o_items = 0, o_ttasks = 0;
+  int64_t o_queue = 0;        // the work queue counts, followed by o_exp
   int64_t o_exp = 0;          // the rhs scale exponents of all problems
   std::vector<int64_t> exp_off;   // a problem's first exponent in that region
   int64_t n_exp = 0;
@@ -1740,8 +2000,7 @@ int32_t assemble_batch(const char *who, int dev, int n_sm, int ctas_opt, int32_t
       sl.problem = i;
       sl.nch = g.nch;
       sl.kc = g.kc;
-      sl.grid_x = (int)n_x;
-      sl.grid_y = g.np / g.nch;
+      sl.n_items = (unsigned long long)ctas;
       L.solos.push_back(sl);
     }
   }
@@ -1793,8 +2052,6 @@ int32_t assemble_batch(const char *who, int dev, int n_sm, int ctas_opt, int32_t
   off += round256(sizeof(PrepTask) * (L.tasks.size() + 1));
   L.o_items = off;
   off += round256(sizeof(BatchItem) * (L.all.size() + 1));
-  L.o_queue = off;
-  off += round256(sizeof(int) * (L.groups.size() + 1));
   L.o_ttasks = off;
   off += round256(sizeof(PrepTask) * (L.ttasks.size() + 1));
   L.param_bytes = off;
@@ -1804,8 +2061,9 @@ int32_t assemble_batch(const char *who, int dev, int n_sm, int ctas_opt, int32_t
     L.exp_off[i] = L.n_exp;
     L.n_exp += problems[i].nrhs;
   }
-  L.o_exp = off;
-  off += round256(sizeof(int) * L.n_exp);
+  L.o_queue = off;
+  L.o_exp = off + 8 * (int64_t)(L.solos.size() + L.groups.size());
+  off = round256(L.o_exp + sizeof(int) * L.n_exp);
   L.o_ws.resize(n_problems);
   for (int i = 0; i < n_problems; ++i) {
     L.o_ws[i] = off;
@@ -1857,7 +2115,7 @@ void place_batch(vl1_batch *b, BatchLayout &L, const vl1_batch_problem *problems
   b->d_tasks = base + L.o_tasks;
   b->d_items = base + L.o_items;
   b->n_tasks = (int)L.tasks.size();
-  b->d_queue = reinterpret_cast<int *>(base + L.o_queue);
+  b->d_queue = reinterpret_cast<unsigned long long *>(base + L.o_queue);
   b->d_ttasks = base + L.o_ttasks;
   b->n_ttasks = (int)L.ttasks.size();
   b->d_exp = reinterpret_cast<int *>(base + L.o_exp);
@@ -2000,12 +2258,9 @@ extern "C" int32_t vl1_batch_eval(vl1_batch *b, void *stream) {
     return VL1_E_ARG;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaError_t e = cudaMemsetAsync(b->d_queue, 0, sizeof(int) * b->groups.size(), s);
+  cudaError_t e = cudaMemsetAsync(
+      b->d_queue, 0, 8 * (b->solos.size() + b->groups.size()) + sizeof(int) * b->n_exp, s);
   if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(batch)");
-  if (b->n_exp > 0) {
-    e = cudaMemsetAsync(b->d_exp, 0, sizeof(int) * b->n_exp, s);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaMemsetAsync(batch exponents)");
-  }
   if (b->n_tasks > 0) {
     x_exponent_batch_kernel<<<b->n_tasks, 256, 0, s>>>(
         static_cast<const PrepProblem *>(b->d_prep), static_cast<const PrepTask *>(b->d_tasks));
@@ -2032,13 +2287,17 @@ extern "C" int32_t vl1_batch_eval(vl1_batch *b, void *stream) {
   const MixedParams unused{};
   int32_t st = record_kernel_event(g_kernel_begin, s);
   if (st) return st;
+  unsigned long long *queue = b->d_queue;
   for (const SoloLaunch &sl : b->solos) {
-    const BatchLaunch none{};
+    BatchLaunch bl{};
+    bl.n_items = sl.n_items;
+    bl.queue = queue++;
     MixedParams mp = sl.mp;
     mp.wait_limit_us = g_test_wait_limit_us;
     mp.withhold_arrival = g_test_withhold;
-    void *args[] = {&mp, const_cast<BatchLaunch *>(&none)};
-    e = cudaLaunchKernel(mixed_kernel_ptr(sl.nch, sl.kc, false), dim3(sl.grid_x, sl.grid_y),
+    void *args[] = {&mp, &bl};
+    e = cudaLaunchKernel(mixed_kernel_ptr(sl.nch, sl.kc, false),
+                         dim3(mixed_grid(sl.n_items, b->n_sm, sl.nch)),
                          dim3(mixed_threads(sl.nch)), args, mixed_smem_bytes(sl.nch, sl.kc), s);
     if (e != cudaSuccess) return cuda_fail(e, "batch mixed_kernel launch (one problem)");
   }
@@ -2048,7 +2307,7 @@ extern "C" int32_t vl1_batch_eval(vl1_batch *b, void *stream) {
     bl.probs = static_cast<const MixedParams *>(b->d_probs);
     bl.items = static_cast<const BatchItem *>(b->d_items) + g.item0;
     bl.n_items = g.n_items;
-    bl.queue = b->d_queue + gi;
+    bl.queue = queue++;
     bl.wait_limit_us = g_test_wait_limit_us;
     bl.withhold_arrival = g_test_withhold;
     void *args[] = {const_cast<MixedParams *>(&unused), &bl};

@@ -99,4 +99,25 @@ __device__ __forceinline__ double scaled_i64_to_double(long long v, int k) {
   return ldexp((double)v, k);   // subnormal or overflowing results
 }
 
+// The same without a branch when the result is zero or a normal number;
+// otherwise `rare` is set and the value is to come from scaled_i64_to_double.
+// For threads that convert many independent values: their dependent chains
+// overlap, which the branches above (for zero, for the rounding's carry, for
+// the exponent range) prevent.  The rounded 53 bits, leading one included,
+// are added to the exponent field, so that the rounding's carry moves into
+// the exponent.
+__device__ __forceinline__ double scaled_i64_select(long long v, int k, bool &rare) {
+  const long long sg = v >> 63;
+  const unsigned long long mag = (unsigned long long)((v ^ sg) - sg);
+  const int lz = __clzll((long long)(mag | 1ull));
+  const unsigned long long m = mag << lz;   // leading one at bit 63
+  const unsigned lo = (unsigned)m;
+  const unsigned up = ((lo & 0x7FFu) + 0x3FFu + ((lo >> 11) & 1u)) >> 11;
+  const unsigned field = mag == 0ull ? 0u : (unsigned)(1085 - lz + k);   // biased exponent - 1
+  const unsigned long long bits = (m >> 11) + up + ((unsigned long long)field << 52);
+  rare |= field >= 2046u;
+  return __longlong_as_double(
+      (long long)(bits | ((unsigned long long)sg & 0x8000000000000000ull)));
+}
+
 }  // namespace vl1

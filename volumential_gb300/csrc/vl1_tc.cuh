@@ -71,8 +71,9 @@ __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t by
 // ---------------------------------------------------- cp.async (16 bytes)
 // 16 bytes, of which the first `src_bytes` (0 or 16) are read and the rest
 // zero-filled; with src_bytes == 0 nothing is read from `src`
-__device__ __forceinline__ void cp_async16_zfill(void *dst, const void *src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void *src,
+                                                 uint32_t src_bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
                "r"(src_bytes)
                : "memory");
 }

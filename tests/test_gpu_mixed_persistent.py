@@ -9,6 +9,8 @@ give the same bits.  Tolerances: sums of digit products that keep ~2^-38 of
 the largest products, as for the other tests of this path.
 """
 
+import gc
+
 import numpy as np
 import pytest
 
@@ -20,6 +22,13 @@ from volumential_gb300.kernels import HelmholtzKernel
 from volumential_gb300.plan import as_device_tensor
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _collect():
+    """Leave no device tensors in reference cycles for later memory checks."""
+    yield
+    gc.collect()
 
 TOL_MIXED = 1e-9
 

@@ -128,6 +128,38 @@ __device__ __forceinline__ void plane_values(double v, int e, __half &x1, __half
   rr = __float2half_rn((float)(sgn * ((int)(lp & 0xFFFFu) - 0x8080)) * (1.0f / 256.0f));
 }
 
+// The same for |v| < 2^e and scale = 2^(kFixedBits - e), both normal numbers:
+// the magnitude from one FP64 multiply-add (adding 2^52 rounds |v| * scale to
+// an integer, ties to even, in the low bits of the sum), the digits from its
+// biased bytes b as FP16 1024 + b (0x6400 | b) minus 1152, the sign by its bit
+// (a digit 0 may become -0), and R = X4 + X5 / 256 by one FP16 multiply-add,
+// rounded once.  p12 = (X1, X2), p3r = (X3, R).
+__device__ __forceinline__ void plane_values_scaled(double v, double scale, uint32_t &p12,
+                                                    uint32_t &p3r) {
+  const double r = __fma_rn(fabs(v), scale, 4503599627370496.0);
+  uint32_t lo = (uint32_t)__double2loint(r);
+  uint32_t hi = (uint32_t)__double2hiint(r) & 0xFFu;
+  if (hi >= (1u << (kFixedBits - 32))) {   // v at the scale bound
+    lo = 0xFFFFFFFFu;
+    hi = (1u << (kFixedBits - 32)) - 1u;
+  }
+  const uint32_t neg = ((uint32_t)__double2hiint(v) & 0x80000000u) ? 0x80008000u : 0u;
+  const uint32_t lp = lo + 0x80808080u;
+  const uint32_t top = hi + (lp < lo ? 1u : 0u);
+  // (1024 + top, 1024 + b2) - (1024, 1152); (1024 + b4, 1024 + b5) - 1152
+  const uint32_t w12 = __byte_perm(lp, top | 0x6400u, 0x5354);
+  const uint32_t w3 = __byte_perm(lp, 0x6400u, 0x5552) & 0xFFFFu;
+  const uint32_t w45 = __byte_perm(lp, 0x6400u, 0x5051);
+  const __half2 bias12 = __halves2half2(__ushort_as_half(0x6400), __ushort_as_half(0x6480));
+  const __half2 bias = __half2half2(__ushort_as_half(0x6480));
+  const __half2 d12 = __hsub2(*reinterpret_cast<const __half2 *>(&w12), bias12);
+  const __half2 d45 = __hsub2(*reinterpret_cast<const __half2 *>(&w45), bias);
+  const __half d3 = __hsub(__ushort_as_half((unsigned short)w3), __ushort_as_half(0x6480));
+  const __half rr = __hfma(__high2half(d45), __ushort_as_half(0x1C00), __low2half(d45));
+  p12 = *reinterpret_cast<const uint32_t *>(&d12) ^ neg;
+  p3r = ((uint32_t)__half_as_ushort(d3) | ((uint32_t)__half_as_ushort(rr) << 16)) ^ neg;
+}
+
 // ------------------------------------------------- plan: A digit operands
 
 __global__ void build_adig_kernel(DevDesc d, MixedGeom g, __half *adig, int a_exp) {
@@ -332,37 +364,71 @@ __device__ __forceinline__ void exp_block_end(int nrhs, const int *s_max, int *x
 // staging (G slices of 8 * kp bytes) and writes them out with 16-byte
 // stores.
 constexpr int kXPlanes = 4;          // density planes: X1, X2, X3, R
-#ifndef VL1_PLANE_GROUP
-#define VL1_PLANE_GROUP 4
-#endif
-// rows per warp group of the plane pass (its digit work holds every row's
-// state in registers, so it takes fewer rows than the exponent pass)
-constexpr int kPlaneGroup = VL1_PLANE_GROUP;
+// Rows per warp group of the plane pass: four, or, with short rows (one step
+// of the point loop each) of many right-hand sides, eight, of which most are
+// then rows of one box; the groups that are not go two rows at a time, so that
+// the kernel's 64 registers leave 32 warps to an SM.  2D q = 5, 4096 boxes and
+// 256 right-hand sides (520 MB in and out): 289 us with the digits by integer
+// shifts (240 instructions a row), 240 us with groups of four and the FP64
+// multiply-add, 189 us with groups of eight in 95 registers, 130 us so; the
+// FP64 pipe is then half busy.
+constexpr int kPlaneGroup = 4;
+constexpr int kPlaneGroupMany = 8;
+constexpr int kPlaneManyRhs = 32;
+// The scale factor of a row's digits (plane_values_scaled), 0 when they are to
+// come from plane_values: its scale exponent lies in [-900, 1000] (then the
+// densities of its rhs are finite and every power of two of it normal).  sl:
+// the binary logarithm of the box scaling if that is a power of two within
+// 2^+-60 (folded into the factor), else kNoScaleLog2.
+__device__ __forceinline__ double plane_scale(int ex, int sl) {
+  if (ex < -900 || ex > 1000) return 0.0;
+  return __longlong_as_double(
+      (long long)(1023 + kFixedBits - ex + (sl != kNoScaleLog2 ? sl : 0)) << 52);
+}
+
+__device__ __forceinline__ int plane_scale_log2(const TreeDev &tr, int level) {
+  const int sl = level < kScaleLevels ? tr.level_scale_log2[level] : kNoScaleLog2;
+  return sl >= -60 && sl <= 60 ? sl : kNoScaleLog2;
+}
+
+// the four FP16 values of source mode m (kc is 16 or 32: chunk and column by
+// shift and mask)
+__device__ __forceinline__ int plane_position(int m, int kc_shift, int kc) {
+  return ((m >> kc_shift) * kXPlanes << kc_shift) + (m & (kc - 1));
+}
+__device__ __forceinline__ void store_planes(uint8_t *row, int pos, int kc, uint32_t p12,
+                                             uint32_t p3r) {
+  uint16_t *hv = reinterpret_cast<uint16_t *>(row) + pos;
+  hv[0] = (uint16_t)p12;
+  hv[kc] = (uint16_t)(p12 >> 16);
+  hv[2 * kc] = (uint16_t)p3r;
+  hv[3 * kc] = (uint16_t)(p3r >> 16);
+}
+
+// The rows of a group into its stage, any boxes: every row's data in every
+// lane.
 template <int G>
-__device__ __forceinline__ void group_planes(const DevDesc &d, const TreeDev &tr,
+__device__ __forceinline__ void stage_planes(const DevDesc &d, const TreeDev &tr,
                                              const double *coefs, int nrhs, const int *x_exp,
-                                             __half *xpl, int kp, int kc, vl1_status *st,
-                                             int64_t r0, int n, int lane, uint8_t *stage) {
-  const int row_bytes = kp * kXPlanes * 2;
-  const int kc_shift = 31 - __clz(kc);
+                                             int row_bytes, int kc, int kc_shift,
+                                             vl1_status *st, int64_t r0, int n, int lane,
+                                             uint8_t *stage) {
   const RowGroup g = load_row_group(d, tr, nrhs, r0, n, lane, st);
   int ex = 0, sl = kNoScaleLog2;
   double sc = 0.0;
   if (lane < n) {
     ex = x_exp[g.rhs] - kExpBias;
     sc = box_scaling(d, tr, g.level);
-    // a power-of-two scaling: digits of c against 2^(e - log2 sc), the same
-    // as those of sc * c against 2^e when the product is exact (no overflow:
-    // e <= 1000; an underflowing product has zero digits when e >= -900)
-    if (g.level < kScaleLevels && ex >= -900 && ex <= 1000)
-      sl = tr.level_scale_log2[g.level];
+    sl = plane_scale_log2(tr, g.level);
   }
-  for (int k = lane * 16; k < G * row_bytes; k += 32 * 16)
-    *reinterpret_cast<uint4 *>(stage + k) = make_uint4(0u, 0u, 0u, 0u);
-  // every row's data in every lane (shuffles before the point loop, which
-  // not all lanes enter when nq is not a multiple of 32)
-  int cnt[G], st0[G], eu[G], bx[G], slu[G];
-  double scu[G];
+  const double scale = plane_scale(ex, sl);
+  // a power-of-two scaling folded into the factor gives the digits of sc * c:
+  // the product would be exact, or underflow to zero digits
+  const int how = scale == 0.0 ? 2 : (sl != kNoScaleLog2 ? 0 : 1);
+  // (shuffles before the point loop, which not all lanes enter when nq is not
+  // a multiple of 32)
+  int cnt[G], st0[G], eu[G], bx[G], hu[G];
+  double scu[G], mul[G];
   const double *c[G];
 #pragma unroll
   for (int u = 0; u < G; ++u) {
@@ -370,13 +436,13 @@ __device__ __forceinline__ void group_planes(const DevDesc &d, const TreeDev &tr
     st0[u] = __shfl_sync(0xffffffffu, g.start, u);
     const int rh = __shfl_sync(0xffffffffu, g.rhs, u);
     eu[u] = __shfl_sync(0xffffffffu, ex, u);
-    scu[u] = __shfl_sync(0xffffffffu, sc, u);
-    slu[u] = __shfl_sync(0xffffffffu, sl, u);
+    scu[u] = __shfl_sync(0xffffffffu, scale, u);
+    mul[u] = __shfl_sync(0xffffffffu, sc, u);
+    hu[u] = __shfl_sync(0xffffffffu, how, u);
     bx[u] = __shfl_sync(0xffffffffu, g.box, u);
     c[u] = coefs + (int64_t)rh * tr.n_particles + st0[u];
     if (u >= n) cnt[u] = 0;
   }
-  __syncwarp();
   for (int k = lane; k < d.nq; k += 32) {
     double v[G];
     int m[G];
@@ -389,30 +455,88 @@ __device__ __forceinline__ void group_planes(const DevDesc &d, const TreeDev &tr
 #pragma unroll
     for (int u = 0; u < G; ++u) {
       if (m[u] == -2) continue;
-      if (m[u] < 0 || m[u] >= d.nq) {
+      if ((unsigned)m[u] >= (unsigned)d.nq) {
         report(st, VL1_E_LAYOUT, bx[u], -1 - k);
         continue;
       }
-      const bool shift = slu[u] != kNoScaleLog2;
-      __half x1, x2, x3, rr;
-      plane_values(shift ? v[u] : scu[u] * v[u], shift ? eu[u] - slu[u] : eu[u], x1, x2, x3,
-                   rr);
-      // kc is 16 or 32: chunk and column by shift and mask
-      __half *hv = reinterpret_cast<__half *>(stage + u * row_bytes) +
-                   ((m[u] >> kc_shift) * kXPlanes << kc_shift) + (m[u] & (kc - 1));
-      hv[0] = x1;
-      hv[kc] = x2;
-      hv[2 * kc] = x3;
-      hv[3 * kc] = rr;
+      uint32_t p12, p3r;
+      if (hu[u] == 0) {   // uniform over the warp
+        plane_values_scaled(v[u], scu[u], p12, p3r);
+      } else if (hu[u] == 1) {
+        plane_values_scaled(mul[u] * v[u], scu[u], p12, p3r);
+      } else {
+        __half x1, x2, x3, rr;
+        plane_values(mul[u] * v[u], eu[u], x1, x2, x3, rr);
+        p12 = (uint32_t)__half_as_ushort(x1) | ((uint32_t)__half_as_ushort(x2) << 16);
+        p3r = (uint32_t)__half_as_ushort(x3) | ((uint32_t)__half_as_ushort(rr) << 16);
+      }
+      store_planes(stage + u * row_bytes, plane_position(m[u], kc_shift, kc), kc, p12, p3r);
     }
   }
+}
+
+// A group of rows into the digit planes.  When its rows are right-hand sides
+// of one box whose factors all have the power-of-two form, the box's data and
+// modes are read once for the group (25 points: 173 -> 79 instructions a row).
+template <int G, int A>
+__device__ __forceinline__ void group_planes(const DevDesc &d, const TreeDev &tr,
+                                             const double *coefs, int nrhs, const int *x_exp,
+                                             __half *xpl, int kp, int kc, vl1_status *st,
+                                             int64_t r0, int n, int lane, uint8_t *stage) {
+  const int row_bytes = kp * kXPlanes * 2;
+  const int kc_shift = 31 - __clz(kc);
+  for (int k = lane * 16; k < G * row_bytes; k += 32 * 16)
+    *reinterpret_cast<uint4 *>(stage + k) = make_uint4(0u, 0u, 0u, 0u);
   __syncwarp();
-  for (int u = 0; u < n; ++u) {
-    uint8_t *row = reinterpret_cast<uint8_t *>(xpl) + (r0 + u) * row_bytes;
-    for (int k = lane * 16; k < row_bytes; k += 32 * 16)
-      *reinterpret_cast<uint4 *>(row + k) =
-          *reinterpret_cast<const uint4 *>(stage + u * row_bytes + k);
+  const unsigned b = (unsigned)r0 / (unsigned)nrhs;   // row numbers fit 31 bits
+  const int rh0 = (int)((unsigned)r0 - b * (unsigned)nrhs);
+  bool one = n == G && rh0 + G <= nrhs;
+  double scale = 1.0;
+  if (one) {
+    const int sl = plane_scale_log2(tr, tr.levels[b]);
+    if (lane < G) scale = plane_scale(x_exp[rh0 + lane] - kExpBias, sl);
+    one = sl != kNoScaleLog2 && __all_sync(0xffffffffu, scale != 0.0);
   }
+  if (one) {
+    int cnt = tr.src_counts[b];
+    if (cnt > d.nq) {
+      if (lane == 0) report(st, VL1_E_LAYOUT, (int)b, cnt);
+      cnt = d.nq;
+    }
+    const int st0 = tr.src_starts[b];
+    const double *c = coefs + (int64_t)rh0 * tr.n_particles + st0;
+    double scu[G];
+#pragma unroll
+    for (int u = 0; u < G; ++u) scu[u] = __shfl_sync(0xffffffffu, scale, u);
+    for (int k = lane; k < cnt; k += 32) {
+      const int m = tr.smode[st0 + k];
+      double v[G];
+#pragma unroll
+      for (int u = 0; u < G; ++u) v[u] = c[u * tr.n_particles + k];
+      if ((unsigned)m >= (unsigned)d.nq) {
+        report(st, VL1_E_LAYOUT, (int)b, -1 - k);
+        continue;
+      }
+      const int pos = plane_position(m, kc_shift, kc);
+#pragma unroll
+      for (int u = 0; u < G; ++u) {
+        uint32_t p12, p3r;
+        plane_values_scaled(v[u], scu[u], p12, p3r);
+        store_planes(stage + u * row_bytes, pos, kc, p12, p3r);
+      }
+    }
+  } else {
+    // (A rows at a time: every row's state is in registers)
+#pragma unroll 1
+    for (int u0 = 0; u0 < n; u0 += A)
+      stage_planes<A>(d, tr, coefs, nrhs, x_exp, row_bytes, kc, kc_shift, st, r0 + u0,
+                      min(A, n - u0), lane, stage + u0 * row_bytes);
+  }
+  __syncwarp();
+  // (the group's rows lie one after the other, in the stage as in the planes)
+  uint8_t *const rows = reinterpret_cast<uint8_t *>(xpl) + r0 * row_bytes;
+  for (int k = lane * 16; k < n * row_bytes; k += 32 * 16)
+    *reinterpret_cast<uint4 *>(rows + k) = *reinterpret_cast<const uint4 *>(stage + k);
   __syncwarp();
 }
 
@@ -432,21 +556,22 @@ __global__ void x_exponent_kernel(DevDesc d, TreeDev tr, int nboxes, const doubl
   exp_block_end(nrhs, s_max, x_exp);
 }
 
-// dynamic shared memory: (blockDim.x / 32) x kPlaneGroup x kp * 8 bytes (kp a
-// multiple of 16, so every slice and row stays 16-byte aligned)
-__global__ void __launch_bounds__(128)
+// dynamic shared memory: (blockDim.x / 32) x G x kp * 8 bytes (kp a multiple
+// of 16, so every slice and row stays 16-byte aligned)
+template <int G>
+__global__ void __launch_bounds__(128, G == kPlaneGroupMany ? 8 : 6)
     x_planes_kernel(DevDesc d, TreeDev tr, int nboxes, const double *coefs, int nrhs,
                     const int *x_exp, __half *xpl, int kp, int kc, vl1_status *st) {
   extern __shared__ __align__(16) uint8_t s_stage[];
   const int64_t n = (int64_t)nboxes * nrhs;
   const int lane = threadIdx.x & 31;
-  uint8_t *stage = s_stage + (threadIdx.x >> 5) * kPlaneGroup * kp * kXPlanes * 2;
+  uint8_t *stage = s_stage + (threadIdx.x >> 5) * G * kp * kXPlanes * 2;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-       g * kPlaneGroup < n; g += warps) {
-    const int64_t r0 = g * kPlaneGroup;
-    group_planes<kPlaneGroup>(d, tr, coefs, nrhs, x_exp, xpl, kp, kc, st, r0,
-                              (int)min((int64_t)kPlaneGroup, n - r0), lane, stage);
+       g * G < n; g += warps) {
+    const int64_t r0 = g * G;
+    group_planes<G, G == kPlaneGroupMany ? 2 : G>(d, tr, coefs, nrhs, x_exp, xpl, kp, kc, st, r0,
+                                                  (int)min((int64_t)G, n - r0), lane, stage);
   }
 }
 
@@ -510,18 +635,19 @@ __global__ void x_exponent_batch_kernel(const PrepProblem *probs, const PrepTask
   exp_block_end(P.nrhs, s_max, P.x_exp);
 }
 
-// Dynamic shared memory: (blockDim.x / 32) x kPlaneGroup x (largest kp) * 8 bytes.
-__global__ void __launch_bounds__(128)
+// Dynamic shared memory: (blockDim.x / 32) x kBatchPlaneGroup x (largest kp) * 8 bytes.
+constexpr int kBatchPlaneGroup = 4;
+__global__ void __launch_bounds__(128, 6)
     x_planes_batch_kernel(const PrepProblem *probs, const PrepTask *tasks, int max_row_bytes) {
   extern __shared__ __align__(16) uint8_t s_stage[];
   const PrepTask t = tasks[blockIdx.x];
   const PrepProblem &P = probs[t.problem];
   const int lane = threadIdx.x & 31;
-  uint8_t *stage = s_stage + (threadIdx.x >> 5) * kPlaneGroup * max_row_bytes;
-  for (int i = (threadIdx.x >> 5) * kPlaneGroup; i < t.nrows;
-       i += (blockDim.x >> 5) * kPlaneGroup)
-    group_planes<kPlaneGroup>(P.d, P.tr, P.coefs, P.nrhs, P.x_exp, P.xpl, P.kp, P.kc, P.st,
-                              t.row0 + i, min(kPlaneGroup, t.nrows - i), lane, stage);
+  uint8_t *stage = s_stage + (threadIdx.x >> 5) * kBatchPlaneGroup * max_row_bytes;
+  for (int i = (threadIdx.x >> 5) * kBatchPlaneGroup; i < t.nrows;
+       i += (blockDim.x >> 5) * kBatchPlaneGroup)
+    group_planes<kBatchPlaneGroup, kBatchPlaneGroup>(P.d, P.tr, P.coefs, P.nrhs, P.x_exp, P.xpl, P.kp, P.kc, P.st,
+                                   t.row0 + i, min(kBatchPlaneGroup, t.nrows - i), lane, stage);
 }
 
 // 2D log displacement: w[b, r] = dispfac(b) * sum_s nmlz[lev(b), s] * coef
@@ -1731,14 +1857,17 @@ int32_t launch_mixed(vl1_plan *plan, const TreeDev &tree, int64_t nboxes,
     x_exponent_kernel<<<grid_for(n_groups * 32, 256), 256, 0, s>>>(d, tree, (int)nboxes,
                                                                   coefs, nrhs, x_exp);
   }
-  const size_t plane_smem = (size_t)4 * kPlaneGroup * g.kp * kXPlanes * 2;
+  const bool many = g.kp <= 32 && nrhs >= kPlaneManyRhs;
+  const int group = many ? kPlaneGroupMany : kPlaneGroup;
+  const auto planes = many ? x_planes_kernel<kPlaneGroupMany> : x_planes_kernel<kPlaneGroup>;
+  const size_t plane_smem = (size_t)4 * group * g.kp * kXPlanes * 2;
   if (plane_smem > 48 * 1024) {
-    e = cudaFuncSetAttribute(x_planes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(planes, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)plane_smem);
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(x_planes_kernel)");
   }
-  const int64_t n_plane_groups = (nbr + kPlaneGroup - 1) / kPlaneGroup;
-  x_planes_kernel<<<grid_for(n_plane_groups * 32, 128), 128, plane_smem, s>>>(
+  const int64_t n_plane_groups = (nbr + group - 1) / group;
+  planes<<<grid_for(n_plane_groups * 32, 128), 128, plane_smem, s>>>(
       d, tree, (int)nboxes, coefs, nrhs, x_exp, xpl, g.kp, g.kc, plan->status);
   if (disp) {
     disp_box_kernel<<<grid_for(nbr, 256), 256, 0, s>>>(d, tree, (int)nboxes, coefs, nrhs,
@@ -2264,7 +2393,7 @@ extern "C" int32_t vl1_batch_eval(vl1_batch *b, void *stream) {
   if (b->n_tasks > 0) {
     x_exponent_batch_kernel<<<b->n_tasks, 256, 0, s>>>(
         static_cast<const PrepProblem *>(b->d_prep), static_cast<const PrepTask *>(b->d_tasks));
-    const size_t plane_smem = (size_t)4 * kPlaneGroup * b->max_row_bytes;
+    const size_t plane_smem = (size_t)4 * kBatchPlaneGroup * b->max_row_bytes;
     if (plane_smem > 48 * 1024) {
       e = cudaFuncSetAttribute(x_planes_batch_kernel,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem);

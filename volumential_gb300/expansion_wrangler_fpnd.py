@@ -84,8 +84,8 @@ def _normalize_term_key(key):
     return kind, power
 
 
-def _compute_box_local_ids(tree, n_q_points):
-    """Box-local particle index of every particle, in tree order."""
+def _check_box_local_ids(tree, n_q_points):
+    """The particle count, after the checks of ``_compute_box_local_ids``."""
     if not getattr(tree, "sources_are_targets", False):
         raise ValueError(
             "table-based near-field evaluation requires sources and targets "
@@ -93,8 +93,33 @@ def _compute_box_local_ids(tree, n_q_points):
     n = int(tree.ntargets)
     if n % n_q_points != 0:
         raise ValueError("particle count is not divisible by box-local quadrature size")
+    return n
+
+
+def _identity_order(tree):
+    """Whether the tree's particle order is the user's (``ParticleTree``)."""
+    from .tree_build import ParticleTree
+    t = type(tree)
+    return (getattr(t, "sorted_target_ids", None) is ParticleTree.sorted_target_ids
+            and getattr(t, "user_source_ids", None) is ParticleTree.user_source_ids)
+
+
+def _compute_box_local_ids(tree, n_q_points):
+    """Box-local particle index of every particle, in tree order."""
+    n = _check_box_local_ids(tree, n_q_points)
     local = np.tile(np.arange(n_q_points, dtype=np.int32), n // n_q_points)
-    return local[_np(tree.sorted_target_ids)]
+    return local if _identity_order(tree) else local[_np(tree.sorted_target_ids)]
+
+
+def _leading(x, n, fresh=False):
+    """``x[..., arange(n)]``, a new tensor (``fresh``: x itself is one)."""
+    import torch
+
+    if x.shape[-1] < n:
+        raise IndexError(f"array of {x.shape[-1]} entries for {n} particles")
+    if fresh and x.shape[-1] == n:
+        return x
+    return x[..., :n].clone(memory_format=torch.contiguous_format)
 
 
 def _validate_table_box_particle_layout(tree, target_boxes, source_boxes, n_q_points):
@@ -285,6 +310,7 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
         self.kernel_extra_kwargs = kernel_extra_kwargs or {}
         self.self_extra_kwargs = self_extra_kwargs or {}
         self.list1_extra_kwargs = dict(list1_extra_kwargs or {})
+        self._local_ids = {}   # see _device_local_ids
 
         knames = [repr(k) for k in tree_indep.target_kernels]
         if isinstance(near_field_table, dict):
@@ -451,7 +477,8 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
         vals = []
         for part in parts:
             kw = self._near_field_kwargs(payload, target_boxes, starts, lists,
-                                         part.to(torch.float64).contiguous())
+                                         part.to(torch.float64).contiguous(),
+                                         self._device_local_ids(payload))
             res = torch.zeros(int(self.tree.ntargets), dtype=torch.float64, device="cuda")
             res, _ = near_field(self.queue, result=res, **kw)
             vals.append(res)
@@ -523,9 +550,10 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
         out, events = [], []
         r_max = max_neighbor_distance(self.tree)
         for k in self.tree_indep.target_kernels:
-            kw = self._near_field_kwargs(self.get_payload(k), target_boxes,
-                                         neighbor_source_boxes_starts,
-                                         neighbor_source_boxes_lists, None)
+            payload = self.get_payload(k)
+            kw = self._near_field_kwargs(payload, target_boxes, neighbor_source_boxes_starts,
+                                         neighbor_source_boxes_lists, None,
+                                         self._device_local_ids(payload))
             view, keep = tree_view_from_arrays(**{n: kw[n] for n in (
                 "target_boxes", "neighbor_source_boxes_starts", "neighbor_source_boxes_lists",
                 "box_centers", "box_levels", "box_source_starts",
@@ -636,10 +664,31 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
             self._payload_cache.popitem(last=False)
         return payload
 
-    def _near_field_kwargs(self, payload, target_boxes, starts, lists, mode_coefs):
+    def _device_local_ids(self, payload):
+        """``_compute_box_local_ids`` for an evaluation: on the device when the
+        particle order is the user's (the ids are then i mod q^d: computed
+        there, and kept per (count, q^d))."""
+        import torch
+
+        nq = int(payload["table_data_shapes"]["n_q_points"])
+        n = _check_box_local_ids(self.tree, nq)
+        if (not _identity_order(self.tree) or not torch.cuda.is_available()
+                or torch.cuda.is_current_stream_capturing()):
+            return _compute_box_local_ids(self.tree, nq)
+        ids = self._local_ids.get((n, nq))
+        if ids is None:
+            ids = torch.arange(n, dtype=torch.int32, device="cuda").remainder_(nq)
+            torch.cuda.current_stream().synchronize()   # read on any stream
+            if len(self._local_ids) >= 4:
+                self._local_ids.clear()
+            self._local_ids[n, nq] = ids
+        return ids
+
+    def _near_field_kwargs(self, payload, target_boxes, starts, lists, mode_coefs, local=None):
         tree = self.tree
         nq = payload["table_data_shapes"]["n_q_points"]
-        local = _compute_box_local_ids(tree, nq)
+        if local is None:
+            local = _compute_box_local_ids(tree, nq)
         key = (id(target_boxes), id(lists), nq)
         if key not in self._layout_validated:
             _validate_table_box_particle_layout(tree, target_boxes, lists, nq)
@@ -701,7 +750,8 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
                     f"{min_lev} are not covered.")
         near_field = self.near_field_evaluator(out_kernel, payload, list1_extra_kwargs)
         kw = self._near_field_kwargs(payload, target_boxes, neighbor_source_boxes_starts,
-                                     neighbor_source_boxes_lists, mode_coefs)
+                                     neighbor_source_boxes_lists, mode_coefs,
+                                     self._device_local_ids(payload))
         if self.helmholtz_split and out_pot.is_complex():
             import torch
 
@@ -754,7 +804,8 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
             payload = self.get_payload(k)
             nf = self.near_field_evaluator(k, payload)
             kw = self._near_field_kwargs(payload, target_boxes, neighbor_source_boxes_starts,
-                                         neighbor_source_boxes_lists, None)
+                                         neighbor_source_boxes_lists, None,
+                                         self._device_local_ids(payload))
             plan = nf.get_plan(
                 table_data_combined=kw["table_data_combined"],
                 mode_nmlz_combined=kw["mode_nmlz_combined"], case_indices=kw["case_indices"],
@@ -808,6 +859,8 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
     def reorder_sources(self, source_array):
         from .plan import as_device_tensor
         x = as_device_tensor(source_array)
+        if _identity_order(self.tree):
+            return _leading(x, int(self.tree.nsources), fresh=x is not source_array)
         idx = as_device_tensor(_np(self.tree.user_source_ids).astype(np.int64))
         return x[..., idx]
 
@@ -816,6 +869,8 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
 
     def reorder_potentials(self, potentials):
         from .plan import as_device_tensor
+        if _identity_order(self.tree):
+            return [_leading(p, int(self.tree.ntargets)) for p in potentials]
         idx = as_device_tensor(_np(self.tree.sorted_target_ids).astype(np.int64))
         return [p[..., idx] for p in potentials]
 

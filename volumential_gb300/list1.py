@@ -248,7 +248,7 @@ def _array_token(ary):
         return ("t", int(ary.data_ptr()), int(getattr(ary, "_version", 0)),
                 tuple(ary.shape), str(ary.dtype))
     if isinstance(ary, np.ndarray):
-        return ("np", int(ary.ctypes.data), tuple(ary.shape), ary.dtype.str)
+        return ("np", ary.__array_interface__["data"][0], ary.shape, ary.dtype.str)
     return ("py", id(ary))
 
 

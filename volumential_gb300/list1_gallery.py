@@ -35,25 +35,16 @@ def touching_vectors(dim: int) -> list[tuple[int, ...]]:
     if dim < 1:
         raise ValueError("dim must be positive")
 
-    boxes = []  # (center vector, half width)
-    for level in range(4):
-        width = 16 >> level
-        half = width // 2
-        ticks = np.arange(half, 16, width)
-        for center in itertools.product(ticks.tolist(), repeat=dim):
-            boxes.append((np.asarray(center, dtype=np.int64), half))
+    def centers(half, lo, hi):
+        ticks = [t for t in range(half, 16, 2 * half) if lo < t < hi]
+        return np.array(list(itertools.product(ticks, repeat=dim)), dtype=np.int64)
 
-    targets = [
-        (c, h) for c, h in boxes
-        if h == 2 and int(c.min()) > 2 and int(c.max()) < 14
-    ]
-
+    targets = centers(2, 2, 14)
     vecs = {tuple([0] * dim)}
-    for tc, th in targets:
-        for sc, sh in boxes:
-            gap = int(np.max(np.abs(tc - sc) - (th + sh)))
-            if gap == 0:
-                vecs.add(tuple(int(v) for v in (tc - sc)))
+    for half in (8, 4, 2, 1):
+        diff = targets[:, None, :] - centers(half, -1, 17)[None, :, :]
+        touch = np.max(np.abs(diff), axis=-1) == 2 + half
+        vecs.update(map(tuple, diff[touch].tolist()))
     return sorted(vecs)
 
 

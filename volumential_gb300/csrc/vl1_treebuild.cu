@@ -56,34 +56,39 @@ __global__ void tb_hash_leaves_kernel(int dim, int n, const uint8_t *levels,
   }
 }
 
+// x / 2^level: the product with 2^-level rounds the same way (levels here are
+// at most 30)
+__device__ __forceinline__ double exact_scale(double x, int level) {
+  return __dmul_rn(x, __longlong_as_double((long long)(1023 - level) << 52));
+}
+
 // flag[j] = 1 for every leaf j at a level below L - 1 that contains a
 // same-level neighbour position of a leaf at level L
 __global__ void tb_mark_kernel(int dim, int n, const uint8_t *levels, const int32_t *coords,
                                KeyHash h, int32_t *flag, int32_t *n_flagged) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x) {
+  // a thread per (leaf, neighbour position): a leaf's look-ups are chains of
+  // dependent loads, and 27 of them in one thread took 79 us for 23,000 leaves
+  const int n3 = dim == 3 ? 27 : 9;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < (int64_t)n * n3;
+       t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = t / n3;
+    int rem = (int)(t - i * n3);
     const int lev = levels[i];
     if (lev < 2) continue;
-    long long c[3];
-    for (int a = 0; a < dim; ++a) c[a] = coords[i * dim + a];
     const long long side = 1ll << lev;
-    const int n3 = dim == 3 ? 27 : 9;
-    for (int di = 0; di < n3; ++di) {
-      long long pos[3];
-      bool valid = true;
-      int rem = di;
-      for (int a = dim - 1; a >= 0; --a) {
-        pos[a] = c[a] + (rem % 3 - 1);
-        rem /= 3;
-        valid = valid && pos[a] >= 0 && pos[a] < side;
-      }
-      if (!valid) continue;
-      for (int coarse = 0; coarse < lev - 1; ++coarse) {
-        long long anc[3];
-        for (int a = 0; a < dim; ++a) anc[a] = pos[a] >> (lev - coarse);
-        const int j = h.find(box_key(dim, coarse, anc));
-        if (j >= 0 && atomicExch(flag + j, 1) == 0) atomicAdd(n_flagged, 1);
-      }
+    long long pos[3];
+    bool valid = true;
+    for (int a = dim - 1; a >= 0; --a) {
+      pos[a] = coords[i * dim + a] + (rem % 3 - 1);
+      rem /= 3;
+      valid = valid && pos[a] >= 0 && pos[a] < side;
+    }
+    if (!valid) continue;
+    for (int coarse = 0; coarse < lev - 1; ++coarse) {
+      long long anc[3];
+      for (int a = 0; a < dim; ++a) anc[a] = pos[a] >> (lev - coarse);
+      const int j = h.find(box_key(dim, coarse, anc));
+      if (j >= 0 && atomicExch(flag + j, 1) == 0) atomicAdd(n_flagged, 1);
     }
   }
 }
@@ -173,7 +178,7 @@ __global__ void tb_boxes_kernel(BoxOut B) {
     // extent = root_extent / 2^lev; centre = vertex + (coord + 0.5) * extent
     // (the host builder's operations, in its order)
     // (separately rounded operations: no contraction into fused multiply-adds)
-    const double ext = __ddiv_rn(B.root_extent, (double)(1ll << lev));
+    const double ext = exact_scale(B.root_extent, lev);
     for (int a = 0; a < B.dim; ++a) {
       B.coords[b * B.dim + a] = (int32_t)c[a];
       B.centers[a * B.aligned + b] =
@@ -206,7 +211,7 @@ __global__ void tb_particles_kernel(Particles P) {
     const int j = (int)(idx - i * P.nq);
     const int b = P.leaf_boxes[i];
     // centre + (0.5 * extent) * node, separately rounded (the host's order)
-    const double ext = __ddiv_rn(P.root_extent, (double)(1ll << P.levels[b]));
+    const double ext = exact_scale(P.root_extent, P.levels[b]);
     const double half = __dmul_rn(0.5, ext);
     const int64_t N = (int64_t)P.n_leaves * P.nq;
     for (int a = 0; a < P.dim; ++a)
@@ -293,7 +298,7 @@ int32_t balance(int dim, int32_t *n_leaves, int capacity, uint8_t *levels, int32
     cudaMemsetAsync(flag, 0, 4 * (size_t)n, s);
     cudaMemsetAsync(ctr, 0, 16, s);
     tb_hash_leaves_kernel<<<tb_grid(n), kTB, 0, s>>>(dim, n, levels, coords, h, ctr + 2);
-    tb_mark_kernel<<<tb_grid(n), kTB, 0, s>>>(dim, n, levels, coords, h, flag, ctr);
+    tb_mark_kernel<<<tb_grid((int64_t)n * 27), kTB, 0, s>>>(dim, n, levels, coords, h, flag, ctr);
     if ((e = cudaMemcpyAsync(host, ctr, 16, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess) {
       release();

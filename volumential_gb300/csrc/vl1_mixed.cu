@@ -623,7 +623,11 @@ __global__ void __launch_bounds__(128)
 
 // Batch versions: block i handles rows [row0, row0 + nrows) of one problem
 // (tasks built on the host), its warps taking groups of rows.
-__global__ void x_exponent_batch_kernel(const PrepProblem *probs, const PrepTask *tasks) {
+// (64 registers each, so that more warps hide the rows' dependent loads: on
+// eight 3D problems of 240,000 rows together 57 -> 44 us and, with the rows of
+// mixed boxes two at a time, 92 -> 83 us.)
+__global__ void __launch_bounds__(256, 4)
+    x_exponent_batch_kernel(const PrepProblem *probs, const PrepTask *tasks) {
   __shared__ int s_max[kExpSmemRhs];
   const PrepTask t = tasks[blockIdx.x];
   const PrepProblem &P = probs[t.problem];
@@ -637,7 +641,7 @@ __global__ void x_exponent_batch_kernel(const PrepProblem *probs, const PrepTask
 
 // Dynamic shared memory: (blockDim.x / 32) x kBatchPlaneGroup x (largest kp) * 8 bytes.
 constexpr int kBatchPlaneGroup = 4;
-__global__ void __launch_bounds__(128, 6)
+__global__ void __launch_bounds__(128, 8)
     x_planes_batch_kernel(const PrepProblem *probs, const PrepTask *tasks, int max_row_bytes) {
   extern __shared__ __align__(16) uint8_t s_stage[];
   const PrepTask t = tasks[blockIdx.x];
@@ -646,7 +650,7 @@ __global__ void __launch_bounds__(128, 6)
   uint8_t *stage = s_stage + (threadIdx.x >> 5) * kBatchPlaneGroup * max_row_bytes;
   for (int i = (threadIdx.x >> 5) * kBatchPlaneGroup; i < t.nrows;
        i += (blockDim.x >> 5) * kBatchPlaneGroup)
-    group_planes<kBatchPlaneGroup, kBatchPlaneGroup>(P.d, P.tr, P.coefs, P.nrhs, P.x_exp, P.xpl, P.kp, P.kc, P.st,
+    group_planes<kBatchPlaneGroup, 2>(P.d, P.tr, P.coefs, P.nrhs, P.x_exp, P.xpl, P.kp, P.kc, P.st,
                                    t.row0 + i, min(kBatchPlaneGroup, t.nrows - i), lane, stage);
 }
 

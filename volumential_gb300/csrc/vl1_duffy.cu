@@ -25,11 +25,14 @@
 // FMA per k and node), then turned into all q modes through their values at
 // r_0 .. r_{d-2} xi_k.  Per node: the distance, one kernel value and q FMAs,
 // against the kernel value and d (q - 1) products per node *and entry* of
-// duffy_entry_kernel.
+// duffy_entry_kernel.  Every FP64 operation of a node counts: the kernel's
+// constant factor and the basis' weights multiply the sums instead, and the
+// test for a zero distance is an integer one (3D Laplace q = 4: 12.3 -> 10.8
+// ms a build).
 //
 // Measured (GB300, default orders, whole build calls): 3D Laplace q = 4
-// (12,936 entries, 636 targets) 370 -> 12 ms, 3D Helmholtz q = 4 604 -> 32 ms,
-// 2D Helmholtz q = 5 4.3 -> 1.3 ms; entries within 1e-15 of the per-entry
+// (12,936 entries, 636 targets) 370 -> 10.5 ms, 3D Helmholtz q = 4 604 -> 30 ms,
+// 2D Helmholtz q = 5 4.4 -> 1.4 ms; entries within 1e-15 of the per-entry
 // sums, relative to the largest.
 //
 // duffy_entry_kernel (plane waves, derivatives, q beyond the instances): one
@@ -318,16 +321,23 @@ __global__ void duffy_reduce_kernel(const double *part, int n_entries, int n_chu
 
 // ---------------------------------------------- all modes of a target
 
-// G(r) times the kernel's scaling constant for the radial kernels
+// G(r) for the radial kernels, up to the factor green_factor(kind), which the
+// group kernel applies once per sum instead of once per node
+__host__ __device__ constexpr double green_factor(int kind) {
+  return kind == VL1_DUFFY_LAPLACE2D ? -0.25 / 3.141592653589793
+         : kind == VL1_DUFFY_LAPLACE3D || kind == VL1_DUFFY_HELMHOLTZ3D
+             ? 0.25 / 3.141592653589793
+             : 1.0;
+}
 __device__ __forceinline__ void green_radial(int kind, double k, int power, double r2,
                                              double &re, double &im) {
   im = 0.0;
   switch (kind) {
-    case VL1_DUFFY_LAPLACE2D:   // -log(r) / (2 pi)
-      re = -0.5 * log(r2) * (0.5 / 3.141592653589793);
+    case VL1_DUFFY_LAPLACE2D:   // -log(r) / (2 pi) = -log(r^2) / (4 pi)
+      re = log(r2);
       break;
     case VL1_DUFFY_LAPLACE3D:   // 1 / (4 pi r)
-      re = rsqrt(r2) * (0.25 / 3.141592653589793);
+      re = rsqrt(r2);
       break;
     case VL1_DUFFY_HELMHOLTZ2D: {
       const double kr = k * sqrt(r2);
@@ -335,11 +345,11 @@ __device__ __forceinline__ void green_radial(int kind, double k, int power, doub
       im = 0.25 * j0(kr);
       break;
     }
-    case VL1_DUFFY_HELMHOLTZ3D: {
+    case VL1_DUFFY_HELMHOLTZ3D: {   // exp(i k r) / (4 pi r)
       const double r = sqrt(r2);
       double s, c;
       sincos(k * r, &s, &c);
-      const double f = (0.25 / 3.141592653589793) / r;
+      const double f = 1.0 / r;
       re = c * f;
       im = s * f;
       break;
@@ -357,22 +367,25 @@ __device__ __forceinline__ void green_radial(int kind, double k, int power, doub
   }
 }
 
-// values of the Q Lagrange polynomials on the nodes x at y (first form,
-// products from the left and from the right)
+// The Q Lagrange polynomials on the nodes x at y without their weights (the
+// products of the differences to the other nodes, from the left and from the
+// right; the weights are applied once per sum).
 template <int Q>
-__device__ __forceinline__ void lagrange_values(double y, const double *x, const double *bw,
-                                                double (&l)[Q]) {
+__device__ __forceinline__ void node_products(double y, const double *x, double (&l)[Q]) {
+  double d[Q];
+#pragma unroll
+  for (int m = 0; m < Q; ++m) d[m] = y - x[m];
   double left = 1.0;
 #pragma unroll
   for (int m = 0; m < Q; ++m) {
-    l[m] = bw[m] * left;
-    left *= y - x[m];
+    l[m] = left;
+    left = m == 0 ? d[0] : left * d[m];
   }
   double right = 1.0;
 #pragma unroll
   for (int m = Q - 1; m >= 0; --m) {
-    l[m] *= right;
-    right *= y - x[m];
+    l[m] = m == Q - 1 ? l[m] : (m == 0 ? right : l[m] * right);
+    right = m == Q - 1 ? d[m] : right * d[m];
   }
 }
 
@@ -481,7 +494,9 @@ __global__ void __launch_bounds__(kGroupThreads) duffy_group_kernel(const DuffyG
             const double d2 = fma(-c, s_r[j2], b[DIM - 1]);
             const double r2 = fma(d2, d2, base);
             double gre = 0.0, gim = 0.0;
-            if (r2 > 0.0) green_radial(D.kernel, D.k, D.power, r2, gre, gim);
+            // r2 > 0 (a sum of squares), tested off the FP64 pipe
+            if ((unsigned long long)(__double_as_longlong(r2) - 1ll) < 0x7FF0000000000000ull)
+              green_radial(D.kernel, D.k, D.power, r2, gre, gim);
 #pragma unroll
             for (int k = 0; k < Q; ++k) {
               mom[k * CV] = fma(gre, s_phi[j2 * Q + k], mom[k * CV]);
@@ -495,7 +510,7 @@ __global__ void __launch_bounds__(kGroupThreads) duffy_group_kernel(const DuffyG
 #pragma unroll
           for (int k = 0; k < Q; ++k) {
             double l[Q];
-            lagrange_values<Q>(fma(c, s_xi[k], dc[DIM - 1]), s_x, s_bw, l);
+            node_products<Q>(fma(c, s_xi[k], dc[DIM - 1]), s_x, l);
 #pragma unroll
             for (int m = 0; m < Q; ++m) {
               tm[m * CV] = fma(l[m], mom[k * CV], tm[m * CV]);
@@ -504,7 +519,7 @@ __global__ void __launch_bounds__(kGroupThreads) duffy_group_kernel(const DuffyG
           }
           if (DIM == 3) {
             double l[Q];
-            lagrange_values<Q>(fma(s[1], a, dc[1]), s_x, s_bw, l);
+            node_products<Q>(fma(s[1], a, dc[1]), s_x, l);
             const double w1 = s_w[j1] * s_r[j1];
 #pragma unroll
             for (int m1 = 0; m1 < Q; ++m1) {
@@ -520,7 +535,7 @@ __global__ void __launch_bounds__(kGroupThreads) duffy_group_kernel(const DuffyG
         }
       }
       double l[Q];
-      lagrange_values<Q>(fma(s[0], r0, dc[0]), s_x, s_bw, l);
+      node_products<Q>(fma(s[0], r0, dc[0]), s_x, l);
       const double w0 = i < D.n_rad ? D.radial_weights[i] * len_prod *
                                           (DIM == 3 ? r0 * r0 : r0)
                                     : 0.0;
@@ -548,15 +563,17 @@ __global__ void __launch_bounds__(kGroupThreads) duffy_group_kernel(const DuffyG
       if (m < NM) {
         // simplex order (m0, m1, (m2)) to axis order, axis 0 slowest
         int rest = m / CV, mode = 0;
+        double factor = green_factor(D.kernel);
 #pragma unroll
         for (int i = DIM - 1; i >= 0; --i) {
           const int a = DIM == 3 ? kPerm3[iperm][i] : kPerm2[iperm][i];
           int stride = 1;
           for (int x = a; x < DIM - 1; ++x) stride *= Q;
           mode += (rest % Q) * stride;
+          factor *= s_bw[rest % Q];
           rest /= Q;
         }
-        part[mode * CV + m % CV] = sum[o];
+        part[mode * CV + m % CV] = sum[o] * factor;
       }
     }
   }

@@ -35,8 +35,8 @@
 // densities, densities over 6 and 200 decades) the relative l2 error is
 // 4e-17 .. 2e-16, the per-box kernel's 1e-16 .. 2e-15.
 //
-// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 236 us here
-// (digits 22 us, tensor-core kernel 208 us, its tensor pipe busy 105 us of
+// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 233 us here
+// (digits 22 us, tensor-core kernel 206 us, its tensor pipe busy 105 us of
 // them); 3D q = 5, 512,000 points 3,240 and 168 us; 3D q = 3, 110,592 points
 // x 8 right-hand sides 1,530 and 131 us; 2D complex q = 5, 102,400 points 185
 // and 46 us.  Bound: shared memory (per unit 120 KB of operand reads and 48 KB
@@ -1044,18 +1044,23 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
   const vl1_mixed_item item = s_item;
   bool write = !s_abort && item.tile >= 0;
   if (item.split >= 0) {
-    longlong2 *mine = p.partials + ((int64_t)item.slot * n_chunks + chunk) * 128 * NCH;
-    if (!s_abort)
+    // (a part that finds all others done keeps its sums in shared memory:
+    // storing a part takes 17,000 clocks with every SM at it; 236 -> 233 us)
+    int *const ctr = p.counters + (int64_t)item.split * n_chunks + chunk;
+    if (tid == 0) s_last = (atomicAdd(ctr, 0) & 0xFFFF) == item.nparts - 1;
+    __syncthreads();
+    if (!s_abort && !s_last) {
+      longlong2 *mine = p.partials + ((int64_t)item.slot * n_chunks + chunk) * 128 * NCH;
       for (int i = tid; i < 128 * NCH; i += R::kThreads) {
         const int o = (i / NCH) * PARK + i % NCH;
         mine[i] = make_longlong2(s_S[o], s_L[o]);
       }
+    }
     __threadfence();
     __syncthreads();
     if (tid == 0) {
       const int inc = s_abort ? (1 << 16) + 1 : 1;
-      const int done =
-          atomicAdd(p.counters + (int64_t)item.split * n_chunks + chunk, inc) + inc;
+      const int done = atomicAdd(ctr, inc) + inc;
       s_last = (done & 0xFFFF) == item.nparts;
       s_poison = done >> 16;
     }
@@ -1070,6 +1075,7 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
       for (int i0 = tid; i0 < 128 * NCH; i0 += BATCH * R::kThreads) {
         long long S[BATCH] = {}, L[BATCH] = {};
         for (int q = 0; q < item.nparts; ++q) {
+          if (q == item.part) continue;   // in shared memory
           longlong2 v[BATCH];
 #pragma unroll
           for (int c = 0; c < BATCH; ++c) {
@@ -1086,8 +1092,8 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
         for (int c = 0; c < BATCH; ++c) {
           const int i = i0 + c * R::kThreads;
           if (i < 128 * NCH) {
-            s_S[(i / NCH) * PARK + i % NCH] = S[c];
-            s_L[(i / NCH) * PARK + i % NCH] = L[c];
+            s_S[(i / NCH) * PARK + i % NCH] += S[c];
+            s_L[(i / NCH) * PARK + i % NCH] += L[c];
           }
         }
       }

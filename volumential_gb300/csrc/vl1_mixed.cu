@@ -543,6 +543,7 @@ __device__ __forceinline__ void group_planes(const DevDesc &d, const TreeDev &tr
 __global__ void x_exponent_kernel(DevDesc d, TreeDev tr, int nboxes, const double *coefs,
                                   int nrhs, int *x_exp) {
   __shared__ int s_max[kExpSmemRhs];
+  grid_dep_launch();
   exp_block_begin(nrhs, s_max);
   const int64_t n = (int64_t)nboxes * nrhs;
   const int lane = threadIdx.x & 31;
@@ -563,6 +564,8 @@ __global__ void __launch_bounds__(128, G == kPlaneGroupMany ? 8 : 6)
     x_planes_kernel(DevDesc d, TreeDev tr, int nboxes, const double *coefs, int nrhs,
                     const int *x_exp, __half *xpl, int kp, int kc, vl1_status *st) {
   extern __shared__ __align__(16) uint8_t s_stage[];
+  grid_dep_launch();
+  grid_dep_wait();   // the exponents
   const int64_t n = (int64_t)nboxes * nrhs;
   const int lane = threadIdx.x & 31;
   uint8_t *stage = s_stage + (threadIdx.x >> 5) * G * kp * kXPlanes * 2;
@@ -578,16 +581,17 @@ __global__ void __launch_bounds__(128, G == kPlaneGroupMany ? 8 : 6)
 // The exponent pass for small boxes (nq <= 32) with several rhs: rows in row
 // order put one box's rhs next to each other, whose densities lie
 // n_particles values apart, so the row-group pass reads scattered 8 * nq-byte
-// pieces (C3: 210 MB at ~1.9 TB/s).  Here a warp takes one rhs of 32
+// pieces (210 MB of 25-point boxes at ~1.9 TB/s).  Here a warp takes one rhs of 32
 // consecutive boxes.  When their points follow one another and they have one
 // level (equal scaling), the maximum of |c| bits is taken over the whole
 // range, 32 neighbouring values a load; otherwise one lane per box, its values
-// one after the other (63 us on C3, 44 us with whole ranges).  One multiply, the
+// one after the other (63 us for those 210 MB, 44 us with whole ranges).  One multiply, the
 // maximum over the warp, one shared-memory maximum per warp.
 __global__ void __launch_bounds__(128)
     x_exponent_small_kernel(DevDesc d, TreeDev tr, int nboxes, const double *coefs, int nrhs,
                             int *x_exp) {
   __shared__ int s_max[kExpSmemRhs];
+  grid_dep_launch();
   exp_block_begin(nrhs, s_max);
   const int lane = threadIdx.x & 31;
   const int64_t n_tiles = (int64_t)((nboxes + 31) / 32) * nrhs;   // (32 boxes, one rhs)
@@ -649,6 +653,7 @@ __global__ void __launch_bounds__(128)
 __global__ void __launch_bounds__(256, 4)
     x_exponent_batch_kernel(const PrepProblem *probs, const PrepTask *tasks) {
   __shared__ int s_max[kExpSmemRhs];
+  grid_dep_launch();
   const PrepTask t = tasks[blockIdx.x];
   const PrepProblem &P = probs[t.problem];
   exp_block_begin(P.nrhs, s_max);
@@ -664,6 +669,8 @@ constexpr int kBatchPlaneGroup = 4;
 __global__ void __launch_bounds__(128, 8)
     x_planes_batch_kernel(const PrepProblem *probs, const PrepTask *tasks, int max_row_bytes) {
   extern __shared__ __align__(16) uint8_t s_stage[];
+  grid_dep_launch();
+  grid_dep_wait();   // the exponents
   const PrepTask t = tasks[blockIdx.x];
   const PrepProblem &P = probs[t.problem];
   const int lane = threadIdx.x & 31;
@@ -1111,6 +1118,7 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
     tc::tmem_alloc(&tmem_base, COLS);
     tc::tmem_relinquish();
   }
+  grid_dep_wait();   // the digit planes
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -1740,7 +1748,7 @@ cudaError_t launch_mixed_kernel(int nch, int kc, bool multi, dim3 grid, cudaStre
                                        (int)smem);
   if (e != cudaSuccess) return e;
   void *args[] = {const_cast<MixedParams *>(&mp), const_cast<BatchLaunch *>(&bl)};
-  return cudaLaunchKernel(fn, grid, dim3(mixed_threads(nch)), args, smem, s);
+  return launch_overlapped(fn, grid, dim3(mixed_threads(nch)), args, smem, s);
 }
 
 int grid_for(int64_t n, int threads) {
@@ -1891,8 +1899,18 @@ int32_t launch_mixed(vl1_plan *plan, const TreeDev &tree, int64_t nboxes,
     if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(x_planes_kernel)");
   }
   const int64_t n_plane_groups = (nbr + group - 1) / group;
-  planes<<<grid_for(n_plane_groups * 32, 128), 128, plane_smem, s>>>(
-      d, tree, (int)nboxes, coefs, nrhs, x_exp, xpl, g.kp, g.kc, plan->status);
+  {
+    int nb = (int)nboxes, kp = g.kp, kc = g.kc;
+    const int *xe = x_exp;
+    vl1_status *st = plan->status;
+    DevDesc dd = d;
+    TreeDev tr = tree;
+    void *args[] = {&dd, &tr, &nb, &coefs, &nrhs, &xe, &xpl, &kp, &kc, &st};
+    e = launch_overlapped(reinterpret_cast<const void *>(planes),
+                          dim3(grid_for(n_plane_groups * 32, 128)), dim3(128), args, plane_smem,
+                          s);
+    if (e != cudaSuccess) return cuda_fail(e, "x_planes_kernel launch");
+  }
   if (disp) {
     disp_box_kernel<<<grid_for(nbr, 256), 256, 0, s>>>(d, tree, (int)nboxes, coefs, nrhs,
                                                       wbox);
@@ -2424,9 +2442,12 @@ extern "C" int32_t vl1_batch_eval(vl1_batch *b, void *stream) {
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plane_smem);
       if (e != cudaSuccess) return cuda_fail(e, "cudaFuncSetAttribute(x_planes_batch_kernel)");
     }
-    x_planes_batch_kernel<<<b->n_tasks, 128, plane_smem, s>>>(
-        static_cast<const PrepProblem *>(b->d_prep), static_cast<const PrepTask *>(b->d_tasks),
-        b->max_row_bytes);
+    const void *prep = b->d_prep, *tasks = b->d_tasks;
+    int row_bytes = b->max_row_bytes;
+    void *args[] = {&prep, &tasks, &row_bytes};
+    e = launch_overlapped(reinterpret_cast<const void *>(&x_planes_batch_kernel),
+                          dim3(b->n_tasks), dim3(128), args, plane_smem, s);
+    if (e != cudaSuccess) return cuda_fail(e, "x_planes_batch_kernel launch");
   }
   if (b->has_disp && b->n_tasks > 0) {
     disp_box_batch_kernel<<<b->n_tasks, 64, 0, s>>>(static_cast<const PrepProblem *>(b->d_prep),

@@ -35,11 +35,11 @@
 // densities, densities over 6 and 200 decades) the relative l2 error is
 // 4e-17 .. 2e-16, the per-box kernel's 1e-16 .. 2e-15.
 //
-// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 233 us here
+// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 229 us here
 // (digits 22 us, tensor-core kernel 206 us, its tensor pipe busy 105 us of
-// them); 3D q = 5, 512,000 points 3,240 and 168 us; 3D q = 3, 110,592 points
-// x 8 right-hand sides 1,530 and 131 us; 2D complex q = 5, 102,400 points 185
-// and 46 us.  Bound: shared memory (per unit 120 KB of operand reads and 48 KB
+// them); 3D q = 5, 512,000 points 3,240 and 167 us; 3D q = 3, 110,592 points
+// x 8 right-hand sides 1,530 and 127 us; 2D complex q = 5, 102,400 points 185
+// and 43 us.  Bound: shared memory (per unit 120 KB of operand reads and 48 KB
 // of stores, 1,350 of the ~1,750 clocks) and the L2's delivery to all SMs (36
 // KB at ~30 bytes per SM and clock, 1,200), close behind them the tensor pipe
 // (1,176); per work item ~12 us of start and result write.
@@ -231,6 +231,7 @@ constexpr int kPrepRows = 4;   // rows per warp and pass: their loads overlap
 // planes (256 bytes a row and unit).
 __global__ void __launch_bounds__(128) wide_prep_kernel(const __grid_constant__ WidePrep P) {
   extern __shared__ __align__(16) uint8_t s_stage[];
+  grid_dep_launch();
   const DevDesc &d = P.d;
   const TreeDev &tr = P.tr;
   const int lane = threadIdx.x & 31;
@@ -658,6 +659,7 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
     s_E[tid] = kZeroExp;
     s_bad[tid] = 0;
   }
+  grid_dep_wait();   // the density digits, their exponents and the split counters
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -1189,8 +1191,9 @@ cudaError_t launch_wide_kernel(const WideParams &p, dim3 grid, cudaStream_t s) {
   cudaError_t e = cudaFuncSetAttribute(wide_kernel<NCH>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  wide_kernel<NCH><<<grid, WideRoles<NCH>::kThreads, smem, s>>>(p);
-  return cudaGetLastError();
+  void *args[] = {const_cast<WideParams *>(&p)};
+  return launch_overlapped(reinterpret_cast<const void *>(&wide_kernel<NCH>), grid,
+                           dim3(WideRoles<NCH>::kThreads), args, smem, s);
 }
 
 int64_t round256(int64_t b) { return (b + 255) / 256 * 256; }

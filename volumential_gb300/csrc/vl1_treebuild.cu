@@ -137,10 +137,55 @@ __global__ void tb_ancestor_keys_kernel(int dim, int n, const uint8_t *levels,
   }
 }
 
-__global__ void tb_key_starts_kernel(int n, const uint8_t *levels, int64_t *counts) {
+// the key count of every leaf (its level + 1), and the largest level into
+// *max_level (kNoLevel when a leaf's coordinates do not fit its level)
+constexpr int kNoLevel = 1 << 20;
+__global__ void tb_key_starts_kernel(int dim, int n, const uint8_t *levels,
+                                     const int32_t *coords, int64_t *count, int32_t *max_level) {
+  int top = 0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    counts[i] = levels[i] + 1;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int lev = levels[i];
+    count[i] = lev + 1;
+    bool ok = lev <= 30;
+    for (int a = 0; a < dim; ++a) {
+      const long long c = coords[i * dim + a];
+      ok = ok && c >= 0 && c < (1ll << lev);
+    }
+    top = max(top, ok ? lev : kNoLevel);
+  }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top > 0) atomicMax(max_level, top);
+}
+
+// out[0]: the number of boxes; out[1 + l]: the first box of level l, for l up
+// to kLevelStarts - 1; out[1 + kLevelStarts]: the last box's level
+constexpr int kLevelStarts = 33;
+__global__ void tb_level_starts_kernel(int dim, const long long *keys, const int32_t *n_boxes,
+                                       int32_t *out) {
+  const int l = threadIdx.x, n = *n_boxes;
+  if (l == 0) {
+    out[0] = n;
+    int lev = 0;
+    while (lev < kLevelStarts - 2 && level_offset(dim, lev + 1) <= keys[n - 1]) ++lev;
+    out[1 + kLevelStarts] = lev;
+  }
+  if (l >= kLevelStarts) return;
+  // (levels whose offset is beyond 63 bits lie beyond every key)
+  int lo = 0, hi = n;
+  if (dim * l > 62) {
+    lo = n;
+  } else {
+    const long long first = level_offset(dim, l);
+    while (lo < hi) {
+      const int mid = lo + (hi - lo) / 2;
+      if (keys[mid] < first)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+  }
+  out[1 + l] = lo;
 }
 
 struct BoxOut {
@@ -381,19 +426,29 @@ extern "C" int32_t vl1_tree_build_begin(int32_t dim, int32_t q, int32_t n_leaves
   int32_t *n_unique = nullptr;
   if ((st = tb_alloc(b, &kcount, 8 * (size_t)n_leaves))) return fail(st);
   if ((st = tb_alloc(b, &kstart, 8 * ((size_t)n_leaves + 1)))) return fail(st);
-  tb_key_starts_kernel<<<tb_grid(n_leaves), kTB, 0, s>>>(n_leaves, leaf_levels, kcount);
+  int32_t *info = nullptr;   // [0]: largest level; then tb_level_starts_kernel's output
+  if ((st = tb_alloc(b, &info, 4 * (3 + kLevelStarts)))) return fail(st);
+  cudaMemsetAsync(info, 0, 4, s);
+  tb_key_starts_kernel<<<tb_grid(n_leaves), kTB, 0, s>>>(dim, n_leaves, leaf_levels, leaf_coords,
+                                                        kcount, info);
   size_t scan_bytes = 0;
   cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, kcount, kstart, n_leaves, s);
   void *scan_tmp = nullptr;
   if ((st = tb_alloc(b, &scan_tmp, scan_bytes))) return fail(st);
   cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, kcount, kstart, n_leaves, s);
   int64_t last[2] = {0, 0};
+  int32_t top = 0;
   if ((e = cudaMemcpyAsync(&last[0], kstart + n_leaves - 1, 8, cudaMemcpyDeviceToHost, s)) !=
           cudaSuccess ||
       (e = cudaMemcpyAsync(&last[1], kcount + n_leaves - 1, 8, cudaMemcpyDeviceToHost, s)) !=
           cudaSuccess ||
+      (e = cudaMemcpyAsync(&top, info, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
     return fail(cuda_fail(e, "tree build: key count"));
+  // the keys' bits: below the offset of the level after the last
+  int key_bits = 64;
+  if (dim * (top + 1) <= 60)
+    for (key_bits = 1; (1ll << key_bits) < level_offset(dim, top + 1);) ++key_bits;
   const int64_t n_keys = last[0] + last[1];
   if ((st = tb_alloc(b, &all, 8 * (size_t)n_keys))) return fail(st);
   if ((st = tb_alloc(b, &sorted, 8 * (size_t)n_keys))) return fail(st);
@@ -401,31 +456,26 @@ extern "C" int32_t vl1_tree_build_begin(int32_t dim, int32_t q, int32_t n_leaves
   tb_ancestor_keys_kernel<<<tb_grid(n_leaves), kTB, 0, s>>>(dim, n_leaves, leaf_levels,
                                                            leaf_coords, kstart, all);
   size_t sort_bytes = 0, uniq_bytes = 0;
-  cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, all, sorted, (int)n_keys, 0, 64, s);
+  cub::DeviceRadixSort::SortKeys(nullptr, sort_bytes, all, sorted, (int)n_keys, 0, key_bits, s);
   cub::DeviceSelect::Unique(nullptr, uniq_bytes, sorted, all, n_unique, (int)n_keys, s);
   void *tmp = nullptr;
   if ((st = tb_alloc(b, &tmp, std::max(sort_bytes, uniq_bytes)))) return fail(st);
-  cub::DeviceRadixSort::SortKeys(tmp, sort_bytes, all, sorted, (int)n_keys, 0, 64, s);
+  cub::DeviceRadixSort::SortKeys(tmp, sort_bytes, all, sorted, (int)n_keys, 0, key_bits, s);
   cub::DeviceSelect::Unique(tmp, uniq_bytes, sorted, all, n_unique, (int)n_keys, s);
-  int32_t nb = 0;
-  if ((e = cudaMemcpyAsync(&nb, n_unique, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-      (e = cudaStreamSynchronize(s)) != cudaSuccess)
-    return fail(cuda_fail(e, "tree build: box count"));
-  b->nboxes = nb;
-  b->box_keys = all;   // the first nb keys, sorted and distinct
-  // levels from the key ranges (level starts)
-  std::vector<long long> keys_host((size_t)nb);
-  if ((e = cudaMemcpyAsync(keys_host.data(), all, 8 * (size_t)nb, cudaMemcpyDeviceToHost, s)) !=
+  // the number of boxes and the levels' first ones, in one read-back
+  tb_level_starts_kernel<<<1, 64, 0, s>>>(dim, all, n_unique, info + 1);
+  int32_t host[2 + kLevelStarts];
+  if ((e = cudaGetLastError()) != cudaSuccess ||
+      (e = cudaMemcpyAsync(host, info + 1, sizeof(host), cudaMemcpyDeviceToHost, s)) !=
           cudaSuccess ||
       (e = cudaStreamSynchronize(s)) != cudaSuccess)
-    return fail(cuda_fail(e, "tree build: box keys"));
-  int lev = 0;
-  while (level_offset(dim, lev + 1) <= keys_host[nb - 1]) ++lev;
+    return fail(cuda_fail(e, "tree build: box count"));
+  const int32_t nb = host[0];
+  b->nboxes = nb;
+  b->box_keys = all;   // the first nb keys, sorted and distinct
+  const int lev = host[1 + kLevelStarts];
   b->max_level = lev;
-  b->level_start.assign(lev + 2, 0);
-  for (int l = 0; l <= lev + 1; ++l)
-    b->level_start[l] = (int32_t)(std::lower_bound(keys_host.begin(), keys_host.end(),
-                                                   level_offset(dim, l)) - keys_host.begin());
+  b->level_start.assign(host + 1, host + 1 + lev + 2);
   // leaf hash (leaf keys)
   const uint64_t cap = hash_capacity(n_leaves);
   long long *hk = nullptr;

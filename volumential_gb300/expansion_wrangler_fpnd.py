@@ -667,7 +667,7 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
     def _device_local_ids(self, payload):
         """``_compute_box_local_ids`` for an evaluation: on the device when the
         particle order is the user's (the ids are then i mod q^d: computed
-        there, and kept per (count, q^d))."""
+        there, and kept per (count, q^d, device))."""
         import torch
 
         nq = int(payload["table_data_shapes"]["n_q_points"])
@@ -675,13 +675,14 @@ class FPNDExpansionWrangler(ExpansionWranglerInterface):
         if (not _identity_order(self.tree) or not torch.cuda.is_available()
                 or torch.cuda.is_current_stream_capturing()):
             return _compute_box_local_ids(self.tree, nq)
-        ids = self._local_ids.get((n, nq))
+        key = (n, nq, torch.cuda.current_device())
+        ids = self._local_ids.get(key)
         if ids is None:
             ids = torch.arange(n, dtype=torch.int32, device="cuda").remainder_(nq)
             torch.cuda.current_stream().synchronize()   # read on any stream
             if len(self._local_ids) >= 4:
                 self._local_ids.clear()
-            self._local_ids[n, nq] = ids
+            self._local_ids[key] = ids
         return ids
 
     def _near_field_kwargs(self, payload, target_boxes, starts, lists, mode_coefs, local=None):

@@ -21,12 +21,15 @@ __all__ = ["Plan", "plan_cache_get", "tree_view_from_arrays", "as_device_tensor"
 
 PLAN_CACHE_MAX = 16
 #: modelled time of the per-box FP64 kernel from which the tensor-core path is
-#: taken, and from which a tree's schedule is built on its first evaluation
-#: (``Plan._fp64_schedule``): at 60 us both take the same time (2D, q = 4,
-#: level 6: 75 and 57 us; 3D, q = 3, level 3: 49 and 51 us; 2D, level 5: 21
-#: and 53 us), at 1.5 ms the schedule costs what it saves at once (3D, q = 4,
-#: level 4: 875 us against 700 + 75 us)
+#: taken, with up to 32 tiles and per tile beyond, and from which a tree's
+#: schedule is built on its first evaluation (``Plan._fp64_schedule``).  Per-box
+#: and tensor-core times on both sides of the line: 2D, q = 5, level 6 (32
+#: tiles) 91 and 57 us; q = 4 61 and 56; q = 3 45 and 56; 3D, q = 3, level 3 45
+#: and 63; 2D, q = 3, level 7 (128 tiles) 146 and 90; q = 2 96 and 90, with
+#: complex densities (256 tiles) 127 and 174.  At 1.5 ms the schedule costs what
+#: it saves at once (3D, q = 4, level 4: 875 us against 700 + 75 us)
 FP64_TILE_US = 60.0
+FP64_TILE_STEP_US = 0.31
 FP64_BUILD_US = 1500.0
 _cache: "collections.OrderedDict" = collections.OrderedDict()
 _cache_lock = threading.Lock()
@@ -272,6 +275,7 @@ class Plan:
         d.table_starting_level = int(table_starting_level)
         self.desc = d
         self.dim, self.quad_order, self.nq = int(dim), int(quad_order), nq
+        self.displaced = int(displacement_kind) != 0   # a 2D log displacement
         self.n_tables = int(n_tables)
         self.n_cases = d.n_cases
         handle = C.c_void_p()
@@ -355,8 +359,9 @@ class Plan:
         hit = known.get(rows)
         if hit is not None and hit[0] is self:
             return hit[1]
-        us = self._per_box_us(view, keep, rows)
-        if us < FP64_TILE_US or self.nq > 256:
+        us = self._per_box_us(view, keep, rows, nrhs)
+        tiles = int(view.n_target_boxes) * rows / 128.0
+        if us < FP64_TILE_US + FP64_TILE_STEP_US * max(tiles - 32.0, 0.0) or self.nq > 256:
             known[rows] = (self, None)
             return None
         if us < FP64_BUILD_US and hit != (self.handle.value, None):
@@ -377,17 +382,19 @@ class Plan:
         known[rows] = (self, sched)
         return sched
 
-    def _per_box_us(self, view, keep, rows):
+    def _per_box_us(self, view, keep, rows, nrhs):
         """Modelled time of the per-box FP64 kernel: its products at the
-        0.95 TFLOP/s that the FP64 pipe gives it, or, with few boxes, one
-        box's chain of sources (0.38 us each, split over up to 128 / q^d
-        threads per target point); within 20 % of the measured times from
-        60 us to 7 ms."""
+        0.95 TFLOP/s that the FP64 pipe gives it plus the pairs' case ids and
+        displacement logarithms (0.6 ns a pair in 2D with a displacement, 0.18
+        without), or, with few boxes, one box's chain of sources (0.38 us each,
+        split over up to 128 / q^d threads per target point); within 30 % of
+        the measured times from 60 us to 7 ms."""
         pairs = keep["lists"].numel()
         flops = 2.0 * pairs * self.nq * self.nq * rows * (2.0 if self.complex_table else 1.0)
         split = min(max(round(128.0 / self.nq), 1), 8)
         chain = pairs / max(int(view.n_target_boxes), 1) * self.nq / split
-        return max(flops / 0.95e6, 0.38 * chain)
+        pair_us = (6e-4 if self.displaced else 1.8e-4) * pairs * nrhs
+        return max(flops / 0.95e6 + pair_us, 0.38 * chain)
 
     def mixed_geometry(self):
         out = (C.c_int32 * 5)()

@@ -84,10 +84,19 @@ __global__ void index_map_kernel(DevDesc d, int32_t *rows, int8_t *signs) {
   }
 }
 
+// 2D displacement factor of a source box of level l: coefficient * scaling *
+// log(extent / table extent), computed once per call on the host (a
+// logarithm and a division per pair were most of the kernel's FP64 work on
+// trees of many small boxes: 2D level 7, q = 2 94 us, 56 with the table)
+struct LevelDisp {
+  double f[kScaleLevels];
+};
+
 template <bool TC, bool CC>
 __global__ void __launch_bounds__(256)
 plain_kernel(DevDesc d, TreeDev tr, const double *__restrict__ coefs,
-             double *__restrict__ result, int split, int pch, vl1_status *st) {
+             double *__restrict__ result, int split, int pch,
+             const __grid_constant__ LevelDisp level_disp, vl1_status *st) {
   constexpr bool OC = TC || CC;
   constexpr int CV = CC ? 2 : 1;  // doubles per coefficient
   constexpr int OV = OC ? 2 : 1;  // doubles per output
@@ -139,15 +148,17 @@ plain_kernel(DevDesc d, TreeDev tr, const double *__restrict__ coefs,
       const int c = pair_case_id(d, tr, tbox_id, sbox, ext);
       PairInfo pi;
       pi.lev = pair_table_level(d, lvl);
-      // (per level, from the call's table: the division chain of pair_scaling
-      // is on a small launch's critical path; with the reciprocal in
-      // pair_case_id a 2D level-5 tree, q = 4, takes 15.6 instead of 18.7 us,
-      // level 7, q = 2, 94 instead of 144)
+      // (per level, from the call's tables: the divisions and the logarithm
+      // are on a small launch's critical path; with the reciprocal in
+      // pair_case_id a 2D level-5 tree, q = 4, takes 13.8 instead of 18.7 us,
+      // level 7, q = 2, 56 instead of 144)
       pi.scaling = box_scaling(d, tr, lvl);
       pi.dispfac = 0.0;
       if (d.disp_kind == VL1_DISP_LOG2D)
-        pi.dispfac = __dmul_rn(__dmul_rn(d.disp_coef, pi.scaling),
-                               log(__ddiv_rn(ext, d.table_root_extent)));
+        pi.dispfac = lvl < kScaleLevels
+                         ? level_disp.f[lvl]
+                         : __dmul_rn(__dmul_rn(d.disp_coef, pi.scaling),
+                                     log(__ddiv_rn(ext, d.table_root_extent)));
       pi.src_beg = tr.src_starts[sbox];
       pi.nsrc = tr.src_counts[sbox];
       if (pi.nsrc > nq) {
@@ -340,19 +351,26 @@ int32_t launch_plain(vl1_plan *plan, const TreeDev &tree, const double *coefs,
     set_error("plain kernel shared memory %zu exceeds 48 KiB", smem);
     return VL1_E_UNSUPPORTED;
   }
+  LevelDisp level_disp{};
+  if (d.disp_kind == VL1_DISP_LOG2D)
+    for (int l = 0; l < kScaleLevels; ++l) {
+      const double ext = tree.root_extent * (1.0 / (double)(1LL << l));
+      level_disp.f[l] =
+          (d.disp_coef * tree.level_scale[l]) * std::log(ext / d.table_root_extent);
+    }
   dim3 grid(tree.n_tgt_boxes, nrhs);
   if (nrhs > 65535) {
     set_error("nrhs %d exceeds 65535", nrhs);
     return VL1_E_ARG;
   }
   if (tc && cc)
-    plain_kernel<true, true><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, plan->status);
+    plain_kernel<true, true><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, level_disp, plan->status);
   else if (tc)
-    plain_kernel<true, false><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, plan->status);
+    plain_kernel<true, false><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, level_disp, plan->status);
   else if (cc)
-    plain_kernel<false, true><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, plan->status);
+    plain_kernel<false, true><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, level_disp, plan->status);
   else
-    plain_kernel<false, false><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, plan->status);
+    plain_kernel<false, false><<<grid, threads, smem, s>>>(d, tree, coefs, result, split, pch, level_disp, plan->status);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? VL1_OK : cuda_fail(e, "plain_kernel launch");
 }

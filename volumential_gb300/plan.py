@@ -24,9 +24,9 @@ PLAN_CACHE_MAX = 16
 #: taken, with up to 32 tiles and per tile beyond, and from which a tree's
 #: schedule is built on its first evaluation (``Plan._fp64_schedule``).  Per-box
 #: and tensor-core times on both sides of the line: 2D, q = 5, level 6 (32
-#: tiles) 91 and 57 us; q = 4 61 and 56; q = 3 45 and 56; 3D, q = 3, level 3 45
-#: and 63; 2D, q = 3, level 7 (128 tiles) 146 and 90; q = 2 96 and 90, with
-#: complex densities (256 tiles) 127 and 174.  At 1.5 ms the schedule costs what
+#: tiles) 82 and 57 us; q = 4 51 and 57; q = 3 35 and 56; 3D, q = 3, level 3 45
+#: and 63; 2D, q = 3, level 7 (128 tiles) 115 and 90; q = 2 58 and 90, with
+#: complex densities (256 tiles) 89 and 174.  At 1.5 ms the schedule costs what
 #: it saves at once (3D, q = 4, level 4: 875 us against 700 + 75 us)
 FP64_TILE_US = 60.0
 FP64_TILE_STEP_US = 0.31
@@ -384,16 +384,16 @@ class Plan:
 
     def _per_box_us(self, view, keep, rows, nrhs):
         """Modelled time of the per-box FP64 kernel: its products at the
-        0.95 TFLOP/s that the FP64 pipe gives it plus the pairs' case ids and
-        displacement logarithms (0.6 ns a pair in 2D with a displacement, 0.18
-        without), or, with few boxes, one box's chain of sources (0.38 us each,
-        split over up to 128 / q^d threads per target point); within 30 % of
-        the measured times from 60 us to 7 ms."""
+        0.95 TFLOP/s that the FP64 pipe gives it plus the pairs' case ids
+        (0.18 ns each; with a 2D displacement 0.33 ns and 0.03 ns a source),
+        or, with few boxes, one box's chain of sources (0.38 us each, split
+        over up to 128 / q^d threads per target point); within 25 % of the
+        measured times from 50 us to 7 ms."""
         pairs = keep["lists"].numel()
         flops = 2.0 * pairs * self.nq * self.nq * rows * (2.0 if self.complex_table else 1.0)
         split = min(max(round(128.0 / self.nq), 1), 8)
         chain = pairs / max(int(view.n_target_boxes), 1) * self.nq / split
-        pair_us = (6e-4 if self.displaced else 1.8e-4) * pairs * nrhs
+        pair_us = (3.3e-4 + 3e-5 * self.nq if self.displaced else 1.8e-4) * pairs * nrhs
         return max(flops / 0.95e6 + pair_us, 0.38 * chain)
 
     def mixed_geometry(self):

@@ -687,16 +687,17 @@ __device__ __forceinline__ void disp_box_row(const DevDesc &d, const TreeDev &tr
                                              const double *coefs, int nrhs, double *w,
                                              int64_t idx) {
   const int cv = d.table_cplx ? 2 : 1;
-  const int b = (int)(idx / nrhs), r = (int)(idx % nrhs);
+  const int b = (int)((unsigned)idx / (unsigned)nrhs), r = (int)((unsigned)idx % (unsigned)nrhs);
   double re = 0.0, im = 0.0;
   int cnt = min(tr.src_counts[b], d.nq);
   if (cnt > 0) {
     const int lvl = tr.levels[b];
     const double ext = level_extent(tr.root_extent, lvl);
-    const double f = __dmul_rn(__dmul_rn(d.disp_coef, pair_scaling(d, ext)),
+    const double f = __dmul_rn(__dmul_rn(d.disp_coef, box_scaling(d, tr, lvl)),
                                log(__ddiv_rn(ext, d.table_root_extent)));
     const int lev = pair_table_level(d, lvl);
     const double *c = coefs + (int64_t)r * tr.n_particles + tr.src_starts[b];
+#pragma unroll 4
     for (int s = 0; s < cnt; ++s) {
       const int64_t ni = (int64_t)lev * d.nq + s;
       re += c[s] * (f * (d.table_cplx ? d.nmlz[2 * ni] : d.nmlz[ni]));
@@ -710,8 +711,9 @@ __device__ __forceinline__ void disp_box_row(const DevDesc &d, const TreeDev &tr
 __device__ __forceinline__ void disp_target_row(const DevDesc &d, const TreeDev &tr, int nrhs,
                                                 const double *w, double *disp, int64_t idx) {
   const int cv = d.table_cplx ? 2 : 1;
-  const int tb = (int)(idx / nrhs), r = (int)(idx % nrhs);
+  const int tb = (int)((unsigned)idx / (unsigned)nrhs), r = (int)((unsigned)idx % (unsigned)nrhs);
   double re = 0.0, im = 0.0;
+#pragma unroll 4
   for (int p = tr.starts[tb]; p < tr.starts[tb + 1]; ++p) {
     const int64_t wi = ((int64_t)tr.lists[p] * nrhs + r) * cv;
     re += w[wi];
@@ -723,6 +725,8 @@ __device__ __forceinline__ void disp_target_row(const DevDesc &d, const TreeDev 
 
 __global__ void disp_box_kernel(DevDesc d, TreeDev tr, int nboxes, const double *coefs,
                                 int nrhs, double *w) {
+  grid_dep_launch();
+  grid_dep_wait();
   const int64_t n = (int64_t)nboxes * nrhs;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n;
        idx += (int64_t)gridDim.x * blockDim.x)
@@ -731,6 +735,8 @@ __global__ void disp_box_kernel(DevDesc d, TreeDev tr, int nboxes, const double 
 
 __global__ void disp_target_kernel(DevDesc d, TreeDev tr, int nrhs, const double *w,
                                    double *disp) {
+  grid_dep_launch();
+  grid_dep_wait();   // the boxes' sums
   const int64_t n = (int64_t)tr.n_tgt_boxes * nrhs;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < n;
        idx += (int64_t)gridDim.x * blockDim.x)
@@ -1912,10 +1918,21 @@ int32_t launch_mixed(vl1_plan *plan, const TreeDev &tree, int64_t nboxes,
     if (e != cudaSuccess) return cuda_fail(e, "x_planes_kernel launch");
   }
   if (disp) {
-    disp_box_kernel<<<grid_for(nbr, 256), 256, 0, s>>>(d, tree, (int)nboxes, coefs, nrhs,
-                                                      wbox);
-    disp_target_kernel<<<grid_for((int64_t)tree.n_tgt_boxes * nrhs, 256), 256, 0, s>>>(
-        d, tree, nrhs, wbox, disp);
+    // (blocks of 64 rows: a thread's chain of loads bounds small trees, so the
+    // rows spread over the SMs)
+    int nb = (int)nboxes;
+    DevDesc dd = d;
+    TreeDev tr = tree;
+    const double *w_in = wbox;
+    void *box_args[] = {&dd, &tr, &nb, &coefs, &nrhs, &wbox};
+    void *target_args[] = {&dd, &tr, &nrhs, &w_in, &disp};
+    e = launch_overlapped(reinterpret_cast<const void *>(&disp_box_kernel),
+                          dim3(grid_for(nbr, 64)), dim3(64), box_args, 0, s);
+    if (e == cudaSuccess)
+      e = launch_overlapped(reinterpret_cast<const void *>(&disp_target_kernel),
+                            dim3(grid_for((int64_t)tree.n_tgt_boxes * nrhs, 64)), dim3(64),
+                            target_args, 0, s);
+    if (e != cudaSuccess) return cuda_fail(e, "displacement launch");
   }
   e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "mixed preparation launch");

@@ -211,13 +211,14 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree,
  * its work items at most vl1_eval_fp64_item_keys keys long.  The first call
  * with a plan builds its table digits and synchronises the stream; scratch
  * is allocated and freed in stream order.  Evaluates as vl1_eval_fp64 while
- * the stream is being captured, where the scratch cannot be had, or where a
- * box has more than 256 points. */
+ * the stream is being captured, where the scratch cannot be had, where a
+ * box has more than 256 points, or where the plan's table holds a NaN. */
 int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
                             const vl1_mixed_schedule *schedule, const void *coefs,
                             int32_t coef_type, int32_t nrhs, void *result, void *stream);
 
-/* The most keys a work item may have in vl1_eval_fp64_tiles. */
+/* The most keys a work item may have in vl1_eval_fp64_tiles; 0 for a plan that
+ * vl1_eval_fp64_tiles evaluates as vl1_eval_fp64 (a NaN in its table). */
 int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan);
 
 /* Table key (table_level * n_cases + case) of every list-1 pair, computed with

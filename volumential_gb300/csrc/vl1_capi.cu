@@ -279,7 +279,10 @@ int32_t vl1_plan_create(const vl1_plan_desc *desc, vl1_plan **plan_out) {
       double amax = 0.0;
       const double *tv = static_cast<const double *>(desc->table_data);
       const int64_t ntv = (int64_t)d.n_tables * d.n_entries * (d.table_cplx ? 2 : 1);
-      for (int64_t i = 0; i < ntv; ++i) amax = fmax(amax, fabs(tv[i]));
+      for (int64_t i = 0; i < ntv; ++i) {
+        amax = fmax(amax, fabs(tv[i]));   // (passes over NaN)
+        if (tv[i] != tv[i]) p->table_nan = 1;
+      }
       if (!(amax < 1e300)) {
         set_error("table data contains non-finite values");
         st = VL1_E_NONFINITE;
@@ -419,7 +422,7 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree, const void *coe
 // a work item's digit sums of weights 2^-56 .. 2^-72 must fit an int32:
 // (2^16 + 7 * 2^14) K < 2^31
 int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan) {
-  if (!plan) return 0;
+  if (!plan || plan->table_nan) return 0;
   const int kp = vl1::wide_geometry(plan->d.nq, plan->d.table_cplx).kp;
   return kp >= 8192 ? 1 : 8192 / kp;
 }
@@ -435,8 +438,9 @@ int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   cudaError_t e = cudaStreamIsCapturing(s, &cap);
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
-  // beyond vl1_eval_fp64's own limits its error is reported
-  if (cap != cudaStreamCaptureStatusNone || plan->d.nq > 256 || nrhs < 1 || nrhs > 65535 ||
+  // beyond vl1_eval_fp64's own limits its error is reported; a NaN in the
+  // table has no digits (its block would take the scale of its whole level)
+  if (cap != cudaStreamCaptureStatusNone || plan->table_nan || plan->d.nq > 256 || nrhs < 1 || nrhs > 65535 ||
       !coefs || !result || (coef_type != VL1_REAL64 && coef_type != VL1_COMPLEX128))
     return vl1_eval_fp64(plan, tree, coefs, coef_type, nrhs, result, stream);
   TreeDev tr;

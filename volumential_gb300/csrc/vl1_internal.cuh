@@ -67,6 +67,7 @@ struct vl1_plan {
   vl1_status *status;   // device
   vl1::MixedPlan mixed;
   vl1::WidePlan wide;
+  int table_nan;        // nonzero: a table value is NaN (no fixed-point digits)
 };
 
 namespace vl1 {

@@ -282,6 +282,8 @@ class Plan:
         _lib.check(lib.vl1_plan_create(C.byref(d), C.byref(handle)), "vl1_plan_create")
         self._handle = handle
         self._lib = lib
+        # keys per work item of the FP64 tensor-core path; 0: per-box kernel only
+        self._tile_keys = int(lib.vl1_eval_fp64_item_keys(handle))
 
     @property
     def handle(self):
@@ -361,7 +363,8 @@ class Plan:
             return hit[1]
         us = self._per_box_us(view, keep, rows, nrhs)
         tiles = int(view.n_target_boxes) * rows / 128.0
-        if us < FP64_TILE_US + FP64_TILE_STEP_US * max(tiles - 32.0, 0.0) or self.nq > 256:
+        if (us < FP64_TILE_US + FP64_TILE_STEP_US * max(tiles - 32.0, 0.0) or self.nq > 256
+                or not self._tile_keys):
             known[rows] = (self, None)
             return None
         if us < FP64_BUILD_US and hit != (self.handle.value, None):
@@ -373,7 +376,7 @@ class Plan:
         if torch.cuda.is_current_stream_capturing():
             return None
         try:
-            cap = int(self._lib.vl1_eval_fp64_item_keys(self.handle))
+            cap = self._tile_keys
             sched = get_schedule(self, view, keep, rows, stream)
             if sched.max_keys_per_item > cap:
                 sched = get_schedule(self, view, keep, rows, stream, max_keys_per_item=cap)

@@ -17,9 +17,9 @@
 // of many boxes R is evaluated once per (source level, relative position) and
 // point pair, and the sums read it from there (split_sum_kernel: two FMAs and
 // 16 bytes from the L2 per pair).  split_mark_kernel checks on the device that
-// every box's points are its level's template (to a few ulps of the
-// coordinates, the rounding of the points themselves) and its source and
-// target points the same; otherwise, and for small trees, the per-pair kernel
+// every box's points are its level's template and every centre lies on the
+// lattice (to a few ulps of the coordinates, the rounding of the points
+// themselves) and its source and target points the same; otherwise, and for small trees, the per-pair kernel
 // runs: one CTA per target box, one thread per target point, the points and
 // strengths of each list-1 source box staged in shared memory.
 //
@@ -141,11 +141,15 @@ __device__ __forceinline__ int split_key(const SplitTables &T, int tb, int sb) {
   int code = 0;
 #pragma unroll
   for (int a = 0; a < DIM; ++a) {
-    const double d =
-        (T.centers[a * T.aligned_nboxes + tb] - T.centers[a * T.aligned_nboxes + sb]) / quarter;
-    const double r = rint(d);
+    const double ct = T.centers[a * T.aligned_nboxes + tb];
+    const double cs = T.centers[a * T.aligned_nboxes + sb];
+    const double r = rint((ct - cs) / quarter);
     // the boxes of one tree lie on its lattice, up to the centres' rounding
-    if (!(fabs(d - r) <= 1e-3) || fabs(r) > 6.0) return -1;
+    // (a centre is the root vertex plus a part of the root extent): the same
+    // few ulps that the points are held to, since the tables take the lattice
+    // position for the distance
+    const double ulp = 2.220446049250313e-16 * (fabs(ct) + fabs(cs) + T.root_extent);
+    if (!(fabs((ct - cs) - r * quarter) <= 2.0 * ulp) || fabs(r) > 6.0) return -1;
     code = code * kSplitBase + (int)r + 6;
   }
   return (ls * 3 + step + 1) * T.n_codes + code;

@@ -132,11 +132,12 @@ struct SplitTables {
 };
 
 // the key of a pair of boxes, or -1: source level, target level - source level
-// (-1, 0, 1) and centre offset in quarters of the source box
-template <int DIM>
+// (-1, 0, 1) and centre offset in quarters of the source box.  CHECK false: a
+// pair that split_mark_kernel has accepted.
+template <int DIM, bool CHECK>
 __device__ __forceinline__ int split_key(const SplitTables &T, int tb, int sb) {
   const int ls = T.levels[sb], step = (int)T.levels[tb] - ls;
-  if (ls >= kSplitLevels || step < -1 || step > 1) return -1;
+  if (CHECK && (ls >= kSplitLevels || step < -1 || step > 1)) return -1;
   const double quarter = 0.25 * T.root_extent / (double)(1ll << ls);
   int code = 0;
 #pragma unroll
@@ -144,13 +145,14 @@ __device__ __forceinline__ int split_key(const SplitTables &T, int tb, int sb) {
     const double ct = T.centers[a * T.aligned_nboxes + tb];
     const double cs = T.centers[a * T.aligned_nboxes + sb];
     const double r = rint((ct - cs) / quarter);
+    code = code * kSplitBase + (int)r + 6;
+    if (!CHECK) continue;
     // the boxes of one tree lie on its lattice, up to the centres' rounding
     // (a centre is the root vertex plus a part of the root extent): the same
     // few ulps that the points are held to, since the tables take the lattice
     // position for the distance
     const double ulp = 2.220446049250313e-16 * (fabs(ct) + fabs(cs) + T.root_extent);
     if (!(fabs((ct - cs) - r * quarter) <= 2.0 * ulp) || fabs(r) > 6.0) return -1;
-    code = code * kSplitBase + (int)r + 6;
   }
   return (ls * 3 + step + 1) * T.n_codes + code;
 }
@@ -197,8 +199,12 @@ __global__ void split_mark_kernel(const SplitArgs A, const SplitTables T) {
     for (int q = A.starts[i] + lane; q < A.starts[i + 1]; q += 32) {
       // (boxes without points need no table, and their levels may have none)
       if (A.tgt_counts[A.target_boxes[i]] <= 0 || A.src_counts[A.lists[q]] <= 0) continue;
-      const int key = split_key<DIM>(T, A.target_boxes[i], A.lists[q]);
-      if (key < 0) {
+      const int key = split_key<DIM, true>(T, A.target_boxes[i], A.lists[q]);
+      // (two boxes in one place: the table of the position has no self pairs)
+      constexpr int kHere = DIM == 2 ? 6 * kSplitBase + 6 : (6 * kSplitBase + 6) * kSplitBase + 6;
+      const bool twin = key >= 0 && A.lists[q] != A.target_boxes[i] &&
+                        (key / T.n_codes) % 3 == 1 && key % T.n_codes == kHere;
+      if (key < 0 || twin) {
         *T.bad = 1;
       } else if (T.slot_of[key] < 0 && atomicCAS(T.slot_of + key, -1, -2) == -1) {
         const int slot = atomicAdd(T.n_slots, 1);
@@ -263,6 +269,7 @@ __global__ void __launch_bounds__(256)
   if (A.tgt_counts[tb] <= 0) return;
   const int t = threadIdx.x % nq, sg = threadIdx.x / nq;
   __shared__ int s_slot[kSplitChunk], s_src[kSplitChunk];
+  __shared__ bool s_self[kSplitChunk];
   double re = 0.0, im = 0.0;
   const int q_end = A.starts[blockIdx.x + 1];
   for (int q0 = A.starts[blockIdx.x]; q0 < q_end; q0 += kSplitChunk) {
@@ -271,8 +278,9 @@ __global__ void __launch_bounds__(256)
     if (threadIdx.x < m) {   // one thread per source box: its table and points
       const int sb = A.lists[q0 + threadIdx.x];
       const bool have = A.src_counts[sb] > 0;
-      s_slot[threadIdx.x] = have ? T.slot_of[split_key<DIM>(T, tb, sb)] : -1;
+      s_slot[threadIdx.x] = have ? T.slot_of[split_key<DIM, false>(T, tb, sb)] : -1;
       s_src[threadIdx.x] = A.src_starts[sb];
+      s_self[threadIdx.x] = A.exclude_self && sb == tb;
     }
     __syncthreads();
     // strengths of the chunk's sources
@@ -289,10 +297,14 @@ __global__ void __launch_bounds__(256)
       if (s_slot[p] < 0) continue;
       const double2 *R = T.table + (int64_t)s_slot[p] * nq * nq + t;
       const double2 *w = s_w + p * nq;
+      // an excluded self pair adds nothing, whatever its weight (the table's
+      // zero times an infinite or NaN weight would be NaN)
+      const int skip = s_self[p] ? t : -1;
       if (A.wcplx) {
 #pragma unroll 4
         for (int s = sg; s < nq; s += split) {
-          const double2 r = __ldg(R + (int64_t)s * nq), v = w[s];
+          const double2 r = __ldg(R + (int64_t)s * nq);
+          const double2 v = s == skip ? make_double2(0.0, 0.0) : w[s];
           re = fma(v.x, r.x, fma(-v.y, r.y, re));
           im = fma(v.x, r.y, fma(v.y, r.x, im));
         }
@@ -300,7 +312,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 8
         for (int s = sg; s < nq; s += split) {
           const double2 r = __ldg(R + (int64_t)s * nq);
-          const double v = w[s].x;
+          const double v = s == skip ? 0.0 : w[s].x;
           re = fma(v, r.x, re);
           im = fma(v, r.y, im);
         }

@@ -10,7 +10,9 @@ from __future__ import annotations
 
 import collections
 import ctypes as C
+import itertools
 import threading
+import weakref
 
 import numpy as np
 
@@ -31,8 +33,11 @@ PLAN_CACHE_MAX = 16
 FP64_TILE_US = 60.0
 FP64_TILE_STEP_US = 0.31
 FP64_BUILD_US = 1500.0
+#: FP64 schedules that a tree view keeps (plans and row counts)
+FP64_SCHEDULES_PER_VIEW = 16
 _cache: "collections.OrderedDict" = collections.OrderedDict()
 _cache_lock = threading.Lock()
+_serial = itertools.count()
 
 
 _cuda_ok = False
@@ -282,6 +287,8 @@ class Plan:
         _lib.check(lib.vl1_plan_create(C.byref(d), C.byref(handle)), "vl1_plan_create")
         self._handle = handle
         self._lib = lib
+        self._serial = next(_serial)          # never used again, unlike id() or the handle
+        self._proxy = weakref.proxy(self)
         # keys per work item of the FP64 tensor-core path; 0: per-box kernel only
         self._tile_keys = int(lib.vl1_eval_fp64_item_keys(handle))
 
@@ -350,31 +357,44 @@ class Plan:
         kernel ``_per_box_us``.  A tree seen for the first time has no
         schedule yet, and building one takes 0.4 ms (2D, a thousand boxes) to
         1.5 ms (3D, 23,000 boxes): below FP64_BUILD_US only a tree that comes
-        again (the same view object) gets one.  Trees that no schedule
+        again (the same view object, with the same plan and row count: each
+        pair has a schedule of its own) gets one.  Trees that no schedule
         describes (two sources of a box in one mode, two list-1 boxes of one
         case) stay with the per-box kernel, as do calls under graph capture
         that would have to build one."""
         rows = 2 * nrhs if complex_coefs else nrhs
-        known = view.__dict__.get("fp64_schedules")
+        known = view.__dict__.get("_fp64_known")
         if known is None:
-            known = view.fp64_schedules = {}
-        hit = known.get(rows)
-        if hit is not None and hit[0] is self:
-            return hit[1]
+            known = view._fp64_known = collections.OrderedDict()
+            view.fp64_schedules = {}
+        key = (self._serial, rows)
+        hit = known.get(key)       # None, or (seen before without a schedule, record)
+        if hit is None or hit[0]:
+            hit = self._fp64_decide(view, keep, rows, nrhs, stream, hit is not None)
+            known[key] = hit
+            while len(known) > FP64_SCHEDULES_PER_VIEW:
+                known.popitem(last=False)
+        # the decision of the last call, by row count: (plan, schedule or None)
+        if view.fp64_schedules.get(rows) is not hit[1]:
+            view.fp64_schedules[rows] = hit[1]
+        return hit[1][1]
+
+    def _fp64_decide(self, view, keep, rows, nrhs, stream, again):
+        """(to be asked again, (this plan, schedule or None)) for a view that
+        has no schedule of this plan yet; ``again``: seen before."""
+        none = (self._proxy, None)
         us = self._per_box_us(view, keep, rows, nrhs)
         tiles = int(view.n_target_boxes) * rows / 128.0
         if (us < FP64_TILE_US + FP64_TILE_STEP_US * max(tiles - 32.0, 0.0) or self.nq > 256
                 or not self._tile_keys):
-            known[rows] = (self, None)
-            return None
-        if us < FP64_BUILD_US and hit != (self.handle.value, None):
-            known[rows] = (self.handle.value, None)     # built when the tree comes again
-            return None
+            return False, none
+        if us < FP64_BUILD_US and not again:
+            return True, none          # built when the tree comes again
         import torch
 
         from .batched import get_schedule
         if torch.cuda.is_current_stream_capturing():
-            return None
+            return True, none
         try:
             cap = self._tile_keys
             sched = get_schedule(self, view, keep, rows, stream)
@@ -382,8 +402,7 @@ class Plan:
                 sched = get_schedule(self, view, keep, rows, stream, max_keys_per_item=cap)
         except (ValueError, RuntimeError):
             sched = None
-        known[rows] = (self, sched)
-        return sched
+        return False, (self._proxy, sched)
 
     def _per_box_us(self, view, keep, rows, nrhs):
         """Modelled time of the per-box FP64 kernel: its products at the

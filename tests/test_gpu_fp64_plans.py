@@ -7,6 +7,7 @@ they agree to 1e-13 relative l2."""
 import pytest
 
 from helpers import plan_and_view, rel_l2, wrangler_for
+from volumential_gb300 import batched
 from volumential_gb300 import workloads as W
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +42,47 @@ def test_two_plans_alternate_on_one_view(cuda):
             taken.append(view.fp64_schedules[1])
     assert all(t[1] is not None for t in taken)
     assert [t[0] == p for t, p in zip(taken, plans)] == [True, True]
+
+
+def test_a_failed_build_is_tried_again(cuda, monkeypatch):
+    """Out of memory while the schedule is built: this call goes per box, the
+    next one builds it."""
+    torch = cuda
+    w = W.uniform_workload("oom", 3, 3, 4, seed=62)
+    plan, view, keep = plan_and_view(w)
+    c = torch.from_numpy(w.coefs[0]).cuda()
+    out, ref = torch.empty_like(c), torch.empty_like(c)
+    plan.eval_fp64(view, c, ref, stream=0)
+    plan.eval_fp64(view, c, out, stream=0, keep=keep)    # seen once
+    calls = []
+    init = batched.MixedSchedule.__init__
+
+    def fails_once(self, *a, **k):
+        calls.append(1)
+        if len(calls) == 1:
+            raise torch.OutOfMemoryError("CUDA out of memory (planted)")
+        init(self, *a, **k)
+
+    monkeypatch.setattr(batched.MixedSchedule, "__init__", fails_once)
+    plan.eval_fp64(view, c, out, stream=0, keep=keep)
+    assert torch.equal(out, ref)
+    for _ in range(2):
+        plan.eval_fp64(view, c, out, stream=0, keep=keep)
+        assert rel_l2(out.cpu().numpy(), ref.cpu().numpy()) <= 1e-13
+    assert view.fp64_schedules[1][1] is not None and len(calls) == 2
+
+
+def test_other_errors_while_building_are_raised(cuda, monkeypatch):
+    torch = cuda
+    w = W.uniform_workload("err", 3, 3, 4, seed=63)
+    plan, view, keep = plan_and_view(w)
+    c = torch.from_numpy(w.coefs[0]).cuda()
+    out = torch.empty_like(c)
+    plan.eval_fp64(view, c, out, stream=0, keep=keep)
+
+    def fails(self, *a, **k):
+        raise RuntimeError("CUDA error: planted")
+
+    monkeypatch.setattr(batched.MixedSchedule, "__init__", fails)
+    with pytest.raises(RuntimeError, match="planted"):
+        plan.eval_fp64(view, c, out, stream=0, keep=keep)

@@ -27,7 +27,8 @@ import numpy as np
 
 from . import _lib
 
-__all__ = ["MixedSchedule", "get_schedule", "eval_mixed", "DIGITS", "ROWS_PER_TILE"]
+__all__ = ["MixedSchedule", "ScheduleError", "get_schedule", "eval_mixed", "DIGITS",
+           "ROWS_PER_TILE"]
 
 DIGITS = 5
 ROWS_PER_TILE = 128
@@ -35,6 +36,11 @@ ROWS_PER_TILE = 128
 _cache: "collections.OrderedDict" = collections.OrderedDict()
 _lock = threading.Lock()
 _CACHE_MAX = 256
+
+
+class ScheduleError(RuntimeError):
+    """No schedule describes the tree: a target box has two list-1 source
+    boxes of one case."""
 
 
 class MixedSchedule:
@@ -100,7 +106,7 @@ class MixedSchedule:
             raise ValueError("the mixed-precision path requires distinct source mode ids in "
                              f"[0, {plan.nq}) inside every box: {_lib.last_error()}")
         if st == _lib.VL1_E_ARG and "same case" in _lib.last_error():
-            raise RuntimeError(_lib.last_error())
+            raise ScheduleError(_lib.last_error())
         _lib.check(st, "vl1_schedule_build_begin")
         try:
             n_tiles, n_ent = int(sizes.n_tiles), int(sizes.n_entries)
@@ -246,7 +252,7 @@ class MixedSchedule:
         if len(comb) > 1:
             cs = np.sort(comb)
             if np.any(cs[1:] == cs[:-1]):
-                raise RuntimeError("a target box has two list-1 source boxes with the same case")
+                raise ScheduleError("a target box has two list-1 source boxes with the same case")
 
         # (tile, key) entries: every tile that holds a row of a pair's target box
         first_tile = (pos * nrhs) // ROWS_PER_TILE

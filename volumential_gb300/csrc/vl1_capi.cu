@@ -65,7 +65,11 @@ cudaError_t lib_malloc_async(void **ptr, size_t bytes, cudaStream_t s) {
     }
     pool = pools[dev];
   }
-  return cudaMallocFromPoolAsync(ptr, bytes, pool, s);
+  e = cudaMallocFromPoolAsync(ptr, bytes, pool, s);
+  // (reported by the return value; left as the last error it would be taken
+  // for that of the caller's next launch)
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
 }
 
 }  // namespace vl1

@@ -392,7 +392,7 @@ class Plan:
             return True, none          # built when the tree comes again
         import torch
 
-        from .batched import get_schedule
+        from .batched import ScheduleError, get_schedule
         if torch.cuda.is_current_stream_capturing():
             return True, none
         try:
@@ -400,8 +400,17 @@ class Plan:
             sched = get_schedule(self, view, keep, rows, stream)
             if sched.max_keys_per_item > cap:
                 sched = get_schedule(self, view, keep, rows, stream, max_keys_per_item=cap)
-        except (ValueError, RuntimeError):
-            sched = None
+        except (ValueError, ScheduleError):
+            return False, none         # no schedule describes this tree
+        except RuntimeError as e:
+            code = getattr(e, "code", None)
+            if code in (_lib.VL1_E_INVALID_CASE, _lib.VL1_E_LAYOUT, _lib.VL1_E_ARG,
+                        _lib.VL1_E_UNSUPPORTED):
+                return False, none     # (the per-box kernel reports what is wrong)
+            if (isinstance(e, torch.OutOfMemoryError) or code == _lib.VL1_E_NOMEM
+                    or code == _lib.VL1_E_CUDA and "out of memory" in str(e)):
+                return True, none      # this call only
+            raise
         return False, (self._proxy, sched)
 
     def _per_box_us(self, view, keep, rows, nrhs):

@@ -4,6 +4,10 @@ that plans which alternate on one tree all leave the per-box kernel.
 Both kernels are FP64-accurate (a few units of 2^-53 of the sums' magnitude), so
 they agree to 1e-13 relative l2."""
 
+import gc
+import weakref
+
+import numpy as np
 import pytest
 
 from helpers import plan_and_view, rel_l2, wrangler_for
@@ -86,3 +90,54 @@ def test_other_errors_while_building_are_raised(cuda, monkeypatch):
     monkeypatch.setattr(batched.MixedSchedule, "__init__", fails)
     with pytest.raises(RuntimeError, match="planted"):
         plan.eval_fp64(view, c, out, stream=0, keep=keep)
+
+
+def test_schedules_go_with_their_views(cuda):
+    """FP64 evaluations of many trees keep no tree longer than the view cache
+    does, and nothing in the mixed path's schedule cache."""
+    from volumential_gb300 import plan as plan_module
+    from volumential_gb300.plan import tree_view_from_arrays
+
+    torch = cuda
+    w = W.uniform_workload("many_trees", 3, 3, 4, seed=64)
+    plan, view, keep = plan_and_view(w)
+    c = torch.from_numpy(w.coefs[0]).cuda()
+    out = torch.empty_like(c)
+    before = len(batched._cache)
+    seen = []
+    for _ in range(20):
+        k = {n: t.clone() for n, t in keep.items()}
+        args = dict(zip(plan_module._VIEW_ARGS, (k[n] for n in plan_module._VIEW_KEYS)))
+        for _ in range(2):
+            v, kk = tree_view_from_arrays(root_extent=view.root_extent, **args)
+            plan.eval_fp64(v, c, out, stream=0, keep=kk)
+        assert v.fp64_schedules[1][1] is not None
+        seen.append(weakref.ref(k["lists"]))
+        del v, kk, k, args
+    plan.raise_on_status(0)
+    assert len(batched._cache) == before
+    gc.collect()
+    assert sum(r() is not None for r in seen) <= 8
+
+
+def test_schedules_do_not_keep_plans(cuda):
+    torch = cuda
+    w = W.uniform_workload("plan_ref", 3, 3, 4, seed=65)
+    _, view, keep = plan_and_view(w)
+    c = torch.from_numpy(w.coefs[0]).cuda()
+    out = torch.empty_like(c)
+    p = _second_plan(w, 2.0)
+    for _ in range(2):
+        p.eval_fp64(view, c, out, stream=0, keep=keep)
+    assert view.fp64_schedules[1][1] is not None
+    torch.cuda.synchronize()
+    ref = weakref.ref(p)
+    del p
+    gc.collect()
+    assert ref() is None
+    plan, _, _ = plan_and_view(w)
+    for _ in range(3):                 # another plan, perhaps at the same address
+        plan.eval_fp64(view, c, out, stream=0, keep=keep)
+    want = torch.empty_like(c)
+    plan.eval_fp64(view, c, want, stream=0)
+    assert rel_l2(out.cpu().numpy(), np.asarray(want.cpu())) <= 1e-13

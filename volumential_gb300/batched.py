@@ -54,12 +54,11 @@ class MixedSchedule:
     ~1 s of host time), for trees evaluated many times."""
 
     def __init__(self, plan, view, keep, nrhs, stream, max_keys_per_item=None, base=None,
-                 workspace=True, packing="device"):
-        import torch
-
+                 workspace=True, packing="device", split_scratch=True):
         lib = _lib.lib()
         self.nrhs = int(nrhs)
         self._workspace = None
+        self._split_scratch = split_scratch
         self.packing = packing if base is None else base.packing
         # bytes of vl1_eval_mixed's workspace, allocated on first use
         # (schedules of a batch use the batch's buffer instead)
@@ -192,10 +191,13 @@ class MixedSchedule:
                                              else np.zeros((1, 8), np.int32))
         self.items = torch.from_numpy(self.items_np).to("cuda")
         # one counter per split tile and column chunk, spaced 16 apart
-        self.split_counters = torch.zeros(max(1, n_splits * n_chunks * 16), dtype=torch.int32,
-                                          device="cuda")
-        self.split_partials = torch.zeros(max(16, n_slots * ROWS_PER_TILE * geo["np"] * 8),
-                                          dtype=torch.uint8, device="cuda")
+        # (vl1_eval_fp64_tiles has scratch of its own)
+        self.split_counters = self.split_partials = None
+        if self._split_scratch:
+            self.split_counters = torch.zeros(max(1, n_splits * n_chunks * 16),
+                                              dtype=torch.int32, device="cuda")
+            self.split_partials = torch.zeros(max(16, n_slots * ROWS_PER_TILE * geo["np"] * 8),
+                                              dtype=torch.uint8, device="cuda")
         s = _lib.MixedSchedule()
         s.n_tiles = n_tiles
         s.tile_rows = self.tile_rows.data_ptr()
@@ -206,8 +208,9 @@ class MixedSchedule:
         s.items = self.items.data_ptr()
         s.n_splits = n_splits
         s.n_slots = n_slots
-        s.split_counters = self.split_counters.data_ptr()
-        s.split_partials = self.split_partials.data_ptr()
+        if self._split_scratch:
+            s.split_counters = self.split_counters.data_ptr()
+            s.split_partials = self.split_partials.data_ptr()
         s.n_chunks = n_chunks
         self.n_chunks = n_chunks
         self.geometry = (geo["kc"], geo["nch"])

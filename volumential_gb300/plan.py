@@ -392,14 +392,16 @@ class Plan:
             return True, none          # built when the tree comes again
         import torch
 
-        from .batched import ScheduleError, get_schedule
+        from .batched import MixedSchedule, ScheduleError
         if torch.cuda.is_current_stream_capturing():
             return True, none
         try:
-            cap = self._tile_keys
-            sched = get_schedule(self, view, keep, rows, stream)
+            # the view's own: it goes with the view, not into the mixed path's
+            # cache of schedules (which holds their trees and plans)
+            cap, own = self._tile_keys, dict(workspace=False, split_scratch=False)
+            sched = MixedSchedule(self, view, keep, rows, stream, **own)
             if sched.max_keys_per_item > cap:
-                sched = get_schedule(self, view, keep, rows, stream, max_keys_per_item=cap)
+                sched = MixedSchedule(self, view, keep, rows, stream, cap, base=sched, **own)
         except (ValueError, ScheduleError):
             return False, none         # no schedule describes this tree
         except RuntimeError as e:

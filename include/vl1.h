@@ -217,6 +217,9 @@ int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
                             const vl1_mixed_schedule *schedule, const void *coefs,
                             int32_t coef_type, int32_t nrhs, void *result, void *stream);
 
+/* 1 while `stream` is being captured, 0 if not, -1 on an error. */
+int32_t vl1_stream_capturing(void *stream);
+
 /* The most keys a work item may have in vl1_eval_fp64_tiles; 0 for a plan that
  * vl1_eval_fp64_tiles evaluates as vl1_eval_fp64 (a NaN in its table). */
 int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan);

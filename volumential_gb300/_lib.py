@@ -183,6 +183,7 @@ SIGNATURES = {
                                         C.POINTER(MixedSchedule), C.c_void_p, C.c_int32,
                                         C.c_int32, C.c_void_p, C.c_void_p]),
     "vl1_eval_fp64_item_keys": (C.c_int32, [C.c_void_p]),
+    "vl1_stream_capturing": (C.c_int32, [C.c_void_p]),
     "vl1_orbit_index_map": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p,
                                         C.c_void_p]),
     "vl1_classify_pairs": (C.c_int32, [C.c_void_p, C.POINTER(TreeView), C.c_void_p,

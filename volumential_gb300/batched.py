@@ -43,6 +43,46 @@ class ScheduleError(RuntimeError):
     boxes of one case."""
 
 
+def stream_object(handle):
+    """The torch stream of a cudaStream_t."""
+    import torch
+
+    return torch.cuda.ExternalStream(handle) if handle else torch.cuda.default_stream()
+
+
+def _after_current(stream):
+    """Work queued on ``stream`` from here on runs after what torch's current
+    stream holds (whose memory pool the schedules' arrays come from)."""
+    import torch
+
+    current = torch.cuda.current_stream()
+    if current.cuda_stream != stream:
+        stream_object(stream).wait_stream(current)
+
+
+#: arrays of dropped schedules that could not be given back yet, with the
+#: stream they belong to and the events of the other streams that read them
+#: (a deque: entries come from finalizers, which must not wait for a lock)
+_held: "collections.deque" = collections.deque()
+_READERS_MAX = 64
+
+
+def _give_back(owner, events, arrays):
+    """Let ``owner``, the stream whose pool ``arrays`` return to, wait for the
+    ``events``; while it is being captured the arrays are kept."""
+    _held.append((owner, events, arrays))
+    for _ in range(len(_held)):
+        try:
+            entry = _held.popleft()
+        except IndexError:
+            return
+        if _lib.lib().vl1_stream_capturing(entry[0].cuda_stream) == 0:
+            for e in entry[1]:
+                entry[0].wait_event(e)
+        else:
+            _held.append(entry)
+
+
 class MixedSchedule:
     """Device-resident schedule (and workspace) of one (plan, tree, nrhs).
 
@@ -55,7 +95,12 @@ class MixedSchedule:
 
     def __init__(self, plan, view, keep, nrhs, stream, max_keys_per_item=None, base=None,
                  workspace=True, packing="device", split_scratch=True):
+        import torch
+
         lib = _lib.lib()
+        self._owner = torch.cuda.current_stream()
+        self._owner_handle = self._owner.cuda_stream
+        self._readers = {}
         self.nrhs = int(nrhs)
         self._workspace = None
         self._split_scratch = split_scratch
@@ -69,6 +114,7 @@ class MixedSchedule:
         if base is not None:
             # same plan, tree and nrhs: only the work items differ
             self._init_items(plan, base, max_keys_per_item)
+            _after_current(stream)
             if workspace:
                 _ = self.workspace
             return
@@ -79,8 +125,33 @@ class MixedSchedule:
         else:
             raise ValueError(f"packing must be 'device' or 'greedy', got {packing!r}")
         self._init_items(plan, self, max_keys_per_item)
+        _after_current(stream)
         if workspace:
             _ = self.workspace
+
+    def read_by(self, stream):
+        """Note that work queued on ``stream`` so far reads the schedule: its
+        arrays go back to their owner's memory pool after it."""
+        if stream == self._owner_handle or _lib.lib().vl1_stream_capturing(stream) != 0:
+            return
+        import torch
+
+        event = self._readers.get(stream)
+        if event is None:
+            if len(self._readers) >= _READERS_MAX:
+                _give_back(self._owner, list(self._readers.values()), None)
+                self._readers = {}
+            event = self._readers[stream] = torch.cuda.Event()
+        event.record(stream_object(stream))
+
+    def __del__(self):
+        readers = self.__dict__.get("_readers")
+        if not readers:
+            return
+        try:
+            _give_back(self._owner, list(readers.values()), dict(self.__dict__))
+        except Exception:      # the interpreter or the context is going away
+            pass
 
     @property
     def workspace(self):
@@ -117,6 +188,7 @@ class MixedSchedule:
             self.tile_key_start = dev(n_tiles + 1)
             self.key_ids = dev(n_ent)
             self.key_xrow = dev(max(n_ent, 1) * ROWS_PER_TILE)
+            _after_current(stream)
             _lib.check(lib.vl1_schedule_build_fill(
                 b, self.tile_rows.data_ptr(), self.tile_key_start.data_ptr(),
                 self.key_ids.data_ptr(), self.key_xrow.data_ptr(), C.c_void_p(stream)),

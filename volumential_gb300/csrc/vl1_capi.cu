@@ -423,6 +423,16 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree, const void *coe
                       static_cast<cudaStream_t>(stream));
 }
 
+int32_t vl1_stream_capturing(void *stream) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap);
+  if (e != cudaSuccess) {
+    cuda_fail(e, "cudaStreamIsCapturing");
+    return -1;
+  }
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // a work item's digit sums of weights 2^-56 .. 2^-72 must fit an int32:
 // (2^16 + 7 * 2^14) K < 2^31
 int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan) {

@@ -344,6 +344,7 @@ class Plan:
                 self.handle, C.byref(view), C.byref(sched.c_struct), coefs.data_ptr(), ctype,
                 int(nrhs), out.data_ptr(), C.c_void_p(stream))
             _lib.check(st, "vl1_eval_fp64_tiles")
+            sched.read_by(stream)
             return
         st = self._lib.vl1_eval_fp64(self.handle, C.byref(view), coefs.data_ptr(), ctype,
                                      int(nrhs), out.data_ptr(), C.c_void_p(stream))
@@ -392,7 +393,7 @@ class Plan:
             return True, none          # built when the tree comes again
         import torch
 
-        from .batched import MixedSchedule, ScheduleError
+        from .batched import MixedSchedule, ScheduleError, stream_object
         if torch.cuda.is_current_stream_capturing():
             return True, none
         try:
@@ -402,6 +403,7 @@ class Plan:
             sched = MixedSchedule(self, view, keep, rows, stream, **own)
             if sched.max_keys_per_item > cap:
                 sched = MixedSchedule(self, view, keep, rows, stream, cap, base=sched, **own)
+            stream_object(stream).synchronize()   # read on any stream from here on
         except (ValueError, ScheduleError):
             return False, none         # no schedule describes this tree
         except RuntimeError as e:

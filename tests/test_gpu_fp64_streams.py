@@ -149,3 +149,34 @@ def test_many_streams(problem, cuda):
     del s
     gc.collect()
     assert not _held
+
+
+def test_capture_of_a_stream_that_is_not_current(problem, cuda):
+    """The evaluation's stream is captured while torch's current stream is
+    another: no schedule is built (that would end the capture), the graph
+    replays the per-box kernel."""
+    torch = cuda
+    plan, view, keep, c, want = problem
+    ref = torch.empty_like(c)
+    plan.eval_fp64(view, c, ref, stream=0)
+    _forget(view)
+    a, out = torch.cuda.Stream(), torch.zeros_like(c)
+    plan.eval_fp64(view, c, out, stream=a.cuda_stream, keep=keep)      # seen
+    torch.cuda.synchronize()
+    out.zero_()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(a):
+        g.capture_begin(capture_error_mode="thread_local")
+        with torch.cuda.stream(torch.cuda.default_stream()):
+            plan.eval_fp64(view, c, out, stream=a.cuda_stream, keep=keep)
+        g.capture_end()
+    torch.cuda.synchronize()
+    assert torch.count_nonzero(out) == 0
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, ref)
+    plan.eval_fp64(view, c, out, stream=a.cuda_stream, keep=keep)
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    plan.raise_on_status(0)

@@ -394,7 +394,9 @@ class Plan:
         import torch
 
         from .batched import MixedSchedule, ScheduleError, stream_object
-        if torch.cuda.is_current_stream_capturing():
+        # (the build waits for `stream` and allocates on the current stream)
+        if (torch.cuda.is_current_stream_capturing()
+                or self._lib.vl1_stream_capturing(C.c_void_p(stream)) != 0):
             return True, none
         try:
             # the view's own: it goes with the view, not into the mixed path's

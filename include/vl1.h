@@ -208,7 +208,8 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree,
  * keeps FP64 accuracy against its own largest list-1 density (see
  * csrc/vl1_wide.cu); rows with non-finite sources are summed in FP64.
  * schedule: built for nrhs rows per box (2 nrhs for complex coefficients),
- * its work items at most vl1_eval_fp64_item_keys keys long.  The first call
+ * its work items at most vl1_eval_fp64_item_keys keys long (longer ones write
+ * nothing and set the status word to VL1_E_ARG).  The first call
  * with a plan builds its table digits and synchronises the stream; scratch
  * is allocated and freed in stream order.  Evaluates as vl1_eval_fp64 while
  * the stream is being captured, where the scratch cannot be had, where a

@@ -433,12 +433,10 @@ int32_t vl1_stream_capturing(void *stream) {
   return cap != cudaStreamCaptureStatusNone;
 }
 
-// a work item's digit sums of weights 2^-56 .. 2^-72 must fit an int32:
-// (2^16 + 7 * 2^14) K < 2^31
 int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan) {
   if (!plan || plan->table_nan) return 0;
   const int kp = vl1::wide_geometry(plan->d.nq, plan->d.table_cplx).kp;
-  return kp >= 8192 ? 1 : 8192 / kp;
+  return kp >= vl1::kItemPoints ? 1 : vl1::kItemPoints / kp;
 }
 
 int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,

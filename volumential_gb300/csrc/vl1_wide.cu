@@ -619,6 +619,9 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
       ok = item.key_begin >= p.sched.tile_key_start[item.tile] &&
            item.key_end <= p.sched.tile_key_start[item.tile + 1] &&
            item.key_begin <= item.key_end;
+    // (longer items' d = 7..9 sums could leave the int32 range unnoticed)
+    const int n_keys = item.key_end - item.key_begin;
+    ok = ok && (n_keys <= 1 || (int64_t)n_keys * p.g.kp <= kItemPoints);
     if (item.split >= 0)
       ok = ok && item.split < p.sched.n_splits && item.part >= 0 && item.part < item.nparts &&
            item.nparts < (1 << 16) && item.slot >= item.part &&

@@ -12,6 +12,10 @@ struct WideGeom {
   int kp, np, nch;
 };
 
+// source points of a work item of several keys: its digit sums of weights
+// 2^-56 .. 2^-72 must fit an int32, (2^16 + 7 * 2^14) K < 2^31
+constexpr int kItemPoints = 8192;
+
 struct WidePlan {
   WideGeom geom;
   __half *adig;    // table digits (nullptr until first needed)

@@ -218,6 +218,29 @@ int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
                             const vl1_mixed_schedule *schedule, const void *coefs,
                             int32_t coef_type, int32_t nrhs, void *result, void *stream);
 
+/* The arrays that a schedule was made from: device copies of a tree's
+ * target_boxes, neighbour starts and lists, box_centers, box_levels,
+ * box_source_starts, box_source_counts_nonchild and source_mode_ids (the other
+ * pointers are not read), the tree's sizes and root_extent, the number of
+ * list entries, and one int32 in device memory that is zero at first and set
+ * for good by an evaluation that finds other arrays. */
+typedef struct {
+  vl1_tree_view tree;
+  int64_t nnz;
+  int32_t *stale;
+} vl1_tree_copy;
+
+/* As vl1_eval_fp64_tiles, for a schedule made from the arrays in `made_from`:
+ * the tree's arrays are compared with them (on the device, in every call).
+ * Where they differ the results are those of vl1_eval_fp64 on the arrays as
+ * they are, *made_from->stale is set and vl1_status_read_stale returns 1; the
+ * schedule is then of no use (summing without it is far slower than
+ * vl1_eval_fp64). */
+int32_t vl1_eval_fp64_tiles_of(vl1_plan *plan, const vl1_tree_view *tree,
+                               const vl1_tree_copy *made_from,
+                               const vl1_mixed_schedule *schedule, const void *coefs,
+                               int32_t coef_type, int32_t nrhs, void *result, void *stream);
+
 /* 1 while `stream` is being captured, 0 if not, -1 on an error. */
 int32_t vl1_stream_capturing(void *stream);
 
@@ -579,6 +602,12 @@ int32_t vl1_orbit_index_map(vl1_plan *plan, int32_t *rows, int8_t *signs,
  * when reset != 0, clear it. */
 int32_t vl1_status_read(vl1_plan *plan, vl1_status *out, int32_t reset,
                         void *stream);
+
+/* The same, and in *stale (when not null) whether an evaluation of the plan
+ * found a schedule made from other arrays (vl1_eval_fp64_tiles_of); no error.
+ * reset clears that too. */
+int32_t vl1_status_read_stale(vl1_plan *plan, vl1_status *out, int32_t *stale,
+                              int32_t reset, void *stream);
 
 /* Bytes of device memory the plan holds (tables, blocks, descriptors). */
 int64_t vl1_plan_device_bytes(const vl1_plan *plan);

@@ -103,6 +103,10 @@ class MixedItem(C.Structure):
                 ("slot", C.c_int32), ("reserved", C.c_int32)]
 
 
+class TreeCopy(C.Structure):
+    _fields_ = [("tree", TreeView), ("nnz", C.c_int64), ("stale", C.c_void_p)]
+
+
 class MixedSchedule(C.Structure):
     _fields_ = [
         ("n_tiles", C.c_int32), ("tile_rows", C.c_void_p), ("tile_key_start", C.c_void_p),
@@ -182,6 +186,10 @@ SIGNATURES = {
     "vl1_eval_fp64_tiles": (C.c_int32, [C.c_void_p, C.POINTER(TreeView),
                                         C.POINTER(MixedSchedule), C.c_void_p, C.c_int32,
                                         C.c_int32, C.c_void_p, C.c_void_p]),
+    "vl1_eval_fp64_tiles_of": (C.c_int32, [C.c_void_p, C.POINTER(TreeView),
+                                           C.POINTER(TreeCopy), C.POINTER(MixedSchedule),
+                                           C.c_void_p, C.c_int32, C.c_int32, C.c_void_p,
+                                           C.c_void_p]),
     "vl1_eval_fp64_item_keys": (C.c_int32, [C.c_void_p]),
     "vl1_stream_capturing": (C.c_int32, [C.c_void_p]),
     "vl1_orbit_index_map": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p,
@@ -234,6 +242,8 @@ SIGNATURES = {
                                            C.c_void_p, C.c_void_p]),
     "vl1_status_read": (C.c_int32, [C.c_void_p, C.POINTER(Status), C.c_int32,
                                     C.c_void_p]),
+    "vl1_status_read_stale": (C.c_int32, [C.c_void_p, C.POINTER(Status),
+                                          C.POINTER(C.c_int32), C.c_int32, C.c_void_p]),
     "vl1_plan_device_bytes": (C.c_int64, [C.c_void_p]),
 }
 

@@ -83,6 +83,13 @@ def _give_back(owner, events, arrays):
             _held.append(entry)
 
 
+#: the tree arrays that a schedule depends on: name in ``keep``, view field
+_COPIED = (("target_boxes", "target_boxes"), ("starts", "neighbor_source_boxes_starts"),
+           ("lists", "neighbor_source_boxes_lists"), ("centers", "box_centers"),
+           ("levels", "box_levels"), ("src_starts", "box_source_starts"),
+           ("src_counts", "box_source_counts_nonchild"), ("smode", "source_mode_ids"))
+
+
 class MixedSchedule:
     """Device-resident schedule (and workspace) of one (plan, tree, nrhs).
 
@@ -128,6 +135,31 @@ class MixedSchedule:
         _after_current(stream)
         if workspace:
             _ = self.workspace
+
+    def copy_tree(self, view, keep, stream):
+        """Keep a copy of the tree arrays that the schedule depends on
+        (``tree_copy``, a ``vl1_tree_copy``), for evaluations to compare the
+        tree with: the arrays belong to the caller, who may write them."""
+        import torch
+
+        copies = {name: torch.empty_like(keep[name]) for name, _ in _COPIED}
+        self._stale = torch.zeros(1, dtype=torch.int32, device="cuda")
+        _after_current(stream)
+        with torch.cuda.stream(stream_object(stream)):
+            for name, t in copies.items():
+                t.copy_(keep[name])
+        c = _lib.TreeCopy()
+        C.memmove(C.byref(c.tree), C.byref(view), C.sizeof(_lib.TreeView))
+        for name, field in _COPIED:
+            setattr(c.tree, field, copies[name].data_ptr())
+        c.nnz = int(keep["lists"].numel())
+        c.stale = self._stale.data_ptr()
+        self._tree_arrays = copies
+        self.tree_copy = c
+
+    def is_stale(self):
+        """Whether an evaluation found other tree arrays (a device read)."""
+        return bool(self._stale.item())
 
     def read_by(self, stream):
         """Note that work queued on ``stream`` so far reads the schedule: its

@@ -221,10 +221,10 @@ int32_t vl1_plan_create(const vl1_plan_desc *desc, vl1_plan **plan_out) {
   }
   if (!st) {
     void *ptr = nullptr;
-    st = plan_alloc(p, &ptr, sizeof(vl1_status));
+    st = plan_alloc(p, &ptr, sizeof(PlanStatus));
     if (!st) {
       p->status = static_cast<vl1_status *>(ptr);
-      cudaError_t e = cudaMemset(ptr, 0, sizeof(vl1_status));
+      cudaError_t e = cudaMemset(ptr, 0, sizeof(PlanStatus));
       if (e != cudaSuccess) st = cuda_fail(e, "cudaMemset(status)");
     }
   }
@@ -439,9 +439,10 @@ int32_t vl1_eval_fp64_item_keys(const vl1_plan *plan) {
   return kp >= vl1::kItemPoints ? 1 : vl1::kItemPoints / kp;
 }
 
-int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
-                            const vl1_mixed_schedule *schedule, const void *coefs,
-                            int32_t coef_type, int32_t nrhs, void *result, void *stream) {
+int32_t vl1_eval_fp64_tiles_of(vl1_plan *plan, const vl1_tree_view *tree,
+                               const vl1_tree_copy *made_from,
+                               const vl1_mixed_schedule *schedule, const void *coefs,
+                               int32_t coef_type, int32_t nrhs, void *result, void *stream) {
   if (!plan || !schedule) {
     set_error("vl1_eval_fp64_tiles: null plan or schedule");
     return VL1_E_ARG;
@@ -452,8 +453,9 @@ int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamIsCapturing");
   // beyond vl1_eval_fp64's own limits its error is reported; a NaN in the
   // table has no digits (its block would take the scale of its whole level)
-  if (cap != cudaStreamCaptureStatusNone || plan->table_nan || plan->d.nq > 256 || nrhs < 1 || nrhs > 65535 ||
-      !coefs || !result || (coef_type != VL1_REAL64 && coef_type != VL1_COMPLEX128))
+  if (cap != cudaStreamCaptureStatusNone || plan->table_nan || plan->d.nq > 256 ||
+      nrhs < 1 || nrhs > 65535 || !coefs || !result ||
+      (coef_type != VL1_REAL64 && coef_type != VL1_COMPLEX128))
     return vl1_eval_fp64(plan, tree, coefs, coef_type, nrhs, result, stream);
   TreeDev tr;
   int32_t st = make_tree(plan, tree, tr);
@@ -467,11 +469,33 @@ int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
     set_error("vl1_eval_fp64_tiles: invalid schedule");
     return VL1_E_ARG;
   }
-  st = launch_wide(plan, tr, sc, static_cast<const double *>(coefs),
+  if (made_from) {
+    const vl1_tree_view &c = made_from->tree;
+    if (!made_from->stale || made_from->nnz < 0 || !c.target_boxes ||
+        !c.neighbor_source_boxes_starts || !c.neighbor_source_boxes_lists || !c.box_centers ||
+        !c.box_levels || !c.box_source_starts || !c.box_source_counts_nonchild ||
+        !c.source_mode_ids) {
+      set_error("vl1_eval_fp64_tiles_of: a copied tree array is missing");
+      return VL1_E_ARG;
+    }
+    // another tree altogether
+    if (c.n_target_boxes != tree->n_target_boxes || c.nboxes != tree->nboxes ||
+        c.aligned_nboxes != tree->aligned_nboxes || c.n_particles != tree->n_particles ||
+        c.root_extent != tree->root_extent)
+      return vl1_eval_fp64(plan, tree, coefs, coef_type, nrhs, result, stream);
+  }
+  st = launch_wide(plan, tr, made_from, sc, static_cast<const double *>(coefs),
                    coef_type == VL1_COMPLEX128, nrhs, static_cast<double *>(result), s);
   if (st == VL1_E_NOMEM || st == VL1_E_UNSUPPORTED)
     return vl1_eval_fp64(plan, tree, coefs, coef_type, nrhs, result, stream);
   return st;
+}
+
+int32_t vl1_eval_fp64_tiles(vl1_plan *plan, const vl1_tree_view *tree,
+                            const vl1_mixed_schedule *schedule, const void *coefs,
+                            int32_t coef_type, int32_t nrhs, void *result, void *stream) {
+  return vl1_eval_fp64_tiles_of(plan, tree, nullptr, schedule, coefs, coef_type, nrhs, result,
+                                stream);
 }
 
 int32_t vl1_classify_pairs(vl1_plan *plan, const vl1_tree_view *tree, int32_t *keys,
@@ -590,23 +614,32 @@ int32_t vl1_orbit_index_map(vl1_plan *plan, int32_t *rows, int8_t *signs, void *
   return launch_index_map(plan, rows, signs, static_cast<cudaStream_t>(stream));
 }
 
-int32_t vl1_status_read(vl1_plan *plan, vl1_status *out, int32_t reset, void *stream) {
+int32_t vl1_status_read_stale(vl1_plan *plan, vl1_status *out, int32_t *stale, int32_t reset,
+                              void *stream) {
   if (!plan || !out) {
     set_error("vl1_status_read: null argument");
     return VL1_E_ARG;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaError_t e = cudaMemcpyAsync(out, plan->status, sizeof(vl1_status),
-                                  cudaMemcpyDeviceToHost, s);
+  PlanStatus host;
+  cudaError_t e =
+      cudaMemcpyAsync(&host, plan->status, sizeof(host), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   // a clear word needs no clearing (the usual case: one launch and one wait
   // less behind every evaluation)
-  if (e == cudaSuccess && reset && (out->code != 0 || out->count != 0)) {
-    e = cudaMemsetAsync(plan->status, 0, sizeof(vl1_status), s);
+  if (e == cudaSuccess && reset &&
+      (host.status.code != 0 || host.status.count != 0 || (stale && host.stale != 0))) {
+    e = cudaMemsetAsync(plan->status, 0, stale ? sizeof(PlanStatus) : sizeof(vl1_status), s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   }
   if (e != cudaSuccess) return cuda_fail(e, "vl1_status_read");
+  *out = host.status;
+  if (stale) *stale = host.stale != 0;
   return VL1_OK;
+}
+
+int32_t vl1_status_read(vl1_plan *plan, vl1_status *out, int32_t reset, void *stream) {
+  return vl1_status_read_stale(plan, out, nullptr, reset, stream);
 }
 
 }  // extern "C"

@@ -55,6 +55,13 @@ constexpr int kNoScaleLog2 = 127;
 constexpr int kScaleLevels = 32;
 constexpr int kTileRows = 128;   // rows (target box, rhs) of a mixed-path tile
 
+// a plan's status word in device memory, and whether an evaluation found its
+// schedule made from other arrays than the tree's
+struct PlanStatus {
+  vl1_status status;
+  int32_t stale;
+};
+
 }  // namespace vl1
 
 struct vl1_plan {
@@ -64,7 +71,7 @@ struct vl1_plan {
   int64_t device_bytes;
   void *allocs[16];
   int n_allocs;
-  vl1_status *status;   // device
+  vl1_status *status;   // device, the first member of a vl1::PlanStatus
   vl1::MixedPlan mixed;
   vl1::WidePlan wide;
   int table_nan;        // nonzero: a table value is NaN (no fixed-point digits)
@@ -90,9 +97,10 @@ int32_t launch_plain(vl1_plan *plan, const TreeDev &tree, const double *coefs,
 // wide_operand_bytes of the plan
 int64_t wide_operand_bytes(const vl1_plan *plan);
 WideGeom wide_geometry(int nq, int table_cplx);
-int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_mixed_schedule &sched,
-                    const double *coefs, int coef_cplx, int nrhs, double *result,
-                    cudaStream_t s);
+// made_from: the copy of the arrays that the schedule was made from, or nullptr
+int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_tree_copy *made_from,
+                    const vl1_mixed_schedule &sched, const double *coefs, int coef_cplx,
+                    int nrhs, double *result, cudaStream_t s);
 // operand geometry; kc / nch 0: the default choice (else 16 or 32 / 16, 32
 // or 64, validated by the caller)
 MixedGeom mixed_geometry(int nq, int table_cplx, int kc = 0, int nch = 0);

@@ -201,6 +201,13 @@ __device__ __forceinline__ RowDigits row_digits(double v, int e) {
   return d;
 }
 
+// a tree array now and when the schedule was made
+struct Span {
+  const uint8_t *now, *then;
+  int64_t bytes, chunks;   // chunks: of 16 bytes, 0 for an array at an odd address
+};
+constexpr int kSpans = 8;
+
 // A density row is (source box b, virtual rhs v), row index b * nv + v.  Real
 // coefficients: v is the rhs.  Complex coefficients: v = 2 * rhs + part.
 struct WidePrep {
@@ -215,8 +222,34 @@ struct WidePrep {
   uint8_t *xpl;      // digits [row][unit][160 bytes], see wide_prep_kernel
   int *counters;     // split counters, zeroed here
   int n_counters;
+  Span spans[kSpans];
+  int64_t max_chunks;
+  int *stale;        // nullptr: the caller answers for the schedule
   vl1_status *st;
 };
+
+// Whether the arrays differ from those that the schedule was made from.  A
+// schedule outlives the call that made it, and its arrays' owner may write them
+// by ways that leave no trace on the host (a kernel, a graph's replay): every
+// call compares them, 16 bytes of every array at a time so that the loads are
+// in flight together (10 MB each on the 1.5M-point octree).
+__device__ __forceinline__ bool tree_differs(const WidePrep &P, int64_t i0, int64_t n) {
+  unsigned acc = 0u;
+  for (int64_t c = i0; c < P.max_chunks; c += n) {
+#pragma unroll
+    for (int k = 0; k < kSpans; ++k) {
+      if (c >= P.spans[k].chunks) continue;
+      const uint4 x = __ldg(reinterpret_cast<const uint4 *>(P.spans[k].now) + c);
+      const uint4 y = __ldg(reinterpret_cast<const uint4 *>(P.spans[k].then) + c);
+      acc |= (x.x ^ y.x) | (x.y ^ y.y) | (x.z ^ y.z) | (x.w ^ y.w);
+    }
+  }
+#pragma unroll 1
+  for (int k = 0; k < kSpans; ++k)   // the last bytes, and arrays at odd addresses
+    for (int64_t b = P.spans[k].chunks * 16 + i0; b < P.spans[k].bytes; b += n)
+      acc |= (unsigned)(P.spans[k].now[b] ^ P.spans[k].then[b]);
+  return acc != 0u;
+}
 
 constexpr int kPrepRows = 4;   // rows per warp and pass: their loads overlap
 
@@ -239,6 +272,11 @@ __global__ void __launch_bounds__(128) wide_prep_kernel(const __grid_constant__ 
   uint8_t *stage = s_stage + (threadIdx.x >> 5) * kPrepRows * row_bytes;
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < P.n_counters; i += blockDim.x) P.counters[i] = 0;
+  if (P.stale && tree_differs(P, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
+                              (int64_t)gridDim.x * blockDim.x)) {
+    *P.stale = 1;
+    reinterpret_cast<PlanStatus *>(P.st)->stale = 1;
+  }
   const int64_t n_rows = tr.nboxes * P.nv;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int cs = P.cc ? 2 : 1;
@@ -399,6 +437,7 @@ struct WideParams {
   int *counters;           // [split][chunk]
   const double *coefs;
   double *result;
+  const int *stale;        // nonzero: the schedule is not this tree's (nullptr: it is)
   vl1_status *st;
   uint32_t wait_limit_us;
   int32_t withhold_arrival;
@@ -488,65 +527,67 @@ __device__ __forceinline__ double wide_value(long long S, long long L, int k) {
   return scaled_i64_to_double(tot, k - 48 - sh);
 }
 
-// A row's target outputs in FP64, for rows with non-finite sources: every
-// thread one target point at a time, the pairs in list order.
-__device__ __noinline__ void wide_slow_row(const WideParams &p, int tb, int r) {
+// One target point of a row in FP64, the pairs in list order, from the tree's
+// arrays alone: rows with non-finite sources, and all rows when the schedule is
+// not the tree's.
+__device__ __noinline__ void wide_slow_point(const WideParams &p, int tb, int r, int t) {
   const DevDesc &d = p.d;
   const TreeDev &tr = p.tr;
   const int tbox = tr.target_boxes[tb];
   const int tbeg = tr.tgt_starts[tbox];
-  const int cnt = min(tr.tgt_counts[tbox], d.nq);
   const int64_t ro = (int64_t)r * tr.n_particles;
   const bool oc = d.table_cplx || p.cc;
-  for (int t = threadIdx.x; t < cnt; t += blockDim.x) {
-    const int tm = tr.tmode[tbeg + t];
-    double a_re = 0.0, a_im = 0.0, w_re = 0.0, w_im = 0.0;
-    for (int q = tr.starts[tb]; q < tr.starts[tb + 1] && tm >= 0 && tm < d.nq; ++q) {
-      const int sbox = tr.lists[q];
-      const int lvl = tr.levels[sbox];
-      const double ext = level_extent(tr.root_extent, lvl);
-      const int c = pair_case_id(d, tr, tbox, sbox, ext);
-      if (c < 0) continue;
-      const int lev = pair_table_level(d, lvl);
-      const double scl = pair_scaling(d, ext);
-      const double df = d.disp_kind == VL1_DISP_LOG2D
-                            ? __dmul_rn(__dmul_rn(d.disp_coef, scl),
-                                        log(__ddiv_rn(ext, d.table_root_extent)))
-                            : 0.0;
-      const int sbeg = tr.src_starts[sbox], ns = min(tr.src_counts[sbox], d.nq);
-      const int64_t blk = ((int64_t)lev * d.n_cases + c) * d.nq * d.nq;
-      for (int s = 0; s < ns; ++s) {
-        const int sm = tr.smode[sbeg + s];
-        if (sm < 0 || sm >= d.nq) continue;
-        const int64_t ci = ro + sbeg + s;
-        const double c_re = p.cc ? p.coefs[2 * ci] : p.coefs[ci];
-        const double c_im = p.cc ? p.coefs[2 * ci + 1] : 0.0;
-        const int64_t bi = blk + (int64_t)sm * d.nq + tm;
-        const double b_re = d.table_cplx ? d.blocks[2 * bi] : d.blocks[bi];
-        const double x_re = c_re * scl, x_im = c_im * scl;
-        a_re = fma(x_re, b_re, a_re);
-        if (p.cc) a_im = fma(x_im, b_re, a_im);
-        if (d.table_cplx) {
-          const double b_im = d.blocks[2 * bi + 1];
-          a_im = fma(x_re, b_im, a_im);
-          if (p.cc) a_re = fma(-x_im, b_im, a_re);
-        }
-        if (d.disp_kind == VL1_DISP_LOG2D) {
-          const int64_t ni = (int64_t)lev * d.nq + s;
-          const double n_re = df * (d.table_cplx ? d.nmlz[2 * ni] : d.nmlz[ni]);
-          const double n_im = d.table_cplx ? df * d.nmlz[2 * ni + 1] : 0.0;
-          w_re += c_re * n_re - c_im * n_im;
-          w_im += c_re * n_im + c_im * n_re;
-        }
+  const int tm = tr.tmode[tbeg + t];
+  if (tm < 0 || tm >= d.nq) report(p.st, VL1_E_LAYOUT, tb, -1 - t);
+  double a_re = 0.0, a_im = 0.0, w_re = 0.0, w_im = 0.0;
+  for (int q = tr.starts[tb]; q < tr.starts[tb + 1] && tm >= 0 && tm < d.nq; ++q) {
+    const int sbox = tr.lists[q];
+    const int lvl = tr.levels[sbox];
+    const double ext = level_extent(tr.root_extent, lvl);
+    const int c = pair_case_id(d, tr, tbox, sbox, ext);
+    if (c < 0) {
+      if (t == 0) report(p.st, VL1_E_INVALID_CASE, tb, q);
+      continue;
+    }
+    const int lev = pair_table_level(d, lvl);
+    const double scl = pair_scaling(d, ext);
+    const double df = d.disp_kind == VL1_DISP_LOG2D
+                          ? __dmul_rn(__dmul_rn(d.disp_coef, scl),
+                                      log(__ddiv_rn(ext, d.table_root_extent)))
+                          : 0.0;
+    const int sbeg = tr.src_starts[sbox], ns = min(tr.src_counts[sbox], d.nq);
+    const int64_t blk = ((int64_t)lev * d.n_cases + c) * d.nq * d.nq;
+    for (int s = 0; s < ns; ++s) {
+      const int sm = tr.smode[sbeg + s];
+      if (sm < 0 || sm >= d.nq) continue;
+      const int64_t ci = ro + sbeg + s;
+      const double c_re = p.cc ? p.coefs[2 * ci] : p.coefs[ci];
+      const double c_im = p.cc ? p.coefs[2 * ci + 1] : 0.0;
+      const int64_t bi = blk + (int64_t)sm * d.nq + tm;
+      const double b_re = d.table_cplx ? d.blocks[2 * bi] : d.blocks[bi];
+      const double x_re = c_re * scl, x_im = c_im * scl;
+      a_re = fma(x_re, b_re, a_re);
+      if (p.cc) a_im = fma(x_im, b_re, a_im);
+      if (d.table_cplx) {
+        const double b_im = d.blocks[2 * bi + 1];
+        a_im = fma(x_re, b_im, a_im);
+        if (p.cc) a_re = fma(-x_im, b_im, a_re);
+      }
+      if (d.disp_kind == VL1_DISP_LOG2D) {
+        const int64_t ni = (int64_t)lev * d.nq + s;
+        const double n_re = df * (d.table_cplx ? d.nmlz[2 * ni] : d.nmlz[ni]);
+        const double n_im = d.table_cplx ? df * d.nmlz[2 * ni + 1] : 0.0;
+        w_re += c_re * n_re - c_im * n_im;
+        w_im += c_re * n_im + c_im * n_re;
       }
     }
-    const int64_t o = ro + tbeg + t;
-    if (oc) {
-      p.result[2 * o] = a_re + w_re;
-      p.result[2 * o + 1] = a_im + w_im;
-    } else {
-      p.result[o] = a_re + w_re;
-    }
+  }
+  const int64_t o = ro + tbeg + t;
+  if (oc) {
+    p.result[2 * o] = a_re + w_re;
+    p.result[2 * o + 1] = a_im + w_im;
+  } else {
+    p.result[o] = a_re + w_re;
   }
 }
 
@@ -572,6 +613,7 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
   __shared__ long long s_out[128];          // result index of that particle
   __shared__ double s_disp[128][2];
   __shared__ int s_any_bad, s_last, s_poison;
+  __shared__ bool s_stale;
   __shared__ vl1_mixed_item s_item;   // kept here: the readout needs the registers
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -663,6 +705,7 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
     s_bad[tid] = 0;
   }
   grid_dep_wait();   // the density digits, their exponents and the split counters
+  if (tid == 0) s_stale = p.stale && *reinterpret_cast<const volatile int *>(p.stale) != 0;
   tc::tc_fence_before();
   __syncthreads();
   tc::tc_fence_after();
@@ -719,7 +762,7 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
     if (p.wbox) __syncthreads();   // s_part lies in the stages
   }
 
-  const int k0 = s_item.key_begin, k1 = s_item.key_end;
+  const int k0 = s_item.key_begin, k1 = s_stale ? k0 : s_item.key_end;
   const int n_units = (k1 - k0) * n_units_key;
   const int n_rounds = (n_units + kRoundUnits - 1) / kRoundUnits;
 
@@ -1047,8 +1090,9 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
   long long *s_S = reinterpret_cast<long long *>(smem);
   long long *s_L = s_S + 128 * PARK;
   const vl1_mixed_item item = s_item;
-  bool write = !s_abort && item.tile >= 0;
-  if (item.split >= 0) {
+  const bool stale = s_stale;
+  bool write = !s_abort && item.tile >= 0 && !stale;
+  if (item.split >= 0 && !stale) {
     // (a part that finds all others done keeps its sums in shared memory:
     // storing a part takes 17,000 clocks with every SM at it; 236 -> 233 us)
     int *const ctr = p.counters + (int64_t)item.split * n_chunks + chunk;
@@ -1172,8 +1216,19 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
         const int j = jv / p.nv, v = jv - j * p.nv;
         // complex coefficients: both parts of an output once
         if (p.cc && (v & 1) && s_bad[row - 1]) continue;
-        if (chunk == 0) wide_slow_row(p, j, p.cc ? v >> 1 : v);
+        if (chunk == 0)
+          for (int t = tid; t < s_cnt[row]; t += R::kThreads)
+            wide_slow_point(p, j, p.cc ? v >> 1 : v, t);
       }
+    }
+  }
+  if (stale && item.tile >= 0 && chunk == 0 && item.part == 0) {
+    const int nq = p.d.nq;
+    for (int i = tid; i < 128 * nq; i += R::kThreads) {
+      const int row = i / nq, t = i - row * nq, jv = s_row[row];
+      const int j = jv < 0 ? 0 : jv / p.nv, v = jv - j * p.nv;
+      if (jv >= 0 && t < s_cnt[row] && !(p.cc && (v & 1)))
+        wide_slow_point(p, j, p.cc ? v >> 1 : v, t);
     }
   }
   if (s_abort && tid == 0) report(p.st, VL1_E_TIMEOUT, item.tile, chunk);
@@ -1265,9 +1320,9 @@ static int32_t wide_operands(vl1_plan *plan, cudaStream_t s) {
   return VL1_OK;
 }
 
-int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_mixed_schedule &sched,
-                    const double *coefs, int coef_cplx, int nrhs, double *result,
-                    cudaStream_t s) {
+int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_tree_copy *made_from,
+                    const vl1_mixed_schedule &sched, const double *coefs, int coef_cplx,
+                    int nrhs, double *result, cudaStream_t s) {
   const DevDesc &d = plan->d;
   int32_t st = wide_operands(plan, s);
   if (st) return st;
@@ -1312,6 +1367,26 @@ int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_mixed_schedul
   pp.counters = reinterpret_cast<int *>(w);
   w += b_ctr;
   pp.n_counters = sched.n_splits * n_chunks;
+  pp.stale = made_from ? made_from->stale : nullptr;
+  pp.max_chunks = 0;
+  if (made_from) {
+    const vl1_tree_view &c = made_from->tree;
+    auto span = [&](int k, const void *now, const void *then, int64_t bytes) {
+      const bool odd =
+          ((reinterpret_cast<uintptr_t>(now) | reinterpret_cast<uintptr_t>(then)) & 15) != 0;
+      pp.spans[k] = Span{static_cast<const uint8_t *>(now), static_cast<const uint8_t *>(then),
+                         bytes, odd ? 0 : bytes / 16};
+      if (pp.spans[k].chunks > pp.max_chunks) pp.max_chunks = pp.spans[k].chunks;
+    };
+    span(0, tree.smode, c.source_mode_ids, 4 * tree.n_particles);
+    span(1, tree.lists, c.neighbor_source_boxes_lists, 4 * made_from->nnz);
+    span(2, tree.starts, c.neighbor_source_boxes_starts, 4 * ((int64_t)tree.n_tgt_boxes + 1));
+    span(3, tree.target_boxes, c.target_boxes, 4 * (int64_t)tree.n_tgt_boxes);
+    span(4, tree.src_starts, c.box_source_starts, 4 * tree.nboxes);
+    span(5, tree.src_counts, c.box_source_counts_nonchild, 4 * tree.nboxes);
+    span(6, tree.levels, c.box_levels, tree.nboxes);
+    span(7, tree.centers, c.box_centers, 8 * d.dim * tree.aligned_nboxes);
+  }
   pp.st = plan->status;
   WideParams mp;
   mp.d = d;
@@ -1331,6 +1406,7 @@ int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_mixed_schedul
   mp.counters = pp.counters;
   mp.coefs = coefs;
   mp.result = result;
+  mp.stale = made_from ? made_from->stale : nullptr;
   mp.st = plan->status;
   mp.wait_limit_us = g_test_wait_limit_us;
   mp.withhold_arrival = g_test_withhold;

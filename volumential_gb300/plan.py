@@ -289,6 +289,7 @@ class Plan:
         self._lib = lib
         self._serial = next(_serial)          # never used again, unlike id() or the handle
         self._proxy = weakref.proxy(self)
+        self._stale_seen = 0                  # evaluations that found a schedule stale
         # keys per work item of the FP64 tensor-core path; 0: per-box kernel only
         self._tile_keys = int(lib.vl1_eval_fp64_item_keys(handle))
 
@@ -325,8 +326,13 @@ class Plan:
 
         With ``keep`` (the tree's device tensors, as ``tree_view_from_arrays``
         returns them beside ``view``) large sums run on the tensor cores with
-        FP64-accurate digit products (``vl1_eval_fp64_tiles``), see
-        ``_fp64_schedule``; without it, in the per-box FP64 kernel."""
+        FP64-accurate digit products (``vl1_eval_fp64_tiles_of``), see
+        ``_fp64_schedule``; without it, in the per-box kernel.
+
+        The arrays in ``keep`` may be written in place: both kernels follow
+        them.  Two calls with the same arguments give the same bits when both
+        run in the same kernel: a tree's first call may run per box and the
+        later ones on the tensor cores, and a captured call runs per box."""
         import torch
         if coefs.dtype not in (torch.float64, torch.complex128):
             raise TypeError("coefs must be float64 or complex128")
@@ -340,10 +346,10 @@ class Plan:
         if keep is not None:
             sched = self._fp64_schedule(view, keep, coefs.is_complex(), int(nrhs), stream)
         if sched is not None:
-            st = self._lib.vl1_eval_fp64_tiles(
-                self.handle, C.byref(view), C.byref(sched.c_struct), coefs.data_ptr(), ctype,
-                int(nrhs), out.data_ptr(), C.c_void_p(stream))
-            _lib.check(st, "vl1_eval_fp64_tiles")
+            st = self._lib.vl1_eval_fp64_tiles_of(
+                self.handle, C.byref(view), C.byref(sched.tree_copy), C.byref(sched.c_struct),
+                coefs.data_ptr(), ctype, int(nrhs), out.data_ptr(), C.c_void_p(stream))
+            _lib.check(st, "vl1_eval_fp64_tiles_of")
             sched.read_by(stream)
             return
         st = self._lib.vl1_eval_fp64(self.handle, C.byref(view), coefs.data_ptr(), ctype,
@@ -369,16 +375,30 @@ class Plan:
             known = view._fp64_known = collections.OrderedDict()
             view.fp64_schedules = {}
         key = (self._serial, rows)
-        hit = known.get(key)       # None, or (seen before without a schedule, record)
+        # None, or (to be asked again, record, stale schedules seen until then)
+        hit = known.get(key)
         if hit is None or hit[0]:
             hit = self._fp64_decide(view, keep, rows, nrhs, stream, hit is not None)
-            known[key] = hit
+            hit = known[key] = (*hit, self._stale_seen)
             while len(known) > FP64_SCHEDULES_PER_VIEW:
                 known.popitem(last=False)
+        elif hit[2] != self._stale_seen and not self._capturing(stream):
+            # a tree of this plan was written in place: if this one, it stays
+            # with the per-box kernel, which reads the arrays in every call
+            record = hit[1]
+            if record[1] is not None and record[1].is_stale():
+                record = (self._proxy, None)
+            hit = known[key] = (False, record, self._stale_seen)
         # the decision of the last call, by row count: (plan, schedule or None)
         if view.fp64_schedules.get(rows) is not hit[1]:
             view.fp64_schedules[rows] = hit[1]
         return hit[1][1]
+
+    def _capturing(self, stream):
+        import torch
+
+        return (torch.cuda.is_current_stream_capturing()
+                or self._lib.vl1_stream_capturing(C.c_void_p(stream)) != 0)
 
     def _fp64_decide(self, view, keep, rows, nrhs, stream, again):
         """(to be asked again, (this plan, schedule or None)) for a view that
@@ -395,8 +415,7 @@ class Plan:
 
         from .batched import MixedSchedule, ScheduleError, stream_object
         # (the build waits for `stream` and allocates on the current stream)
-        if (torch.cuda.is_current_stream_capturing()
-                or self._lib.vl1_stream_capturing(C.c_void_p(stream)) != 0):
+        if self._capturing(stream):
             return True, none
         try:
             # the view's own: it goes with the view, not into the mixed path's
@@ -405,6 +424,7 @@ class Plan:
             sched = MixedSchedule(self, view, keep, rows, stream, **own)
             if sched.max_keys_per_item > cap:
                 sched = MixedSchedule(self, view, keep, rows, stream, cap, base=sched, **own)
+            sched.copy_tree(view, keep, stream)
             stream_object(stream).synchronize()   # read on any stream from here on
         except (ValueError, ScheduleError):
             return False, none         # no schedule describes this tree
@@ -460,9 +480,12 @@ class Plan:
         return out
 
     def read_status(self, stream=None, reset=True):
-        s = _lib.Status()
-        _lib.check(self._lib.vl1_status_read(self.handle, C.byref(s), int(reset),
-                                             C.c_void_p(stream or 0)), "vl1_status_read")
+        s, stale = _lib.Status(), C.c_int32()
+        _lib.check(self._lib.vl1_status_read_stale(self.handle, C.byref(s), C.byref(stale),
+                                                   int(reset), C.c_void_p(stream or 0)),
+                   "vl1_status_read")
+        if stale.value:
+            self._stale_seen += 1
         return s
 
     def raise_on_status(self, stream=None):

@@ -905,7 +905,10 @@ struct Barriers {
   uint64_t empty[kMaxStages];
   uint64_t accf[2];
   uint64_t acce[2];
-  uint64_t taile;            // the item's tail accumulators have been read
+  // an item's tail accumulators have been read; one phase per item with units
+  // (an item without has none to read: its phase would not depend on the
+  // tensor-core issuer, and two such could pass before it looked at one)
+  uint64_t taile;
   uint64_t wfull[kWorkSlots], wempty[kWorkSlots];   // work item records
   uint64_t rfull[kWorkSlots];   // the item's row data
   uint64_t drain;            // after an abort: every issued MMA has completed
@@ -1401,6 +1404,7 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
     int s = 0;
     uint32_t ph = 0;   // phase parity of stage s
     uint32_t R = 0;    // exact rounds of this CTA
+    uint32_t n_run = 0;   // items with units so far (the phases of taile)
     // the barriers of the next unit are looked at between the products of
     // this one, and waited for at its start only if they were not complete
     bool have_a = false, have_x = false, aborted = false;
@@ -1453,8 +1457,8 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
 #pragma unroll
           for (int g = 0; g < kExactGroups; ++g)
             group(kk, g, g == 0 && kk == 0 && iu == 0 ? 0u : 1u);
-        if (u == 0 && j > 0) {
-          if (!wait(&bars.taile, (j - 1) & 1)) {
+        if (u == 0 && n_run > 0) {
+          if (!wait(&bars.taile, (n_run - 1) & 1)) {
             aborted = true;
             break;
           }
@@ -1476,8 +1480,7 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
           ++R;
         }
       }
-      // every phase of taile is waited for, also by an item without units
-      if (!aborted && n_units == 0 && j > 0 && !wait(&bars.taile, (j - 1) & 1)) aborted = true;
+      if (n_units > 0) ++n_run;
     }
     if (aborted || s_abort) {
       // MMAs issued before the abort still write TMEM and read the stages:
@@ -1575,10 +1578,6 @@ mixed_kernel(const __grid_constant__ MixedParams p1, const __grid_constant__ Bat
           acc[c] += ((unsigned long long)b2 << 32) + (unsigned long long)b3 * 16777216ull;
           acc[c] += (unsigned long long)((long long)__float2int_rn(__uint_as_float(r4[c])) * 65536);
         }
-      }
-      if (n_rounds == 0) {
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.taile);
       }
       {
         // the constant parts of the raw bits, (kMagicBits << 32) +

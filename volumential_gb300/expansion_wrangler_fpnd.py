@@ -115,6 +115,8 @@ def _leading(x, n, fresh=False):
     """``x[..., arange(n)]``, a new tensor (``fresh``: x itself is one)."""
     import torch
 
+    if not x.is_cuda:   # as an index on the device would
+        raise RuntimeError("potentials and densities must be CUDA tensors here")
     if x.shape[-1] < n:
         raise IndexError(f"array of {x.shape[-1]} entries for {n} particles")
     if fresh and x.shape[-1] == n:

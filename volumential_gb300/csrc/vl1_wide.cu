@@ -4,8 +4,8 @@
 // The FP64 pipe of this GPU (about 1.1 TFLOP/s) bounds the plain kernel: a 3D
 // q = 4 tree of 1.5M points and 2.3e9 point pairs takes 4.7 ms at 0.98
 // TFLOP/s.  Here the same sums are formed from digit products, as in the
-// mixed path (vl1_mixed.cu), but with enough digits that nothing an FP64
-// evaluation would keep is lost:
+// mixed path (vl1_mixed.cu), but with so many digits that a box's results are
+// as accurate as FP64 sums against the largest product of its list:
 //
 //   x' = scaling * coefficient = 2^(E + 1) sum_{i=1..8} X_i 2^(-8i)
 //   T                          = 2^(A + 1) sum_{j=1..8} T_j 2^(-8j)
@@ -19,8 +19,8 @@
 // equal modulo 8 the sum against the largest one is a shift by whole digits,
 // so the producers only read each source's digit planes from an offset
 // (position p takes plane p - (E_t - E - A) / 8, zero above).  Every target
-// box thus has its own scale, as in an FP64 sum, whatever the range of the
-// density over the domain.
+// box thus has its own scale, the largest E + A of the pairs it sums, whatever
+// the range of the density over the domain and of the blocks over the table.
 //
 // The products i + j = d of weight 2^(-8d) share an accumulator: d = 2..6 are
 // exact integers over a round of 128 source points (at most
@@ -30,10 +30,18 @@
 // own, so their sums stay near 2^20, where FP32 is exact too; sums beyond
 // 2^24 need products of one sign throughout, leading digits included, and
 // then the rounding of d = 7 is below 2^-53 of the result.  d >= 10 is dropped
-// (below 2^-72 per pair).  The result is rounded once.  Against 113-bit sums
-// (2D and 3D, q = 1..16, Laplace- and Helmholtz-like tables, real and complex
-// densities, densities over 6 and 200 decades) the relative l2 error is
-// 4e-17 .. 2e-16, the per-box kernel's 1e-16 .. 2e-15.
+// (2^-66 per pair in the mean square).  The result is rounded once.  Against
+// 113-bit sums (2D and 3D, q = 1..16, Laplace- and Helmholtz-like tables, real
+// and complex densities, densities over 6 and 200 decades) the relative l2
+// error is 4e-17 .. 2e-16, the per-box kernel's 1e-16 .. 2e-15.
+//
+// The error is against max|x'| max|T| over a row's pairs, not against each
+// target's own products: with K source points at most 6 * 2^-50.2 sqrt(K) of
+// that maximum where the roundings of E and A to multiples of 8 fall worst
+// (test_gpu_fp64_digits.py), some 2^-60 where they fall well.  A target whose
+// products all lie far below it keeps fewer bits than an FP64 sum: with one
+// source point in the corner neighbour up to 1e-15 (3D, q = 4) and 5e-15 (2D,
+// q = 6) of its value, 1e-16 per box.
 //
 // Measured (GB300): the 1.5M-point octree 4,700 us per-box, 229 us here
 // (digits 22 us, tensor-core kernel 206 us, its tensor pipe busy 105 us of
@@ -119,9 +127,8 @@ __device__ __forceinline__ int wide_digit(const WideDigits &d, int i, int sgn) {
 // ----------------------------------------------------- plan: table digits
 
 // exponent of every (table level, case) block: the smallest A >= the block's
-// own exponent that equals a_max modulo 8 (kZeroExp for a zero block), and
-// the largest of every table level (level_exp, preset below every exponent)
-__global__ void wide_key_exp_kernel(DevDesc d, int a_max, int *key_exp, int *level_exp) {
+// own exponent that equals a_max modulo 8 (kZeroExp for a zero block)
+__global__ void wide_key_exp_kernel(DevDesc d, int a_max, int *key_exp) {
   const int key = blockIdx.x;
   const int64_t n = (int64_t)d.nq * d.nq * (d.table_cplx ? 2 : 1);
   const double *B = d.blocks + (int64_t)key * n;
@@ -135,11 +142,8 @@ __global__ void wide_key_exp_kernel(DevDesc d, int a_max, int *key_exp, int *lev
   __syncthreads();
   if (e != kZeroExp) atomicMax(&s_e, e);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    const int a = s_e == kZeroExp ? kZeroExp : a_max - 8 * ((a_max - s_e) / 8);
-    key_exp[key] = a;
-    atomicMax(level_exp + key / d.n_cases, a);
-  }
+  if (threadIdx.x == 0)
+    key_exp[key] = s_e == kZeroExp ? kZeroExp : a_max - 8 * ((a_max - s_e) / 8);
 }
 
 // digits of the blocks: [key][unit][column chunk][digit][nch][16] FP16 in the
@@ -432,7 +436,7 @@ struct WideParams {
   const double *wbox;
   int n_xrows, n_keys;
   const __half *adig;
-  const int *key_exp;      // per (table level, case) block, then per table level (the largest)
+  const int *key_exp;      // per (table level, case) block
   longlong2 *partials;     // [slot][chunk][128][nch]: (S, L)
   int *counters;           // [split][chunk]
   const double *coefs;
@@ -712,9 +716,8 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
   const uint32_t tbase = tmem_base;
 
   // each row's exponent and displacement sum over its target box's list (all
-  // of it: the parts of a split tile share them); kThreads / 128 threads per
-  // row.  A source counts with the largest block exponent of its table level,
-  // so that the pair's case is not needed here.
+  // of it: the parts of a split tile share them), which is the row's entries
+  // of the tile's keys; kThreads / 128 threads per row
   {
     constexpr int NP = R::kThreads / 128;
     double *s_part = reinterpret_cast<double *>(smem);   // [NP][128][2]
@@ -722,21 +725,22 @@ __global__ void __launch_bounds__(WideRoles<NCH>::kThreads, WideRoles<NCH>::kCta
     if (part < NP) {
       int e = kZeroExp, bad = 0;
       double w_re = 0.0, w_im = 0.0;
-      const int rv = s_row[row];
-      const int j = rv < 0 ? 0 : rv / p.nv, v = rv < 0 ? 0 : rv - j * p.nv;
-      const int q0 = rv < 0 ? 0 : p.tr.starts[j], q1 = rv < 0 ? 0 : p.tr.starts[j + 1];
+      const bool have = s_row[row] >= 0;
+      const int t0 = s_item.tile < 0 ? 0 : p.sched.tile_key_start[s_item.tile];
+      const int t1 = s_item.tile < 0 ? 0 : p.sched.tile_key_start[s_item.tile + 1];
 #pragma unroll 4
-      for (int q = q0 + part; q < q1; q += NP) {
-        const int sb = p.tr.lists[q];
-        const int64_t xr = (int64_t)sb * p.nv + v;
+      for (int k = t0 + part; k < t1; k += NP) {
+        const int xr = have ? p.sched.key_xrow[(int64_t)k * 128 + row] : -1;
+        const int key = p.sched.key_ids[k];
+        if (xr < 0 || xr >= p.n_xrows || key < 0 || key >= p.n_keys) continue;
         const int ex = p.x_exp[xr];
         if (ex == kBadExp)
           bad = 1;
         else
-          e = max(e, ex + p.key_exp[p.n_keys + pair_table_level(p.d, p.tr.levels[sb])]);
+          e = max(e, ex + p.key_exp[key]);
         if (p.wbox) {
-          w_re += p.wbox[2 * xr];
-          w_im += p.wbox[2 * xr + 1];
+          w_re += p.wbox[2 * (int64_t)xr];
+          w_im += p.wbox[2 * (int64_t)xr + 1];
         }
       }
       if (e > kZeroExp / 2) atomicMax(&s_E[row], e);
@@ -1270,7 +1274,7 @@ WideGeom wide_geometry(int nq, int table_cplx) {
 int64_t wide_operand_bytes(const vl1_plan *plan) {
   const WideGeom g = wide_geometry(plan->d.nq, plan->d.table_cplx);
   const int64_t keys = (int64_t)plan->d.n_tables * plan->d.n_cases;
-  return round256((keys + plan->d.n_tables) * 4) + keys * g.kp * (int64_t)g.np * kW * 2;
+  return round256(keys * 4) + keys * g.kp * (int64_t)g.np * kW * 2;
 }
 
 // The plan's table digits, built on the first call that needs them (the
@@ -1297,14 +1301,8 @@ static int32_t wide_operands(vl1_plan *plan, cudaStream_t s) {
   }
   int *key_exp = static_cast<int *>(ptr);
   __half *adig = reinterpret_cast<__half *>(static_cast<uint8_t *>(ptr) +
-                                            round256((keys + d.n_tables) * 4));
-  e = cudaMemsetAsync(key_exp + keys, 0x80, 4 * (size_t)d.n_tables, s);
-  if (e != cudaSuccess) {
-    cudaFreeAsync(ptr, s);
-    return cuda_fail(e, "cudaMemsetAsync(table level exponents)");
-  }
-  wide_key_exp_kernel<<<(unsigned)keys, 256, 0, s>>>(d, plan->mixed.a_exp, key_exp,
-                                                    key_exp + keys);
+                                            round256(keys * 4));
+  wide_key_exp_kernel<<<(unsigned)keys, 256, 0, s>>>(d, plan->mixed.a_exp, key_exp);
   wide_digits_kernel<<<152 * 16, 256, 0, s>>>(d, g, key_exp, adig);
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

@@ -77,14 +77,6 @@ __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void *src,
                "r"(src_bytes)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() {
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
-// wait until at most N of this thread's committed cp.async groups are pending
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
 __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
@@ -180,18 +172,6 @@ __host__ __device__ constexpr uint32_t idesc_f16_f32(int m, int n) {
          | ((uint32_t)(m >> 4) << 24);      // M / 16
 }
 
-// D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread (kind::f16 with the
-// F16 x F16 instruction descriptor above)
-__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc,
-                                         uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // One lane of a converged warp (the same one every time): nonzero there.
 __device__ __forceinline__ uint32_t elect_one() {
   uint32_t e;
@@ -203,8 +183,9 @@ __device__ __forceinline__ uint32_t elect_one() {
   return e;
 }
 
-// mma_f16 and mma_commit issued by a converged warp, executed by the lane
-// whose `elected` is nonzero.  Descriptors are given by their low words (the
+// D[tmem] (+)= A[smem] * B[smem]^T (kind::f16 with the F16 x F16 instruction
+// descriptor above), issued by a converged warp and executed by the lane whose
+// `elected` is nonzero.  Descriptors are given by their low words (the
 // shared-memory address field) and one common high word.  With all lanes in
 // step the operands stay in uniform registers: issued from inside a
 // one-lane branch an MMA took ~100 clocks of that thread's time, as long as
@@ -222,20 +203,14 @@ __device__ __forceinline__ void mma_f16_elected(uint32_t d_tmem, uint32_t a_lo, 
       ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate), "r"(elected)
       : "memory");
 }
+// arrive on `bar` when every prior tcgen05.mma of the elected thread has
+// completed
 __device__ __forceinline__ void mma_commit_elected(uint64_t *bar, uint32_t elected) {
   asm volatile(
       "{\n\t.reg .pred e;\n\t"
       "setp.ne.b32 e, %1, 0;\n\t"
       "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
       ::"r"(smem_addr(bar)), "r"(elected)
-      : "memory");
-}
-
-// arrive on `bar` when every prior tcgen05.mma of this thread has completed
-__device__ __forceinline__ void mma_commit(uint64_t *bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-      ::"r"(smem_addr(bar))
       : "memory");
 }
 

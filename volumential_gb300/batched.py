@@ -76,7 +76,8 @@ def _give_back(owner, events, arrays):
             entry = _held.popleft()
         except IndexError:
             return
-        if _lib.lib().vl1_stream_capturing(entry[0].cuda_stream) == 0:
+        # (the loaded library itself: a finalizer must not wait for lib()'s lock)
+        if _lib._lib.vl1_stream_capturing(entry[0].cuda_stream) == 0:
             for e in entry[1]:
                 entry[0].wait_event(e)
         else:

@@ -230,6 +230,13 @@ typedef struct {
   int32_t *stale;
 } vl1_tree_copy;
 
+/* Bytes of such a copy, and the copy itself: the arrays of `tree` (`nnz` list
+ * entries) into `buffer` (device memory of the caller's, 256-byte aligned, for as
+ * long as the copy is used) in the stream's order. */
+int64_t vl1_tree_copy_bytes(const vl1_plan *plan, const vl1_tree_view *tree, int64_t nnz);
+int32_t vl1_tree_copy_make(const vl1_plan *plan, const vl1_tree_view *tree, int64_t nnz,
+                           void *buffer, vl1_tree_copy *out, void *stream);
+
 /* As vl1_eval_fp64_tiles, for a schedule made from the arrays in `made_from`:
  * the tree's arrays are compared with them (on the device, in every call).
  * Where they differ the results are those of vl1_eval_fp64 on the arrays as

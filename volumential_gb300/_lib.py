@@ -190,6 +190,9 @@ SIGNATURES = {
                                            C.POINTER(TreeCopy), C.POINTER(MixedSchedule),
                                            C.c_void_p, C.c_int32, C.c_int32, C.c_void_p,
                                            C.c_void_p]),
+    "vl1_tree_copy_bytes": (C.c_int64, [C.c_void_p, C.POINTER(TreeView), C.c_int64]),
+    "vl1_tree_copy_make": (C.c_int32, [C.c_void_p, C.POINTER(TreeView), C.c_int64, C.c_void_p,
+                                       C.POINTER(TreeCopy), C.c_void_p]),
     "vl1_eval_fp64_item_keys": (C.c_int32, [C.c_void_p]),
     "vl1_stream_capturing": (C.c_int32, [C.c_void_p]),
     "vl1_orbit_index_map": (C.c_int32, [C.c_void_p, C.c_void_p, C.c_void_p,

@@ -84,13 +84,6 @@ def _give_back(owner, events, arrays):
             _held.append(entry)
 
 
-#: the tree arrays that a schedule depends on: name in ``keep``, view field
-_COPIED = (("target_boxes", "target_boxes"), ("starts", "neighbor_source_boxes_starts"),
-           ("lists", "neighbor_source_boxes_lists"), ("centers", "box_centers"),
-           ("levels", "box_levels"), ("src_starts", "box_source_starts"),
-           ("src_counts", "box_source_counts_nonchild"), ("smode", "source_mode_ids"))
-
-
 class MixedSchedule:
     """Device-resident schedule (and workspace) of one (plan, tree, nrhs).
 
@@ -137,30 +130,24 @@ class MixedSchedule:
         if workspace:
             _ = self.workspace
 
-    def copy_tree(self, view, keep, stream):
+    def copy_tree(self, plan, view, keep, stream):
         """Keep a copy of the tree arrays that the schedule depends on
         (``tree_copy``, a ``vl1_tree_copy``), for evaluations to compare the
         tree with: the arrays belong to the caller, who may write them."""
         import torch
 
-        copies = {name: torch.empty_like(keep[name]) for name, _ in _COPIED}
-        self._stale = torch.zeros(1, dtype=torch.int32, device="cuda")
+        lib, nnz = _lib.lib(), int(keep["lists"].numel())
+        n = int(lib.vl1_tree_copy_bytes(plan.handle, C.byref(view), nnz))
+        self._tree_arrays = torch.empty(n, dtype=torch.uint8, device="cuda")
         _after_current(stream)
-        with torch.cuda.stream(stream_object(stream)):
-            for name, t in copies.items():
-                t.copy_(keep[name])
-        c = _lib.TreeCopy()
-        C.memmove(C.byref(c.tree), C.byref(view), C.sizeof(_lib.TreeView))
-        for name, field in _COPIED:
-            setattr(c.tree, field, copies[name].data_ptr())
-        c.nnz = int(keep["lists"].numel())
-        c.stale = self._stale.data_ptr()
-        self._tree_arrays = copies
-        self.tree_copy = c
+        self.tree_copy = _lib.TreeCopy()
+        _lib.check(lib.vl1_tree_copy_make(
+            plan.handle, C.byref(view), nnz, self._tree_arrays.data_ptr(),
+            C.byref(self.tree_copy), C.c_void_p(stream)), "vl1_tree_copy_make")
 
     def is_stale(self):
         """Whether an evaluation found other tree arrays (a device read)."""
-        return bool(self._stale.item())
+        return bool(self._tree_arrays[0].item())
 
     def read_by(self, stream):
         """Note that work queued on ``stream`` so far reads the schedule: its

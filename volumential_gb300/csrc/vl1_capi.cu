@@ -423,6 +423,75 @@ int32_t vl1_eval_fp64(vl1_plan *plan, const vl1_tree_view *tree, const void *coe
                       static_cast<cudaStream_t>(stream));
 }
 
+}  // extern "C"
+
+namespace {
+
+// the arrays of a tree copy in the order of the buffer: source, bytes
+struct CopyPart {
+  const void *src;
+  int64_t bytes;
+};
+constexpr int kCopyParts = 8;
+void copy_parts(const vl1_plan *plan, const vl1_tree_view &t, int64_t nnz,
+                CopyPart (&p)[kCopyParts]) {
+  p[0] = {t.target_boxes, 4 * (int64_t)t.n_target_boxes};
+  p[1] = {t.neighbor_source_boxes_starts, 4 * ((int64_t)t.n_target_boxes + 1)};
+  p[2] = {t.neighbor_source_boxes_lists, 4 * nnz};
+  p[3] = {t.box_centers, 8 * (int64_t)plan->d.dim * t.aligned_nboxes};
+  p[4] = {t.box_levels, t.nboxes};
+  p[5] = {t.box_source_starts, 4 * t.nboxes};
+  p[6] = {t.box_source_counts_nonchild, 4 * t.nboxes};
+  p[7] = {t.source_mode_ids, 4 * t.n_particles};
+}
+int64_t part256(int64_t b) { return (b + 255) / 256 * 256; }
+
+}  // namespace
+
+extern "C" {
+
+int64_t vl1_tree_copy_bytes(const vl1_plan *plan, const vl1_tree_view *tree, int64_t nnz) {
+  if (!plan || !tree || nnz < 0) return -1;
+  CopyPart p[kCopyParts];
+  copy_parts(plan, *tree, nnz, p);
+  int64_t n = 256;   // the stale word
+  for (const CopyPart &q : p) n += part256(q.bytes);
+  return n;
+}
+
+int32_t vl1_tree_copy_make(const vl1_plan *plan, const vl1_tree_view *tree, int64_t nnz,
+                           void *buffer, vl1_tree_copy *out, void *stream) {
+  if (!plan || !tree || nnz < 0 || !buffer || !out) {
+    set_error("vl1_tree_copy_make: null argument or negative size");
+    return VL1_E_ARG;
+  }
+  CopyPart p[kCopyParts];
+  copy_parts(plan, *tree, nnz, p);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  uint8_t *w = static_cast<uint8_t *>(buffer);
+  out->stale = reinterpret_cast<int32_t *>(w);
+  cudaError_t e = cudaMemsetAsync(w, 0, 256, s);
+  w += 256;
+  const void *at[kCopyParts];
+  for (int k = 0; k < kCopyParts && e == cudaSuccess; ++k) {
+    at[k] = w;
+    if (p[k].bytes > 0) e = cudaMemcpyAsync(w, p[k].src, p[k].bytes, cudaMemcpyDeviceToDevice, s);
+    w += part256(p[k].bytes);
+  }
+  if (e != cudaSuccess) return cuda_fail(e, "vl1_tree_copy_make");
+  out->tree = *tree;
+  out->nnz = nnz;
+  out->tree.target_boxes = static_cast<const int32_t *>(at[0]);
+  out->tree.neighbor_source_boxes_starts = static_cast<const int32_t *>(at[1]);
+  out->tree.neighbor_source_boxes_lists = static_cast<const int32_t *>(at[2]);
+  out->tree.box_centers = static_cast<const double *>(at[3]);
+  out->tree.box_levels = static_cast<const uint8_t *>(at[4]);
+  out->tree.box_source_starts = static_cast<const int32_t *>(at[5]);
+  out->tree.box_source_counts_nonchild = static_cast<const int32_t *>(at[6]);
+  out->tree.source_mode_ids = static_cast<const int32_t *>(at[7]);
+  return VL1_OK;
+}
+
 int32_t vl1_stream_capturing(void *stream) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   const cudaError_t e = cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &cap);

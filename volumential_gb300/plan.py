@@ -424,7 +424,7 @@ class Plan:
             sched = MixedSchedule(self, view, keep, rows, stream, **own)
             if sched.max_keys_per_item > cap:
                 sched = MixedSchedule(self, view, keep, rows, stream, cap, base=sched, **own)
-            sched.copy_tree(view, keep, stream)
+            sched.copy_tree(self, view, keep, stream)
             stream_object(stream).synchronize()   # read on any stream from here on
         except (ValueError, ScheduleError):
             return False, none         # no schedule describes this tree

@@ -300,12 +300,16 @@ def gpu_arm(args):
     odt = torch.complex128 if out_complex else torch.float64
     out_plain = torch.empty(nrhs * n, dtype=odt, device="cuda")
     out_mixed = torch.empty(nrhs * n, dtype=odt, device="cuda")
+    out_fp64 = torch.empty(nrhs * n, dtype=odt, device="cuda")
     flush = torch.empty(L2_FLUSH_BYTES // 4, dtype=torch.float32, device="cuda")
     stream = torch.cuda.current_stream()
     sh = stream.cuda_stream
 
     def plain_step():
         plan.eval_fp64(view, coefs, out_plain, stream=sh, nrhs=nrhs)
+
+    def fp64_step():   # what an evaluator's FP64 call runs (the faster kernel)
+        plan.eval_fp64(view, coefs, out_fp64, stream=sh, nrhs=nrhs, keep=keep)
 
     def mixed_step():
         eval_mixed(plan, view, coefs, out_mixed, stream=sh, nrhs=nrhs, keep=keep)
@@ -319,6 +323,7 @@ def gpu_arm(args):
     for _ in range(args.warmup):
         flush.fill_(1.0)
         plain_step()
+        fp64_step()
         mixed_step()
     plan.raise_on_status(sh)
     torch.cuda.synchronize()
@@ -330,7 +335,7 @@ def gpu_arm(args):
     torch.cuda.synchronize()
     res = {}
     from volumential_gb300 import _lib
-    for name, fn in (("plain", plain_step), ("mixed", mixed_step)):
+    for name, fn in (("plain", plain_step), ("fp64", fp64_step), ("mixed", mixed_step)):
         step_ms, kernel_ms = _timed_steps(torch, fn, flush, args.steps, stream,
                                           _lib.lib() if name == "mixed" else None)
         total = max_over_ranks(float(sum(step_ms)))
@@ -344,6 +349,8 @@ def gpu_arm(args):
     mixed_errs = [float(np.linalg.norm(ym[r] - yp[r]) / np.linalg.norm(yp[r]))
                   for r in range(nrhs)]
     mixed_err = max(mixed_errs)
+    fp64_err = float((out_fp64 - out_plain).norm() / out_plain.norm())
+    del out_fp64
     headline = "plain"
     if mixed_err <= 1e-9 and res["mixed"]["total_ms"] < res["plain"]["total_ms"]:
         headline = "mixed"   # the faster path within its tolerance
@@ -420,6 +427,7 @@ def gpu_arm(args):
         "d2h": int(host_out.numel() * host_out.element_size()),
         "plan_bytes": plan.device_bytes(), "world": world, "rank": rank,
         "mixed_err": mixed_err, "mixed_errs": mixed_errs, "api_err": api_err, "cold": cold,
+        "fp64_err": fp64_err,
         "headline": headline, "fp64_gflops": measured_fp64_gflops(),
         "schedule": {"tiles": sched.n_tiles, "tile_keys": sched.n_tile_keys,
                      "mean_keys_per_tile": sched.mean_keys_per_tile,
@@ -604,6 +612,7 @@ def gb300_main(args):
 
     plain = path_summary("plain")
     mixed = path_summary("mixed")
+    fp64_call = dict(path_summary("fp64"), rel_l2_vs_plain=r["fp64_err"])
     plain.update({"fp64_gflops": F / (plain["ms_per_step"] / 1e3) / 1e9,
                   "fp64_peak_gflops_measured_dgemm": fp64_peak,
                   "fp64_frac_of_measured_dgemm":
@@ -669,7 +678,8 @@ def gb300_main(args):
                        else "FPNDExpansionWrangler.eval_direct_batched"},
         "e2e_cold": _cold_summary(r, n, nrhs),
         "roofline": roof,
-        "paths": {"plain_fp64": plain, "mixed": dict(mixed, rel_l2_vs_fp64=r["mixed_err"]),
+        "paths": {"plain_fp64": plain, "fp64_call": fp64_call,
+                  "mixed": dict(mixed, rel_l2_vs_fp64=r["mixed_err"]),
                   "speedup_mixed_over_plain": plain["ms_per_step"] / mixed["ms_per_step"]},
         "mixed_schedule": r["schedule"], "mixed_geometry": r["geometry"],
         # digit products the tensor pipe executes per step (15 FP16 digit
@@ -1167,6 +1177,7 @@ def table_main(args):
         t = NearFieldInteractionTable(q, dim=dim, sumpy_kernel=knl, dtype=dt)
         ids = t._get_invariant_entry_info()["entry_ids"]
         nodes_per_entry = (2 ** dim) * (6 if dim == 3 else 2) * reg ** (dim - 1) * n_rad
+        n_targets = len(np.unique(ids // t.n_pairs * t.n_q_points + ids % t.n_q_points))
         for _ in range(args.warmup):
             TB.build_table_values(t, entry_ids=ids[:256], k=k, store=False)
         torch.cuda.synchronize()
@@ -1191,18 +1202,19 @@ def table_main(args):
                         creg, crad, k=k or 0.0)
         csec = time.perf_counter() - c0
         out[name] = {"entries": int(len(ids)), "nodes_per_entry": int(nodes_per_entry),
-                     "build_s": tsec, "entries_per_s": len(ids) / tsec,
-                     "node_evals_per_s": len(ids) * nodes_per_entry / tsec,
+                     "targets": n_targets, "build_s": tsec, "entries_per_s": len(ids) / tsec,
+                     # (all modes of a target share its nodes' kernel values)
+                     "node_evals_per_s": n_targets * nodes_per_entry / tsec,
                      "cpu_node_evals_per_s": len(sample) * cn / csec,
                      "cpu_sample": f"{len(sample)} entries at regular {creg} / radial {crad}, "
                                    f"{csec:.2f} s (numpy restatement, 1 core)"}
     head = out["lap3d_q4"]
     hbm, bf16, peak_kind = peaks()
     fp64_peak = measured_fp64_gflops()
-    # FP64 flops per enumerated node of the 3D Laplace q=4 build: DADD + DMUL +
-    # 2 x DFMA thread instructions of one launch (ncu counters) over its nodes,
-    # the nodes of empty sub-boxes included
-    ops_per_node = 10.74
+    # FP64 flops per enumerated node of a target of the 3D Laplace q=4 build:
+    # DADD + DMUL + 2 x DFMA thread instructions of one launch (ncu counters)
+    # over its nodes, the nodes of empty sub-boxes included
+    ops_per_node = 9.26
     line = {
         "metric": "table build: entries/s (FP64 Duffy radial, default orders)",
         "value": head["entries_per_s"], "unit": "entries/s", "n_gpus": world,
@@ -1373,10 +1385,12 @@ def split_main(args):
     """Helmholtz split correction (``vl1_split_correction``): the list-1 sum
     of density x weight x R(r), R = G_k - G_0 by its series, over the C3 tree
     (2D uniform level 6, q = 5, 102,400 points, k = 20).  One step = one
-    device sum (CUDA events); roofline: the FP64 pipe (per pair 4 flops per
-    series term for the two real Horner sums of a real wave number, ~40 for
-    the log and the complex accumulation) against the DGEMM rate measured in
-    the same run."""
+    device sum (CUDA events); roofline: the FP64 pipe against the DGEMM rate
+    measured in the same run.  Counted are 4 flops per pair (a real weight
+    times the complex R) and, once per relative position of two boxes and pair
+    of their points, R itself (4 flops per series term for the two real Horner
+    sums of a real wave number, ~40 for the log and the rest): the sum reads R
+    from tables of the tree's 3^2 positions."""
     import torch
 
     from volumential_gb300 import workloads as W
@@ -1412,7 +1426,8 @@ def split_main(args):
     clock_info = clocks.stop()
     t = float(np.median(ms)) / 1e3
     pairs = w.pair_count()
-    flops = pairs * (4 * n_terms + 40)
+    nq = w.q ** w.dim
+    flops = 4 * pairs + 3 ** w.dim * nq * nq * (4 * n_terms + 40)
     fp64_peak = measured_fp64_gflops()
     # CPU restatement on a sample of target boxes (closed form, numpy)
     from oracle import split_oracle as SO
@@ -1442,7 +1457,7 @@ def split_main(args):
                    "l2": "flushed between steps (256 MiB write)"},
         "roofline": {"bound": "fp64", "achieved": flops / t / 1e9, "peak": fp64_peak,
                      "unit": "GFLOP/s", "frac": flops / t / 1e9 / fp64_peak,
-                     "kernel": "split_remainder_kernel", "traffic": None,
+                     "kernel": "split_sum_kernel", "traffic": None,
                      "peak_note": "cuBLAS DGEMM measured in this run"},
         "rel_l2_vs_cpu_closed_form": err,
         "cpu_baseline": {"value": sub_pairs / cpu_s, "unit": "pairs/s", "cores": 1,

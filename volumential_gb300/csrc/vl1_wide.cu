@@ -57,6 +57,7 @@
 // source is summed in FP64 by the CTA that writes its tile.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "vl1_internal.cuh"
@@ -228,6 +229,7 @@ struct WidePrep {
   int n_counters;
   Span spans[kSpans];
   int64_t max_chunks;
+  int row_blocks;    // blocks that form digits; the others compare the arrays
   int *stale;        // nullptr: the caller answers for the schedule
   vl1_status *st;
 };
@@ -276,13 +278,16 @@ __global__ void __launch_bounds__(128) wide_prep_kernel(const __grid_constant__ 
   uint8_t *stage = s_stage + (threadIdx.x >> 5) * kPrepRows * row_bytes;
   if (blockIdx.x == 0)
     for (int i = threadIdx.x; i < P.n_counters; i += blockDim.x) P.counters[i] = 0;
-  if (P.stale && tree_differs(P, blockIdx.x * (int64_t)blockDim.x + threadIdx.x,
-                              (int64_t)gridDim.x * blockDim.x)) {
-    *P.stale = 1;
-    reinterpret_cast<PlanStatus *>(P.st)->stale = 1;
+  if ((int)blockIdx.x >= P.row_blocks) {   // (uniform) the blocks that compare
+    if (tree_differs(P, (blockIdx.x - P.row_blocks) * (int64_t)blockDim.x + threadIdx.x,
+                     (int64_t)(gridDim.x - P.row_blocks) * blockDim.x)) {
+      *P.stale = 1;
+      reinterpret_cast<PlanStatus *>(P.st)->stale = 1;
+    }
+    return;
   }
   const int64_t n_rows = tr.nboxes * P.nv;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int64_t warps = (int64_t)P.row_blocks * (blockDim.x >> 5);
   const int cs = P.cc ? 2 : 1;
   for (int64_t grp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
        grp * kPrepRows < n_rows; grp += warps) {
@@ -1414,9 +1419,14 @@ int32_t launch_wide(vl1_plan *plan, const TreeDev &tree, const vl1_tree_copy *ma
                              (int)prep_smem);
   if (e == cudaSuccess) {
     const int64_t groups = (n_rows + kPrepRows - 1) / kPrepRows;
-    const int64_t blocks = (groups + 3) / 4;
-    wide_prep_kernel<<<(unsigned)(blocks < 152 * 32 ? blocks : 152 * 32), 128, prep_smem, s>>>(
-        pp);
+    // (blocks of their own compare the arrays, a thread one chunk of each: ahead
+    // of the rows in the same blocks it took 4 us of 3D level 4, q = 5)
+    pp.row_blocks = (int)std::min<int64_t>((groups + 3) / 4, 152 * 32);
+    const int cmp =
+        made_from ? (int)std::min<int64_t>(std::max<int64_t>((pp.max_chunks + 127) / 128, 1),
+                                           152 * 16)
+                  : 0;
+    wide_prep_kernel<<<(unsigned)(pp.row_blocks + cmp), 128, prep_smem, s>>>(pp);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess && sched.n_tiles > 0) {

@@ -100,7 +100,7 @@ class MixedSchedule:
 
         lib = _lib.lib()
         self._owner = torch.cuda.current_stream()
-        self._owner_handle = self._owner.cuda_stream
+        self.owner_handle = self._owner.cuda_stream
         self._readers = {}
         self.nrhs = int(nrhs)
         self._workspace = None
@@ -144,6 +144,8 @@ class MixedSchedule:
         _lib.check(lib.vl1_tree_copy_make(
             plan.handle, C.byref(view), nnz, self._tree_arrays.data_ptr(),
             C.byref(self.tree_copy), C.c_void_p(stream)), "vl1_tree_copy_make")
+        # arguments of vl1_eval_fp64_tiles_of
+        self.fp64_refs = (C.byref(self.tree_copy), C.byref(self.c_struct))
 
     def is_stale(self):
         """Whether an evaluation found other tree arrays (a device read)."""
@@ -152,7 +154,7 @@ class MixedSchedule:
     def read_by(self, stream):
         """Note that work queued on ``stream`` so far reads the schedule: its
         arrays go back to their owner's memory pool after it."""
-        if stream == self._owner_handle or _lib.lib().vl1_stream_capturing(stream) != 0:
+        if stream == self.owner_handle or _lib.lib().vl1_stream_capturing(stream) != 0:
             return
         import torch
 

@@ -16,15 +16,17 @@
 // depends only on the pair of boxes' relative position and levels: on a tree
 // of many boxes R is evaluated once per (source level, relative position) and
 // point pair, and the sums read it from there (split_sum_kernel: two FMAs and
-// 16 bytes from the L2 per pair).  split_mark_kernel checks on the device that
-// every box's points are its level's template and every centre lies on the
-// lattice (to a few ulps of the coordinates, the rounding of the points
-// themselves) and its source and target points the same; otherwise, and for small trees, the per-pair kernel
+// 16 bytes per pair; bound by the FP64 pipe, 82 % busy, the tables in L1).
+// split_mark_kernel checks on the device that every box's points are its
+// level's template and every centre lies on the lattice (to a few ulps of the
+// coordinates, the rounding of the points themselves) and its source and
+// target points the same; otherwise, and for small trees, the per-pair kernel
 // runs: one CTA per target box, one thread per target point, the points and
 // strengths of each list-1 source box staged in shared memory.
 //
 // Measured (GB300, 2D k = 20, 102,400 points, 22.6M point pairs): 3,950 us per
-// pair, about 90 us with the tables.
+// pair; with the tables 164 us on the device (sum 116, marking 30, tables 8,
+// level boxes 6, the per-pair kernel that finds nothing to do 4).
 
 #include <cuda_runtime.h>
 

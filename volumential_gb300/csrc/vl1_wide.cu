@@ -43,14 +43,15 @@
 // source point in the corner neighbour up to 1e-15 (3D, q = 4) and 5e-15 (2D,
 // q = 6) of its value, 1e-16 per box.
 //
-// Measured (GB300): the 1.5M-point octree 4,700 us per-box, 229 us here
-// (digits 22 us, tensor-core kernel 206 us, its tensor pipe busy 105 us of
-// them); 3D q = 5, 512,000 points 3,240 and 167 us; 3D q = 3, 110,592 points
-// x 8 right-hand sides 1,530 and 127 us; 2D complex q = 5, 102,400 points 185
-// and 43 us.  Bound: shared memory (per unit 120 KB of operand reads and 48 KB
-// of stores, 1,350 of the ~1,750 clocks) and the L2's delivery to all SMs (36
-// KB at ~30 bytes per SM and clock, 1,200), close behind them the tensor pipe
-// (1,176); per work item ~12 us of start and result write.
+// Measured (GB300, a call's device time): the 1.5M-point octree 4,610 us
+// per-box, 232 us here (digits and the comparison of the tree's arrays about 24
+// us, tensor-core kernel 206 us, its tensor pipe busy 105 us of them); 3D q = 5,
+// 512,000 points 3,220 and 169 us; 3D q = 3, 110,592 points x 8 right-hand sides
+// 1,400 and 127 us; 2D complex q = 5, 102,400 points 174 and 43 us.  Bound:
+// shared memory (per unit 120 KB of operand reads and 48 KB of stores, 1,350 of
+// the ~1,750 clocks) and the L2's delivery to all SMs (36 KB at ~30 bytes per SM
+// and clock, 1,200), close behind them the tensor pipe (1,176); per work item
+// ~12 us of start and result write.
 //
 // Density rows with an infinite or NaN value (or whose scaled value
 // overflows) cannot be written in fixed point: every target row with such a

@@ -347,10 +347,11 @@ class Plan:
             sched = self._fp64_schedule(view, keep, coefs.is_complex(), int(nrhs), stream)
         if sched is not None:
             st = self._lib.vl1_eval_fp64_tiles_of(
-                self.handle, C.byref(view), C.byref(sched.tree_copy), C.byref(sched.c_struct),
-                coefs.data_ptr(), ctype, int(nrhs), out.data_ptr(), C.c_void_p(stream))
+                self.handle, C.byref(view), *sched.fp64_refs, coefs.data_ptr(), ctype,
+                int(nrhs), out.data_ptr(), stream)
             _lib.check(st, "vl1_eval_fp64_tiles_of")
-            sched.read_by(stream)
+            if stream != sched.owner_handle:
+                sched.read_by(stream)
             return
         st = self._lib.vl1_eval_fp64(self.handle, C.byref(view), coefs.data_ptr(), ctype,
                                      int(nrhs), out.data_ptr(), C.c_void_p(stream))
